@@ -20,17 +20,22 @@
 //    so the TUs of one level are independent of one another.
 // One persistent launch covers the batch.  A CTA claims superblocks from an
 // atomic counter in a topological order (dependency depth, frame, decode
-// order), stages the superblock's samples in shared memory, waits (bounded)
-// for the superblocks it depends on, runs the levels — a level's small TUs one
-// per warp, then its large TUs with the whole CTA — writes the samples back and
-// publishes a done flag.  A CTA only waits for superblocks claimed before its
-// own, by CTAs that are running, so every wait ends; the time bound only
+// order), stages the superblock's samples, a border of its neighbours and its TU
+// records in shared memory and runs the levels: small TUs one per warp, large
+// ones with a group of warps.  A CTA only waits for superblocks claimed before
+// its own, by CTAs that are running, so every wait ends; the time bound only
 // guards against a broken invariant: a wait that runs out sets its frame's
-// abort word in the launch's control block, every superblock of that frame
-// then skips its remaining TUs (still publishing its levels, so no wait of
-// the launch is left hanging), and the host reports that frame of that
-// launch as AV1G_EDEVICE.  Other frames of the batch are not affected: waits
-// never cross frames.
+// abort word in the launch's control block, the superblocks of that frame then
+// no longer wait (they still run and publish their levels, so no wait of the
+// launch is left hanging, but their samples are not to be used), and the host
+// reports that frame of that launch as AV1G_EDEVICE.  Other frames of the batch
+// are not affected: waits never cross frames.
+//
+// What bounds it is the chain of levels: a 1920x1080 key frame's longest one has
+// about 2,200, nearly all with one to four TUs of at most 256 samples.  Measured
+// on that frame (one launch, B200): 8.5 ms with a body per transform size and
+// every level on one barrier, 2.5 ms in this form; 3840x2160 10-bit in 2 x 2
+// tiles 10.0 against 2.6 ms, eight 640x360 frames 2.7 against 0.78 ms.
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -50,17 +55,22 @@ namespace {
 
 using namespace itx;
 
-constexpr int kT = 128;             // threads per CTA
-constexpr int kNW = kT / 32;        // warps per CTA
+constexpr int kT = 128;             // threads per CTA of intra_pre_kernel
+constexpr int kNW = kT / 32;
+constexpr int kGroups = 3;          // worker groups of intra_kernel, which take levels in turn
+constexpr int kGW = 4;              // warps per group
+constexpr int kGT = kGW * 32;
+constexpr int kWW = kGroups * kGW;  // worker warps
+constexpr int kIT = kWW * 32 + 64;  // + the publishing warp and the waiting warp
 constexpr int kSmallPx = kIntraSmallPx;
-constexpr int kLvChunk = 64;        // level-table entries staged at a time
-constexpr int kTuWin = 128;         // TU records staged at a time
-constexpr int kWaitWin = 32;        // waits staged per superblock (more: read from HBM)
+constexpr int kLvStage = 512;       // level-table entries staged per superblock (more: read from HBM)
+constexpr int kTuStage = 512;       // TU records staged per superblock (more: read from HBM)
 constexpr long long kWaitNs = 2000000000LL;  // the bound of one dependency wait
 
+__constant__ AV1T_TX_WIDTH_TYPE c_txw_d AV1T_TX_WIDTH_DIMS = AV1T_TX_WIDTH_INIT;
+__constant__ AV1T_TX_HEIGHT_TYPE c_txh_d AV1T_TX_HEIGHT_DIMS = AV1T_TX_HEIGHT_INIT;
 __constant__ AV1T_MODE_TO_ANGLE_TYPE c_mode_angle AV1T_MODE_TO_ANGLE_DIMS = AV1T_MODE_TO_ANGLE_INIT;
 __constant__ AV1T_DR_INTRA_DERIVATIVE_TYPE c_dr AV1T_DR_INTRA_DERIVATIVE_DIMS = AV1T_DR_INTRA_DERIVATIVE_INIT;
-__constant__ AV1T_INTRA_EDGE_KERNEL_TYPE c_edge_k AV1T_INTRA_EDGE_KERNEL_DIMS = AV1T_INTRA_EDGE_KERNEL_INIT;
 __constant__ AV1T_INTRA_FILTER_TAPS_TYPE c_fi_taps AV1T_INTRA_FILTER_TAPS_DIMS = AV1T_INTRA_FILTER_TAPS_INIT;
 __constant__ AV1T_SM_WEIGHTS_TX_4X4_TYPE c_sm4 AV1T_SM_WEIGHTS_TX_4X4_DIMS = AV1T_SM_WEIGHTS_TX_4X4_INIT;
 __constant__ AV1T_SM_WEIGHTS_TX_8X8_TYPE c_sm8 AV1T_SM_WEIGHTS_TX_8X8_DIMS = AV1T_SM_WEIGHTS_TX_8X8_INIT;
@@ -69,10 +79,24 @@ __constant__ AV1T_SM_WEIGHTS_TX_32X32_TYPE c_sm32 AV1T_SM_WEIGHTS_TX_32X32_DIMS 
 __constant__ AV1T_SM_WEIGHTS_TX_64X64_TYPE c_sm64 AV1T_SM_WEIGHTS_TX_64X64_DIMS = AV1T_SM_WEIGHTS_TX_64X64_INIT;
 __constant__ AV1T_SUBPEL_FILTERS_TYPE c_subpel AV1T_SUBPEL_FILTERS_DIMS = AV1T_SUBPEL_FILTERS_INIT;
 
-// The superblock's area in each plane and where the shared-memory copy keeps it.
+// The superblock's copy in shared memory: per plane its area {x0, y0, w, h}
+// with one row above (running on past the right edge, for above-right edges)
+// and one column to the left, so that an edge is read the same way inside the
+// superblock and across its border.  off: the index of the area's first
+// sample; cs: the row pitch in samples, a multiple of four (four-sample groups
+// are 8-byte aligned) whose 32-bit words advance two banks per row, so that
+// the 16 rows of a left edge fall on 16 banks.
 struct SbCtx {
-    int x0[3], y0[3], w[3], h[3], off[3];
+    int4 rect[3];
+    int off[3], cs[3];
 };
+__device__ __forceinline__ int copy_pitch(int log2sb, int ssx) { return intra_copy_pitch((1 << log2sb) >> ssx); }
+__device__ __forceinline__ int copy_off(int log2sb, int ssx, int ssy, int p) {
+    int o = copy_pitch(log2sb, p ? ssx : 0) + 4;
+    if (p > 0) o += intra_copy_samples(1 << log2sb, 1 << log2sb);
+    if (p > 1) o += intra_copy_samples((1 << log2sb) >> ssx, (1 << log2sb) >> ssy);
+    return o;
+}
 
 __device__ const AV1T_II_WEIGHTS_1D_TYPE g_ii_w AV1T_II_WEIGHTS_1D_DIMS = AV1T_II_WEIGHTS_1D_INIT;
 __device__ const wedge::Master g_wmaster = wedge::kMaster;
@@ -80,25 +104,79 @@ __device__ const wedge::Master g_wmaster = wedge::kMaster;
 // av1g_test_intra_wait_fault).
 __device__ long long g_wait_ns = kWaitNs;
 
+// ---- TU records -------------------------------------------------------------
+// intra_pre_kernel turns every av1g_intra_tu of the launch, in place, into the
+// form the wavefront reads: all that follows from the descriptor, the frame
+// and the superblock (class, angles, edge lengths and filters, the place in
+// the superblock's copy) is worked out there, in parallel, so that the serial
+// chain of TUs holds only what depends on samples.
+
+enum Cls : uint8_t {
+    C_NONE, C_DC, C_V, C_H, C_SMOOTH, C_SMOOTH_V, C_SMOOTH_H, C_PAETH,
+    C_D1,  // directional, angle below 90: the above edge only
+    C_D2,  // between 90 and 180: both edges
+    C_D3,  // from 180: the left edge only
+    C_FI, C_PAL, C_BC
+};
+enum : uint8_t {  // TuHead::bits
+    R_ABOVE = 1, R_LEFT = 2, R_RES = 4, R_CFL = 8,
+    R_EDGE = 16,     // an edge is filtered or upsampled, or the corner is
+    R_CORNER = 32, R_UPA = 64, R_UPL = 128
+};
+enum : uint8_t {  // TuHead::where
+    W_COPY = 1,      // every edge sample lies in the superblock's copy
+    W_DIRECT = 2,    // and the prediction reads both edges there, in place
+    W_CFL = 4,       // CfL's luma lies in the copy, in aligned pairs
+    W_ALIGNED = 8,   // x is a multiple of four
+    W_FAST = 16      // a small TU that fast_decode / fast_run take
+};
+
+struct TuHead {
+    uint32_t res;          // its residual block (R_RES)
+    uint16_t x, y;         // plane sample position
+    uint32_t coff;         // its first sample in the superblock's copy
+    uint8_t dims;          // log2 width | log2 height << 4
+    uint8_t cls, plane, bits;
+    uint8_t strength;      // edge filter strength above | left << 4
+    uint8_t misc;          // filter intra mode | interintra << 4
+    int8_t alpha;
+    uint8_t where;
+    uint16_t na, nl;       // samples the above / left edge has before it repeats the last
+    uint16_t ea, el;       // edge samples the prediction uses
+    uint16_t fa, fl;       // edge filter lengths (corner included)
+    int16_t dx, dy;
+    uint16_t cx, cy;       // CfL: the last luma position averaged
+    uint32_t map;          // palette map, wedge window of an inter-intra block, or the copy's vector (row << 16 | column)
+    uint16_t stride;       // palette map
+    uint8_t ii_mode, pad;
+};
+struct alignas(16) TuRec {
+    TuHead h;
+    union {
+        uint16_t colors[8];
+        uint32_t recip;    // DC: ceil(2^32 / edge samples)
+    };
+};
+static_assert(sizeof(TuHead) == 48 && sizeof(TuRec) == sizeof(av1g_intra_tu), "records are converted in place");
+
 // The intra half of an inter-intra block: blend of the intra prediction
 // with the inter half (mask_blend_interintra, src/inter_pred.rs:3272).  The
 // mask is the §7.11.3.13 smooth mask on the plane block (read at [i][j]
 // directly) or the §7.11.3.11 wedge mask on the luma grid (orientation
-// resolved by the host into palette_map).
-template <int W, int H>
-__device__ __forceinline__ int interintra_px(const IntraFrame& F, const av1g_intra_tu& t, int i, int j, int intra,
-                                             int inter, int maxv) {
+// resolved by the host into map).
+__device__ int interintra_px(const IntraFrame& F, const TuHead& t, int kind, int i, int j, int intra, int inter,
+                             int maxv) {
     int m;
-    if (t.interintra == 2) {
-        const uint32_t o = t.palette_map;
+    if (kind == 2) {
+        const uint32_t o = t.map;
         const wedge::Orient w{(uint8_t)(o & 0xff), (uint8_t)((o >> 8) & 0xff), (uint8_t)((o >> 16) & 0xff),
                               (uint8_t)(o >> 24)};
         m = wedge::mask_px(g_wmaster, w, t.plane ? F.ssx : 0, t.plane ? F.ssy : 0, i, j);
     } else {
-        constexpr int scale = 128 / (W > H ? W : H);
-        const int mode = t.interintra_mode;
-        m = mode == 1 ? __ldg(&g_ii_w[i * scale]) : mode == 2 ? __ldg(&g_ii_w[j * scale])
-          : mode == 3 ? __ldg(&g_ii_w[min(i, j) * scale]) : 32;
+        const int sh = 7 - max(t.dims & 15, t.dims >> 4);  // 128 / max(w, h)
+        const int mode = t.ii_mode;
+        m = mode == 1 ? __ldg(&g_ii_w[i << sh]) : mode == 2 ? __ldg(&g_ii_w[j << sh])
+          : mode == 3 ? __ldg(&g_ii_w[min(i, j) << sh]) : 32;
     }
     return min(max((m * intra + (64 - m) * inter + 32) >> 6, 0), maxv);
 }
@@ -110,60 +188,73 @@ struct WarpG {
     int r;
     __device__ __forceinline__ void sync() const { __syncwarp(); }
 };
-struct CtaG {
+struct CtaG {  // intra_pre_kernel's CTA
     static constexpr int N = kT;
     int r;
     __device__ __forceinline__ void sync() const { __syncthreads(); }
 };
-
-// Per-group scratch: edge arrays (index 0 == position -2), the dense
-// coefficient / residual block, the reduction slots and the TU record.
-template <int E, int PX>
-struct Scr {
-    uint16_t above[E], left[E], dup[E];
-    int buf[PX];
-    long long red[kNW];
-    av1g_intra_tu tu;
+// Hardware barriers of intra_kernel: 0 the CTA, 1..3 the end of a level (the
+// group that ran it arrives, the group of the next level waits), 4..6 within a
+// group.
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int n) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+struct WorkG {  // a worker group
+    static constexpr int N = kGT;
+    int r, id;
+    __device__ __forceinline__ void sync() const { bar_sync(id, kGT); }
 };
-using WScr = Scr<96, kSmallPx>;  // W + H <= 40 for the small sizes: 2 + 2 * 40 entries at most
-using CScr = Scr<272, 64 * 64>;  // 2 * (64 + 64) + 2 rounded up
+
+// Per-group scratch.  The edge arrays hold position k of an edge at [4 + k]
+// (the corner, position -1, at [3]; an upsampled edge starts at position -2):
+// [0, E) above, [E, 2 E) left, as gathered (raw) and after the edge filter or
+// upsampling (fin).
+template <int EN, int PX>
+struct Scr {
+    static constexpr int E = EN;
+    alignas(16) uint16_t raw[2 * EN];
+    alignas(16) uint16_t fin[2 * EN];
+    alignas(16) uint16_t buf[PX];  // CfL luma, intra block copy
+    int red[kGW];
+};
+using WScr = Scr<48, kSmallPx>;  // W + H <= 40 for the small sizes
+using CScr = Scr<136, 64 * 64>;  // W + H <= 128
+
+constexpr int kNoWait = 0x7fffffff;
+
+struct Tables {
+    alignas(8) int8_t fi[5][8][8];  // filter intra taps
+    alignas(4) uint8_t sm[124];     // smooth weights, length n at n - 4
+};
 
 struct alignas(16) Shared {
     union {
-        WScr w[kNW];
+        WScr w[kGW];
         CScr c;
-    } s;
+    } s[kGroups];
     IntraFrame fr;  // the superblock's frame record
-    int2 lv[kLvChunk + 1];
-    int4 wv[kWaitWin];
+    Tables tb;
+    int2 lv[kLvStage];
     SbCtx sb;
-    int idx, abort_seen;
+    int idx;
+    int done;   // levels finished, as far as they are published (workers -> publishing warp)
+    int ready;  // levels below this one may run (waiting warp -> workers)
 };
 static_assert(sizeof(IntraFrame) % 4 == 0, "frame record copied as words");
-
-// The batch's residual blocks (intra_res_kernel); an intra TU's device record
-// carries its block's offset in res.coeff_offset.
-struct Pool {
-    const int32_t* res;
-}; 
 constexpr size_t kSharedBytes = (sizeof(Shared) + 15) & ~(size_t)15;
-
-__device__ __forceinline__ const uint8_t* sm_weights(int log2n) {
-    return log2n == 2 ? c_sm4 : log2n == 3 ? c_sm8 : log2n == 4 ? c_sm16 : log2n == 5 ? c_sm32 : c_sm64;
-}
 
 // Sum over the group (every thread of it calls).
 template <class G, class S>
-__device__ __forceinline__ long long gsum(const G& g, S& s, long long v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffff, v, o);
+__device__ __forceinline__ int gsum(const G& g, S& s, int v) {
+    v = __reduce_add_sync(0xffffffffu, v);
     if constexpr (G::N > 32) {
         if ((g.r & 31) == 0) s.red[g.r >> 5] = v;
-        __syncthreads();
-        long long t = 0;
+        g.sync();
+        int t = 0;
 #pragma unroll
         for (int k = 0; k < G::N / 32; k++) t += s.red[k];
-        __syncthreads();
+        g.sync();
         return t;
     } else {
         return v;
@@ -172,10 +263,11 @@ __device__ __forceinline__ long long gsum(const G& g, S& s, long long v) {
 
 // A sample of plane p at (y, x), inside the plane: from the shared-memory
 // copy when it lies in the current superblock, else from HBM (an earlier
-// superblock's final samples, published by its done flag; read past L1).
+// superblock's final samples, published by its progress word; read past L1).
 __device__ __forceinline__ int rdp(const IntraFrame& F, const SbCtx& c, const uint16_t* cache, int p, int y, int x) {
-    const int ly = y - c.y0[p], lx = x - c.x0[p];
-    if ((unsigned)ly < (unsigned)c.h[p] && (unsigned)lx < (unsigned)c.w[p]) return cache[c.off[p] + ly * c.w[p] + lx];
+    const int4 r = c.rect[p];
+    const int ly = y - r.y, lx = x - r.x;
+    if ((unsigned)ly < (unsigned)r.w && (unsigned)lx < (unsigned)r.z) return cache[c.off[p] + ly * c.cs[p] + lx];
     const PlaneDev& P = F.planes[p];
     const uint8_t* row = P.p + (size_t)y * P.stride;
     return F.hbd ? (int)__ldcg(reinterpret_cast<const unsigned short*>(row) + x) : (int)__ldcg(row + x);
@@ -205,41 +297,132 @@ __device__ int upsample_sel(int w, int h, int ft, int delta) {
     return ft == 0 ? (w + h <= 16) : (w + h <= 8);
 }
 
-// intra_edge_filter (cdf.rs:2760) on an edge array (index 0 == position -2), in parallel
-template <class G, class S>
-__device__ void edge_filter(const G& g, S& s, uint16_t* e, int sz, int strength) {
-    if (strength == 0 || sz == 0) return;  // uniform over the group
-    for (int i = g.r; i < sz; i += G::N) s.dup[i] = e[i + 1];
-    g.sync();
-    for (int i = 1 + g.r; i < sz; i += G::N) {
-        int acc = 0;
-#pragma unroll
-        for (int j = 0; j < 5; j++) acc += c_edge_k[strength - 1][j] * s.dup[clip3(0, sz - 1, i - 2 + j)];
-        e[i + 1] = (uint16_t)max((acc + 8) >> 4, 0);
+// The record of one TU (see TuHead).
+__device__ void prep_tu(const IntraFrame& F, int log2sb, const av1g_intra_tu& t, TuRec& o) {
+    TuHead r{};
+    const int pl = t.plane, ssx = pl ? F.ssx : 0, ssy = pl ? F.ssy : 0;
+    const int W = c_txw_d[t.tx_size], H = c_txh_d[t.tx_size];
+    const int sx = t.x, sy = t.y;
+    const int max_x = F.planes[pl].w - 1, max_y = F.planes[pl].h - 1;
+    const int sbw = (1 << log2sb) >> ssx, sbh = (1 << log2sb) >> ssy;
+    const int lx = sx & (sbw - 1), ly = sy & (sbh - 1);
+    uint32_t recip = 0;
+    r.x = t.x;
+    r.y = t.y;
+    r.coff = (uint32_t)(copy_off(log2sb, F.ssx, F.ssy, pl) + ly * copy_pitch(log2sb, ssx) + lx);
+    r.dims = (uint8_t)((31 - __clz(W)) | (31 - __clz(H)) << 4);
+    r.plane = t.plane;
+    r.res = t.res.coeff_offset;
+    if (!(sx & 3)) r.where |= W_ALIGNED;
+    if (t.flags & AV1G_INTRA_RESIDUAL) r.bits |= R_RES;
+    if ((t.flags & AV1G_INTRA_CFL) && pl > 0) {
+        r.bits |= R_CFL;
+        const int cx = max((int)t.max_luma_w - (1 << F.ssx), 0), cy = max((int)t.max_luma_h - (1 << F.ssy), 0);
+        r.cx = (uint16_t)cx;
+        r.cy = (uint16_t)cy;
+        r.alpha = t.cfl_alpha;
+        const int x0 = (sx - lx) << ssx, y0 = (sy - ly) << ssy, sb = 1 << log2sb;
+        if (cx >= x0 && cy >= y0 && min((sx + W - 1) << ssx, cx) + ssx < x0 + sb &&
+            min((sy + H - 1) << ssy, cy) + ssy < y0 + sb && !(ssx && (cx & 1)))
+            r.where |= W_CFL;
     }
-    g.sync();
+    const int fim = (pl == 0 && t.filter_intra_mode < 5) ? t.filter_intra_mode : -1;
+    r.misc = (uint8_t)((fim >= 0 ? fim : 0) | (t.mode < 13 && fim < 0 ? t.interintra << 4 : 0));
+    r.ii_mode = t.interintra_mode;
+    r.stride = t.palette_stride;
+    r.map = t.mode == AV1G_INTRA_MODE_INTRABC ? (uint32_t)(uint16_t)t.mv[0] << 16 | (uint16_t)t.mv[1] : t.palette_map;
+    if (t.mode < 13) {
+        const bool ha = (t.flags & AV1G_INTRA_HAVE_ABOVE) && sy > 0;
+        const bool hl = (t.flags & AV1G_INTRA_HAVE_LEFT) && sx > 0;
+        const int ft = (t.flags & AV1G_INTRA_FILTER_TYPE) ? 1 : 0;
+        if (ha) r.bits |= R_ABOVE;
+        if (hl) r.bits |= R_LEFT;
+        // intra_predict_block_samples' edge limits (cdf.rs:17030-17075)
+        r.na = (uint16_t)(min(max_x, sx + ((t.flags & AV1G_INTRA_HAVE_ABOVE_RIGHT) ? 2 * W : W) - 1) - sx + 1);
+        r.nl = (uint16_t)(min(max_y, sy + ((t.flags & AV1G_INTRA_HAVE_BELOW_LEFT) ? 2 * H : H) - 1) - sy + 1);
+        int ea = W, el = H;
+        const bool copy_v = t.mode == 1 && t.angle_delta == 0, copy_h = t.mode == 2 && t.angle_delta == 0;
+        const bool dir = t.mode >= 1 && t.mode <= 8 && !copy_v && !copy_h;
+        if (dir) {
+            const int pa = c_mode_angle[t.mode] + t.angle_delta * 3;
+            auto dr = [](int k) { return k >= 0 && k < 90 ? c_dr[k] : (int16_t)0; };
+            r.dx = pa < 90 ? dr(pa) : (pa < 180 ? dr(180 - pa) : (int16_t)0);
+            r.dy = (pa >= 90 && pa < 180) ? dr(pa - 90) : (pa > 180 ? dr(270 - pa) : (int16_t)0);
+            r.cls = pa < 90 ? C_D1 : pa < 180 ? C_D2 : C_D3;
+            ea = pa < 90 ? W + H : (pa < 180 || fim >= 0) ? W : 0;
+            el = pa > 180 ? W + H : pa == 180 ? W + H : (pa >= 90 || fim >= 0) ? H : 0;
+            if ((t.flags & AV1G_INTRA_EDGE_FILTER) && pa != 90 && pa != 180) {
+                if (pa > 90 && pa < 180 && W + H >= 24) r.bits |= R_EDGE | R_CORNER;
+                r.fa = (uint16_t)(min(W, max_x - sx + 1) + (pa < 90 ? H : 0) + 1);
+                r.fl = (uint16_t)(min(H, max_y - sy + 1) + (pa > 180 ? W : 0) + 1);
+                const int sa = ha ? strength_sel(W, H, ft, pa - 90) : 0;
+                const int sl = hl ? strength_sel(W, H, ft, pa - 180) : 0;
+                r.strength = (uint8_t)(sa | sl << 4);
+                if (r.strength) r.bits |= R_EDGE;
+                if (upsample_sel(W, H, ft, pa - 90)) r.bits |= R_EDGE | R_UPA;
+                if (upsample_sel(W, H, ft, pa - 180)) r.bits |= R_EDGE | R_UPL;
+            }
+        } else if (copy_v) {
+            r.cls = C_V;
+            el = 0;
+        } else if (copy_h) {
+            r.cls = C_H;
+            ea = 0;
+        } else if (t.mode == 0) {
+            r.cls = C_DC;
+            if (!ha) ea = 0;
+            if (!hl) el = 0;
+        } else {
+            r.cls = t.mode == 9 ? C_SMOOTH : t.mode == 10 ? C_SMOOTH_V : t.mode == 11 ? C_SMOOTH_H : C_PAETH;
+        }
+        if (fim >= 0) {
+            r.cls = C_FI;
+            ea = max(ea, W);
+            el = max(el, H);
+        }
+        r.ea = (uint16_t)ea;
+        r.el = (uint16_t)el;
+        if (r.cls == C_DC && ea + el) recip = (uint32_t)(((1ull << 32) + ea + el - 1) / (ea + el));
+        // the copy holds the row above up to kIntraCopyExt samples past the
+        // superblock, and otherwise the superblock's own columns
+        const int wide = ly == 0 ? sbw + intra_copy_ext(sbw) : sbw;
+        if (lx + min(ea, (int)r.na) <= wide && ly + min(el, (int)r.nl) <= sbh) {
+            r.where |= W_COPY;
+            const bool a_ok = ha && r.na >= W, l_ok = hl && r.nl >= H;
+            const bool in_place = r.cls == C_V ? a_ok : r.cls == C_H ? l_ok
+                                : r.cls == C_DC ? (!ha || a_ok) && (!hl || l_ok)
+                                : (r.cls >= C_SMOOTH && r.cls <= C_PAETH) || (r.cls == C_FI && !(r.bits & R_EDGE)) ? a_ok && l_ok
+                                : false;
+            if (in_place && !(sx & 3)) r.where |= W_DIRECT;
+        }
+    } else if (t.mode == AV1G_INTRA_MODE_PALETTE) {
+        r.cls = C_PAL;
+    } else if (t.mode == AV1G_INTRA_MODE_INTRABC) {
+        r.cls = C_BC;
+    }
+    const bool cfl = r.bits & R_CFL, direct = r.where & W_DIRECT;
+    bool fast = W * H <= kSmallPx && (r.where & W_ALIGNED) && !(r.misc >> 4);
+    switch (r.cls) {
+        case C_NONE:
+        case C_PAL: fast = fast && !cfl; break;
+        case C_DC: fast = fast && direct && (!cfl || (r.where & W_CFL)); break;
+        case C_D1:
+        case C_D2:
+        case C_D3: fast = fast && !cfl && (r.where & W_COPY) && (r.bits & (R_ABOVE | R_LEFT)); break;
+        case C_BC: fast = false; break;
+        default: fast = fast && direct && !cfl; break;
+    }
+    if (fast) r.where |= W_FAST;
+    o.h = r;
+    for (int k = 0; k < 8; k++) o.colors[k] = t.palette_colors[k];
+    if (r.cls == C_DC) o.recip = recip;
 }
 
-// intra_edge_upsample (cdf.rs:2700), in parallel
-template <class G, class S>
-__device__ void edge_upsample(const G& g, S& s, uint16_t* e, int n, int bd) {
-    if (g.r == 0) {
-        s.dup[0] = e[1];
-        s.dup[1] = e[1];
-        s.dup[n + 2] = e[n + 1];
-    }
-    for (int i = g.r; i < n; i += G::N) s.dup[i + 2] = e[i + 2];
-    g.sync();
-    const int maxv = (1 << bd) - 1;
-    if (g.r == 0) e[0] = s.dup[0];
-    for (int i = g.r; i < n; i += G::N) {
-        int sum = -s.dup[i] + 9 * s.dup[i + 1] + 9 * s.dup[i + 2] - s.dup[i + 3];
-        int r = sum >= 0 ? (sum + 8) >> 4 : -(((-sum) + 8) >> 4);
-        e[2 * i + 1] = (uint16_t)clip3(0, maxv, r);
-        e[2 * i + 2] = (uint16_t)min((int)s.dup[i + 2], maxv);
-    }
-    g.sync();
-}
+// Scratch of one residual block.
+template <int PX>
+struct ResScr {
+    int buf[PX];
+};
 
 // Dequantize (dequantize_step1, cdf.rs:13655-13703) and inverse transform
 // (transform.rs:707-789) one TU's residual, stored as w*h int32 in sample
@@ -356,321 +539,716 @@ __device__ __forceinline__ void residual_task(const G& g, S& s, const IntraFrame
     residual_store<TX>(g, s, F, tu, cf, out);
 }
 
-// One TU: prediction (+ inter-intra blend, + CfL), then the residual, all on
-// the shared-memory copy of the superblock.
-template <int TX, class G, class S>
-__device__ void intra_tu(const G& g, S& s, const IntraFrame& F, const SbCtx& c, uint16_t* cache,
-                         const av1g_intra_tu* rec, Pool pool) {
-    const av1g_intra_tu t = *rec;
-    constexpr int W = kTxW[TX], H = kTxH[TX];
-    constexpr int LW = ilog2<W>(), LH = ilog2<H>();
-    const int tid = g.r;
-    const int pl = t.plane;
-    const PlaneDev& P = F.planes[pl];
-    const int hbd = F.hbd, bd = F.bd;
-    const int sx = t.x, sy = t.y;
-    const int cs = c.w[pl];
-    uint16_t* tp = cache + c.off[pl] + (sy - c.y0[pl]) * cs + (sx - c.x0[pl]);
-    const bool has_res = t.flags & AV1G_INTRA_RESIDUAL;
-    // a warp fetches its residual first, so that the latency overlaps the
-    // prediction (the CTA path reads it at the merge)
-    const int32_t* rp = pool.res + t.res.coeff_offset;
-    constexpr int KP = G::N == 32 ? (W * H + 31) / 32 : 1;
-    int rv[KP];
-    if constexpr (G::N == 32) {
-#pragma unroll
-        for (int q = 0; q < KP; q++) {
-            const int k = tid + q * 32;
-            rv[q] = (has_res && k < W * H) ? __ldg(rp + k) : 0;
-        }
+// ---- small TUs of the common kinds -------------------------------------------
+// What bounds a TU is latency: it is a chain of shared-memory round trips on
+// the wavefront's critical path, run by a single warp at the issue latency of
+// dependent instructions.  So all that does not depend on samples is worked
+// out ahead, while other groups run earlier levels (fast_decode): where each
+// lane's edge samples, filter taps, prediction taps, residual and destination
+// lie.  What is left (fast_run) is loads, a few multiplications and stores.
+
+struct Prog {
+    int cls, bits;
+    uint16_t* cp;       // the lane's first four samples in the copy
+    uint8_t* out;       // and in HBM
+    int cs, cstep, ostep;  // copy row pitch; from the first four samples to the second
+    int ok;             // bit 0 / 1: the first / second four exist; bit 2 / 3: and lie inside the plane
+    int4 r0, r1;        // their residual, 0 where none applies
+    // directional: per edge element of the lane, its place from the TU's first
+    // sample (low half, signed) and in the raw edge arrays (bits 16-23); its
+    // taps in them; coefficients and places after the edge filter
+    // DC: element places in src; recip and edge length in px
+    int two;            // directional: some lanes have a second edge element; copied edges: rows between the groups
+    int src[2];
+    uint32_t tap[2], flt[2];
+    // prediction taps of the two groups: places in the edge arrays, weights
+    uint32_t px[2], wt[2];
+    uint16_t* tp;       // the TU's first sample in the copy
+};
+
+// flt: k0 | k1 << 4 | k2 << 8 | (place << 16) | bits 13 / 14: tap -2 / -1 is
+// the corner | bit 15: upsampled (place holds the interpolated sample, the
+// next one the sample itself) | bit 31: the element exists
+__device__ __forceinline__ void fast_decode(Prog& d, const TuRec* rec, const IntraFrame& F, const SbCtx& c,
+                                            uint16_t* cache, const int32_t* __restrict__ pool, int lane) {
+    constexpr int E = WScr::E;
+    const TuHead t = rec->h;
+    const PlaneDev& P = F.planes[t.plane];
+    const int LW = t.dims & 15, LH = t.dims >> 4, W = 1 << LW, H = 1 << LH, Q = 1 << (LW + LH - 2);
+    const int hbd = F.hbd, cs = c.cs[t.plane];
+    const int q = lane < Q ? lane : 0, i = q >> (LW - 2), j = (q << 2) & (W - 1), rows = 128 >> LW;
+    uint16_t* tp = cache + t.coff;
+    d.cls = t.cls;
+    d.bits = t.bits;
+    d.tp = tp;
+    d.cp = tp + i * cs + j;
+    d.cs = cs;
+    d.cstep = rows * cs;
+    d.ostep = rows * P.stride;
+    d.out = P.p + (size_t)(t.y + i) * P.stride + ((size_t)(t.x + j) << hbd);
+    const bool a0 = lane < Q, a1 = lane + 32 < Q;
+    const bool in0 = a0 && t.y + i < P.h && t.x + j < P.w, in1 = a1 && t.y + i + rows < P.h && t.x + j < P.w;
+    d.ok = (a0 ? 1 : 0) | (a1 ? 2 : 0) | (in0 ? 4 : 0) | (in1 ? 8 : 0) | (Q > 32 ? 16 : 0);
+    d.r0 = d.r1 = make_int4(0, 0, 0, 0);
+    if (t.bits & R_RES) {
+        // chroma past the plane is not merged (luma is: chroma from luma reads it)
+        const int4* rp = reinterpret_cast<const int4*>(pool + t.res);
+        if (t.plane == 0 ? a0 : in0) d.r0 = __ldg(rp + lane);
+        if (t.plane == 0 ? a1 : in1) d.r1 = __ldg(rp + lane + 32);
     }
-    const int maxv = (1 << bd) - 1;
-    if (t.mode < 13) {
-        const int max_x = P.w - 1, max_y = P.h - 1;
-        auto rd = [&](int yy, int xx) { return rdp(F, c, cache, pl, min(yy, max_y), min(xx, max_x)); };
-        const bool ha = (t.flags & AV1G_INTRA_HAVE_ABOVE) && sy > 0;
-        const bool hl = (t.flags & AV1G_INTRA_HAVE_LEFT) && sx > 0;
-        const bool har = t.flags & AV1G_INTRA_HAVE_ABOVE_RIGHT, hbl = t.flags & AV1G_INTRA_HAVE_BELOW_LEFT;
-        const bool eief = t.flags & AV1G_INTRA_EDGE_FILTER;
-        const int ft = (t.flags & AV1G_INTRA_FILTER_TYPE) ? 1 : 0;
-        const int corner = ha && hl ? rd(sy - 1, sx - 1) : ha ? rd(sy - 1, sx) : hl ? rd(sy, sx - 1) : 1 << (bd - 1);
-        constexpr int span = W + H;
-        // edge arrays (intra_predict_block_samples, cdf.rs:17030-17075)
-        for (int i = tid; i < span; i += G::N) {
-            int a, l;
-            if (!ha && hl) a = rd(sy, sx - 1);
-            else if (!ha && !hl) a = (1 << (bd - 1)) - 1;
-            else a = rd(sy - 1, min(min(max_x, sx + (har ? 2 * W : W) - 1), sx + i));
-            if (!hl && ha) l = rd(sy - 1, sx);
-            else if (!hl && !ha) l = (1 << (bd - 1)) + 1;
-            else l = rd(min(min(max_y, sy + (hbl ? 2 * H : H) - 1), sy + i), sx - 1);
-            s.above[2 + i] = (uint16_t)a;
-            s.left[2 + i] = (uint16_t)l;
-        }
-        if (tid < 2) s.above[tid] = s.left[tid] = (uint16_t)corner;
-        g.sync();
-        const bool dir = t.mode >= 1 && t.mode <= 8;
-        const int pa = c_mode_angle[t.mode] + t.angle_delta * 3;
-        int ua = 0, ul = 0;
-        if (dir && eief && pa != 90 && pa != 180) {
-            if (pa > 90 && pa < 180 && span >= 24) {
-                if (tid == 0) {
-                    uint16_t fc = (uint16_t)((s.left[2] * 5 + s.above[1] * 6 + s.above[2] * 5 + 8) >> 4);
-                    s.above[1] = fc;
-                    s.left[1] = fc;
-                }
-                g.sync();
-            }
-            if (ha) edge_filter(g, s, s.above, min(W, max_x - sx + 1) + (pa < 90 ? H : 0) + 1, strength_sel(W, H, ft, pa - 90));
-            if (hl) edge_filter(g, s, s.left, min(H, max_y - sy + 1) + (pa > 180 ? W : 0) + 1, strength_sel(W, H, ft, pa - 180));
-            ua = upsample_sel(W, H, ft, pa - 90);
-            if (ua) edge_upsample(g, s, s.above, W + (pa < 90 ? H : 0), bd);
-            ul = upsample_sel(W, H, ft, pa - 180);
-            if (ul) edge_upsample(g, s, s.left, H + (pa > 180 ? W : 0), bd);
-        }
-        const uint16_t* A = s.above + 2;  // A[k] == AboveRow[k]
-        const uint16_t* Lc = s.left + 2;
-        const int fim = (pl == 0 && t.filter_intra_mode < 5) ? t.filter_intra_mode : -1;
-        // the intra half of an inter-intra block is blended as it is stored
-        // (only inside the plane: the side plane has the plane's extent)
-        auto put = [&](int i, int j, int v) {
-            if (t.interintra && sy + i < P.h && sx + j < P.w)
-                v = interintra_px<W, H>(F, t, i, j, v, ld_px(F.side[pl], hbd, sy + i, sx + j), maxv);
-            tp[i * cs + j] = (uint16_t)v;
-        };
-        if (fim >= 0) {
-            // predict_intra_recursive (cdf.rs:2145): 4x2 cells, wavefront over
-            // i2 + j4, reading earlier cells back from the copy
-            constexpr int W4 = W >> 2, H2 = H >> 1;
-            const int o = tid & 7, i1 = o >> 2, j1 = o & 3;
-            for (int d = 0; d < W4 + H2 - 1; d++) {
-                for (int bb = tid >> 3;; bb += G::N >> 3) {
-                    const int i2 = max(0, d - (W4 - 1)) + bb, j4 = d - i2;
-                    if (i2 >= H2 || j4 < 0) break;
-                    int p[7];
+    if (t.cls >= C_D1 && t.cls <= C_D3) {
+        const bool ha = t.bits & R_ABOVE, hl = t.bits & R_LEFT, edge = t.bits & R_EDGE;
+        const int ea = t.ea, total = ea + 1 + t.el;
+        d.two = total > 32;
 #pragma unroll
-                    for (int i = 0; i < 7; i++) {
-                        if (i < 5) {
-                            if (i2 == 0) p[i] = A[(j4 << 2) + i - 1];
-                            else if (j4 == 0 && i == 0) p[i] = Lc[(i2 << 1) - 1];
-                            else p[i] = tp[((i2 << 1) - 1) * cs + (j4 << 2) + i - 1];
-                        } else if (j4 == 0) {
-                            p[i] = Lc[(i2 << 1) + i - 5];
-                        } else {
-                            p[i] = tp[((i2 << 1) + i - 5) * cs + (j4 << 2) - 1];
-                        }
-                    }
-                    int acc = 0;
+        for (int x = 0; x < 2; x++) {
+            const int k = lane + 32 * x;
+            if (x && !d.two) break;
+            const bool above = k <= ea;
+            const int kk = above ? k : k - ea, p = kk - 1;  // position along its edge
+            const bool from_row = above ? ha : !hl;
+            const int xo = from_row ? (!above ? 0 : p < 0 ? (hl ? -1 : 0) : min(p, t.na - 1)) : -1;
+            const int yo = from_row ? -1 : above ? 0 : min(p, t.nl - 1);
+            const int bs = above ? 3 : E + 3;  // place of the edge's corner
+            const bool live = k < total;
+            d.src[x] = ((yo * cs + xo) & 0xffff) | (bs + kk) << 16;
+            if (!live) d.src[x] = 0;
+            d.flt[x] = live ? 0x80000000u : 0u;
+            if (edge) {
+                const int st = above ? t.strength & 15 : t.strength >> 4, sz = above ? t.fa : t.fl;
+                const int n = above ? ea : t.el;
+                const bool up = t.bits & (above ? R_UPA : R_UPL);
+                const int hi = up ? n : sz - 1;
+                const bool filt = st && kk && kk < sz;
+                const uint32_t tm2 = bs + max(kk - 2, 0), tm1 = bs + max(kk - 1, 0), tp1 = bs + min(kk + 1, max(hi, 0)),
+                               tp2 = bs + min(kk + 2, max(hi, 0));
+                d.tap[x] = tm2 | tm1 << 8 | tp1 << 16 | tp2 << 24;
+                const uint32_t k0 = filt && st == 3 ? 2 : 0, k1 = filt ? (st == 2 ? 5 : 4) : 0,
+                               k2 = filt ? (st == 1 ? 8 : st == 2 ? 6 : 4) : 16;
+                const bool ups = up && kk;
+                // position -1, or -2 of an upsampled edge, for the corner
+                const uint32_t place = ups ? bs + 2 * kk - 2 : bs + kk - (up ? 1 : 0);
+                d.flt[x] |= k0 | k1 << 4 | k2 << 8 | (kk <= 2 && kk ? 1u << 13 : 0) | (kk == 1 ? 1u << 14 : 0) |
+                            (ups ? 1u << 15 : 0) | place << 16;
+                if (!live) d.flt[x] = 0;
+            }
+        }
+        // prediction taps (predict_intra_directional, cdf.rs:2879-3010)
+        const int ua = t.bits & R_UPA ? 1 : 0, ul = t.bits & R_UPL ? 1 : 0;
 #pragma unroll
-                    for (int i = 0; i < 7; i++) acc += c_fi_taps[fim][(i1 << 2) + j1][i] * p[i];
-                    int v = acc >= 0 ? (acc + 8) >> 4 : -(((-acc) + 8) >> 4);
-                    tp[((i2 << 1) + i1) * cs + (j4 << 2) + j1] = (uint16_t)clip3(0, maxv, v);
+        for (int x = 0; x < 2; x++) {
+            if (x && Q <= 32) break;
+            const int ii = i + x * rows;
+            uint32_t pa = 0, wa = 0;
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                int at, sh;
+                if (t.cls == C_D2) {
+                    const int ix = ((j + e) << 6) - (ii + 1) * t.dx, bx = ix >> (6 - ua);
+                    const int iy = (ii << 6) - (j + e + 1) * t.dy, by = max(iy >> (6 - ul), -(1 << ul));
+                    const bool fa = bx >= -(1 << ua);
+                    at = fa ? 4 + bx : E + 4 + by;
+                    sh = ((fa ? ix << ua : iy << ul) >> 1) & 0x1F;
+                } else {
+                    const bool d3 = t.cls == C_D3;
+                    const int up = d3 ? ul : ua, maxb = (W + H - 1) << up;
+                    const int idx = ((d3 ? j + e : ii) + 1) * (d3 ? t.dy : t.dx);
+                    const int base = (idx >> (6 - up)) + ((d3 ? ii : j + e) << up);
+                    at = (d3 ? E + 4 : 4) + min(base, maxb);
+                    sh = base < maxb ? ((idx << up) >> 1) & 0x1F : 0;  // past the end: its last sample
                 }
-                g.sync();
+                pa |= (uint32_t)at << (8 * e);
+                wa |= (uint32_t)sh << (8 * e);
             }
-        } else if (t.mode == 0) {
-            // predict_intra_dc_pred (cdf.rs:1348)
-            long long part = 0;
-            for (int i = tid; i < span; i += G::N) {
-                if (hl && i < H) part += Lc[i];
-                if (ha && i < W) part += A[i];
+            d.px[x] = pa;
+            d.wt[x] = wa;
+        }
+    } else if (t.cls == C_DC) {
+        const int ea = t.ea, n = ea + t.el;
+#pragma unroll
+        for (int x = 0; x < 2; x++) {
+            const int k = lane + 32 * x;
+            d.src[x] = k < ea ? k - cs : k < n ? (k - ea) * cs - 1 : -0x8000;
+        }
+        d.px[0] = rec->recip;
+        d.px[1] = n;
+        if (t.bits & R_CFL) {
+            // luma of the lane's samples: the place of the first group's row
+            // and column, limits and alpha
+            d.tap[0] = t.x + j;
+            d.tap[1] = t.y + i;
+            d.flt[0] = t.cx | (uint32_t)t.cy << 16;
+            d.flt[1] = (uint32_t)(int)t.alpha;
+            d.wt[0] = LW + LH;
+            d.wt[1] = rows;
+        }
+    } else if (t.cls == C_PAL) {
+        const uint8_t* m = F.maps + t.map + i * t.stride + j;
+#pragma unroll
+        for (int x = 0; x < 2; x++) {
+            if (x && Q <= 32) break;
+            const uint8_t* mm = m + x * (a1 ? rows : 0) * t.stride;
+            uint32_t v[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) v[e] = rec->colors[mm[e] & 7];
+            d.px[x] = v[0] | v[1] << 16;
+            d.wt[x] = v[2] | v[3] << 16;
+        }
+    } else if (t.cls == C_FI) {
+        d.px[0] = t.misc & 7;
+        d.px[1] = W >> 2;
+        d.wt[0] = H >> 1;
+    } else {
+        d.px[0] = W;
+        d.px[1] = H;
+        d.wt[0] = j;
+        d.wt[1] = i;
+        d.two = rows;
+    }
+}
+
+__device__ __forceinline__ void fast_run(const Prog& d, WScr& s, const IntraFrame& F, const SbCtx& c,
+                                         const uint16_t* cache, const Tables& tb, int lane) {
+    constexpr int E = WScr::E;
+    const int maxv = (1 << F.bd) - 1, hbd = F.hbd, cs = d.cs;
+    const uint16_t* ed = s.raw;
+    int dc = 0, avg = 0;
+    if (d.cls >= C_D1 && d.cls <= C_D3) {
+        const int v0 = d.tp[(int16_t)(d.src[0] & 0xffff)];
+        const int v1 = d.two ? d.tp[(int16_t)(d.src[1] & 0xffff)] : 0;
+        if (d.flt[0] >> 31) s.raw[d.src[0] >> 16] = (uint16_t)v0;
+        if (d.two && d.flt[1] >> 31) s.raw[d.src[1] >> 16] = (uint16_t)v1;
+        if (lane == 0) s.raw[E + 3] = (uint16_t)v0;
+        __syncwarp();
+        if (d.bits & R_EDGE) {
+            // corner filter, intra_edge_filter (cdf.rs:2760) or
+            // intra_edge_upsample (cdf.rs:2700) of both edges at once
+            int fc = 0;
+            if (d.bits & R_CORNER) fc = (s.raw[E + 4] * 5 + s.raw[3] * 6 + s.raw[4] * 5 + 8) >> 4;
+#pragma unroll
+            for (int x = 0; x < 2; x++) {
+                if (x && !d.two) break;
+                const uint32_t ta = d.tap[x], fl = d.flt[x];
+                int m2 = s.raw[ta & 0xff], m1 = s.raw[(ta >> 8) & 0xff], p1 = s.raw[(ta >> 16) & 0xff], p2 = s.raw[ta >> 24];
+                int v = x ? v1 : v0;
+                if (d.bits & R_CORNER) {
+                    if (fl & (1u << 13)) m2 = fc;
+                    if (fl & (1u << 14)) m1 = fc;
+                    if (x == 0 && lane == 0) v = fc;
+                }
+                const bool up = fl & (1u << 15);
+                const int k0 = up ? -1 : (int)(fl & 15), k1 = up ? 9 : (int)(fl >> 4) & 15, k2 = up ? 9 : (int)(fl >> 8) & 31;
+                const int k3 = up ? -1 : k1, k4 = up ? 0 : k0;
+                const int f = clip3(0, maxv, (k0 * m2 + k1 * m1 + k2 * v + k3 * p1 + k4 * p2 + 8) >> 4);
+                const int place = (fl >> 16) & 0x7fff;
+                if (fl >> 31) {
+                    s.fin[place] = (uint16_t)f;
+                    if (up) s.fin[place + 1] = (uint16_t)v;
+                }
+                if (x == 0 && lane == 0) s.fin[E + (d.bits & R_UPL ? 2 : 3)] = (uint16_t)v;  // the left edge's corner
             }
-            long long sum = gsum(g, s, part);
-            unsigned avg;
-            if (hl && ha) avg = (unsigned)((sum + (span >> 1)) / span);
-            else if (hl) avg = min((unsigned)((sum + (H >> 1)) >> LH), (1u << bd) - 1);
-            else if (ha) avg = min((unsigned)((sum + (W >> 1)) >> LW), (1u << bd) - 1);
-            else avg = 1u << (bd - 1);
-            for (int k = tid; k < W * H; k += G::N) put(k >> LW, k & (W - 1), (int)avg);
-        } else {
-            const int dx = pa < 90 ? c_dr[pa] : (pa < 180 ? c_dr[180 - pa] : 0);
-            const int dy = (pa >= 90 && pa < 180) ? c_dr[pa - 90] : (pa > 180 ? c_dr[270 - pa] : 0);
-            const uint8_t* swx = sm_weights(LW);
-            const uint8_t* swy = sm_weights(LH);
-            for (int k = tid; k < W * H; k += G::N) {
-                int i = k >> LW, j = k & (W - 1);
-                int v;
-                if (t.mode == 1 && t.angle_delta == 0) {
-                    v = A[j];
-                } else if (t.mode == 2 && t.angle_delta == 0) {
-                    v = Lc[i];
-                } else if (dir) {
-                    // predict_intra_directional (cdf.rs:2879-3010)
-                    if (pa < 90) {
-                        int maxb = (W + H - 1) << ua;
-                        int idx = (i + 1) * dx;
-                        int base = (idx >> (6 - ua)) + j * (1 << ua);
-                        int sh = ((idx * (1 << ua)) >> 1) & 0x1F;
-                        v = base < maxb ? (A[base] * (32 - sh) + A[base + 1] * sh + 16) >> 5 : A[maxb];
-                    } else if (pa < 180) {
-                        int ix = (j << 6) - (i + 1) * dx;
-                        int bx = ix >> (6 - ua);
-                        if (bx >= -(1 << ua)) {
-                            int sh = ((ix * (1 << ua)) >> 1) & 0x1F;
-                            v = (A[bx] * (32 - sh) + A[bx + 1] * sh + 16) >> 5;
-                        } else {
-                            int iy = (i << 6) - (j + 1) * dy;
-                            int by = iy >> (6 - ul);
-                            int sh = ((iy * (1 << ul)) >> 1) & 0x1F;
-                            v = (Lc[by] * (32 - sh) + Lc[by + 1] * sh + 16) >> 5;
-                        }
+            ed = s.fin;
+            __syncwarp();
+        }
+    } else if (d.cls == C_DC) {
+        // predict_intra_dc_pred (cdf.rs:1348); a missing edge has length 0.
+        // The quotient by the reciprocal is exact: sum + n / 2 < 2^20, n <= 128.
+        int part = 0;
+        if (d.src[0] != -0x8000) part = d.tp[d.src[0]];
+        if (d.src[1] != -0x8000) part += d.tp[d.src[1]];
+        const unsigned n = d.px[1], sum = __reduce_add_sync(0xffffffffu, part);
+        dc = n == 0 ? (maxv + 1) >> 1 : __umulhi(sum + (n >> 1), d.px[0]);
+        if (d.bits & R_CFL) {
+            // predict_chroma_from_luma_into_curr_frame (cdf.rs:17256-17340)
+            const int ssx = F.ssx, ssy = F.ssy, ycs = c.cs[0];
+            const int cx = d.flt[0] & 0xffff, cy = d.flt[0] >> 16;
+            const uint16_t* Y = cache + c.off[0] - c.rect[0].y * ycs - c.rect[0].x;
+            part = 0;
+#pragma unroll 1
+            for (int x = 0; x < 2; x++) {
+                if (!((d.ok >> x) & 1)) break;
+                const uint16_t* yp = Y + min((int)(d.tap[1] + x * d.wt[1]) << ssy, cy) * ycs;
+                int v[4];
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const uint16_t* p = yp + min((int)(d.tap[0] + e) << ssx, cx);
+                    if (ssx) {
+                        uint32_t w = *reinterpret_cast<const uint32_t*>(p);  // two samples below 4096: no carry
+                        if (ssy) w += *reinterpret_cast<const uint32_t*>(p + ycs);
+                        v[e] = (int)((w & 0xffff) + (w >> 16)) << (2 - ssy);
                     } else {
-                        int maxb = (W + H - 1) << ul;
-                        int idx = (j + 1) * dy;
-                        int base = (idx >> (6 - ul)) + i * (1 << ul);
-                        int sh = ((idx * (1 << ul)) >> 1) & 0x1F;
-                        v = base < maxb ? (Lc[base] * (32 - sh) + Lc[base + 1] * sh + 16) >> 5 : Lc[maxb];
+                        v[e] = ssy ? (p[0] + p[ycs]) << 2 : p[0] << 3;
                     }
-                } else if (t.mode == 9) {  // SMOOTH (cdf.rs:2267)
-                    unsigned sp = swy[i] * A[j] + (256 - swy[i]) * Lc[H - 1] + swx[j] * Lc[i] + (256 - swx[j]) * A[W - 1];
-                    v = (int)((sp + 256) >> 9);
-                } else if (t.mode == 10) {  // SMOOTH_V
-                    v = (int)((swy[i] * A[j] + (256 - swy[i]) * Lc[H - 1] + 128) >> 8);
-                } else if (t.mode == 11) {  // SMOOTH_H
-                    v = (int)((swx[j] * Lc[i] + (256 - swx[j]) * A[W - 1] + 128) >> 8);
-                } else {  // PAETH (cdf.rs:2077)
-                    int base = A[j] + Lc[i] - corner;
-                    int pl_ = abs(base - Lc[i]), pt = abs(base - A[j]), ptl = abs(base - corner);
-                    v = (pl_ <= pt && pl_ <= ptl) ? Lc[i] : (pt <= ptl ? A[j] : corner);
+                    part += v[e];
                 }
-                put(i, j, v);
+                *reinterpret_cast<uint2*>(s.buf + 4 * lane + 128 * x) =
+                    make_uint2((uint32_t)v[0] | (uint32_t)v[1] << 16, (uint32_t)v[2] | (uint32_t)v[3] << 16);
+            }
+            const unsigned lsum = __reduce_add_sync(0xffffffffu, part);
+            avg = (int)((lsum + (1u << (d.wt[0] - 1))) >> d.wt[0]);
+        }
+    } else if (d.cls == C_FI) {
+        // predict_intra_recursive (cdf.rs:2145): 4x2 cells, wavefront over
+        // i2 + j4; eight lanes per cell, four lanes groups on a diagonal.  The
+        // edges lie in place around the block, so every cell reads the same way.
+        const int W4 = d.px[1], H2 = d.wt[0], o = lane & 7;
+        const uint2 tw = *reinterpret_cast<const uint2*>(tb.fi[d.px[0]][o]);
+        auto tap = [&](int q) { return (int)(int8_t)((q < 4 ? tw.x : tw.y) >> (8 * (q & 3))); };
+        const int w0 = tap(0), w1 = tap(1), w2 = tap(2), w3 = tap(3), w4 = tap(4), w5 = tap(5), w6 = tap(6);
+        const int oo = (o >> 2) * cs + (o & 3);
+#pragma unroll 1
+        for (int dd = 0; dd < W4 + H2 - 1; dd++) {
+#pragma unroll 1
+            for (int i2 = max(0, dd - (W4 - 1)) + (lane >> 3); i2 <= min(dd, H2 - 1); i2 += 4) {
+                uint16_t* cell = d.tp + (i2 << 1) * cs + ((dd - i2) << 2);
+                const uint16_t* up = cell - cs;
+                const int acc = w0 * up[-1] + w1 * up[0] + w2 * up[1] + w3 * up[2] + w4 * up[3] + w5 * cell[-1] +
+                                w6 * cell[cs - 1];
+                cell[oo] = (uint16_t)clip3(0, maxv, acc >= 0 ? (acc + 8) >> 4 : -(((-acc) + 8) >> 4));
+            }
+            __syncwarp();
+        }
+    }
+    int4 rv = d.r0;
+    uint16_t* cp = d.cp;
+    uint8_t* out = d.out;
+    uint32_t px = d.px[0], wt = d.wt[0];
+#pragma unroll 1
+    for (int x = 0;; x++) {
+        int v[4];
+        if (d.cls >= C_D1 && d.cls <= C_D3) {
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const uint16_t* a = ed + ((px >> (8 * e)) & 0xff);
+                const int lo = a[0], hi = a[1], w = (wt >> (8 * e)) & 0xff;
+                v[e] = lo + (((hi - lo) * w + 16) >> 5);
+            }
+        } else if (d.cls == C_DC) {
+#pragma unroll
+            for (int e = 0; e < 4; e++) v[e] = dc;
+            if ((d.bits & R_CFL) && ((d.ok >> (2 + x)) & 1)) {
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int al = (int)d.flt[1] * ((int)s.buf[4 * lane + 128 * x + e] - avg);
+                    const int sc = al >= 0 ? (al + 32) >> 6 : -(((-al) + 32) >> 6);
+                    v[e] = min(max(dc + sc, 0), maxv);
+                }
+            }
+        } else if (d.cls == C_PAL) {  // predict_palette (cdf.rs:11907); indices checked on the host
+            v[0] = px & 0xffff;
+            v[1] = px >> 16;
+            v[2] = wt & 0xffff;
+            v[3] = wt >> 16;
+        } else if (d.cls == C_FI || d.cls == C_NONE) {  // in the copy already
+            const uint2 w = *reinterpret_cast<const uint2*>(cp);
+            v[0] = w.x & 0xffff;
+            v[1] = w.x >> 16;
+            v[2] = w.y & 0xffff;
+            v[3] = w.y >> 16;
+        } else {
+            const int j = d.wt[0], i = d.wt[1] + (x ? d.two : 0);
+            const uint2 aw = *reinterpret_cast<const uint2*>(d.tp - cs + j);
+            const int l = d.tp[i * cs - 1];
+            v[0] = aw.x & 0xffff;
+            v[1] = aw.x >> 16;
+            v[2] = aw.y & 0xffff;
+            v[3] = aw.y >> 16;
+            if (d.cls == C_H) {
+#pragma unroll
+                for (int e = 0; e < 4; e++) v[e] = l;
+            } else if (d.cls == C_PAETH) {  // cdf.rs:2077
+                const int corner = d.tp[-cs - 1];
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int base = v[e] + l - corner;
+                    const int dl = abs(base - l), dt = abs(base - v[e]), dtl = abs(base - corner);
+                    v[e] = (dl <= dt && dl <= dtl) ? l : (dt <= dtl ? v[e] : corner);
+                }
+            } else if (d.cls != C_V) {  // SMOOTH (cdf.rs:2267), SMOOTH_V, SMOOTH_H
+                const int W = d.px[0], H = d.px[1];
+                const uint32_t wx = *reinterpret_cast<const uint32_t*>(tb.sm + W - 4 + j);
+                const int wy = tb.sm[H - 4 + i], ar = d.tp[W - 1 - cs], lb = d.tp[(H - 1) * cs - 1];
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int w = (wx >> (8 * e)) & 0xff;
+                    const int vv = wy * v[e] + (256 - wy) * lb, vh = w * l + (256 - w) * ar;
+                    v[e] = d.cls == C_SMOOTH ? (vv + vh + 256) >> 9 : ((d.cls == C_SMOOTH_V ? vv : vh) + 128) >> 8;
+                }
             }
         }
-        g.sync();
-    }
-    if (t.mode == AV1G_INTRA_MODE_PALETTE) {
-        // predict_palette (cdf.rs:11907); indices checked on the host
-        const uint8_t* m = F.maps + t.palette_map;
-        for (int k = tid; k < W * H; k += G::N) {
-            int i = k >> LW, j = k & (W - 1);
-            tp[i * cs + j] = rec->palette_colors[m[i * t.palette_stride + j]];
+        // curr_frame_step3_merge (cdf.rs:17398-17470): Clip1(pred + residual)
+        v[0] = __viaddmin_s32_relu(v[0], rv.x, maxv);
+        v[1] = __viaddmin_s32_relu(v[1], rv.y, maxv);
+        v[2] = __viaddmin_s32_relu(v[2], rv.z, maxv);
+        v[3] = __viaddmin_s32_relu(v[3], rv.w, maxv);
+        // the final samples to the copy and to HBM: other superblocks read
+        // them once this level is published
+        const uint2 pk = make_uint2(__byte_perm(v[0], v[1], 0x5410), __byte_perm(v[2], v[3], 0x5410));
+        if ((d.ok >> x) & 1) *reinterpret_cast<uint2*>(cp) = pk;
+        if ((d.ok >> (2 + x)) & 1) {
+            if (hbd) *reinterpret_cast<uint2*>(out) = pk;
+            else *reinterpret_cast<uint32_t*>(out) = __byte_perm(pk.x, pk.y, 0x6420);
         }
+        if (x || !(d.ok & 16)) break;
+        rv = d.r1;
+        cp += d.cstep;
+        out += d.ostep;
+        px = d.px[1];
+        wt = d.wt[1];
+    }
+}
+
+// One TU: the edges, the prediction (+ inter-intra blend, + CfL), the residual,
+// all on the shared-memory copy of the superblock, and its final samples to
+// HBM.  A thread computes four horizontally adjacent samples at a time (every
+// TU is at least four wide).
+//
+// The general form, for any TU: the large ones (a group of warps each) and what
+// fast_decode does not take (edges past the copy or cut off by the frame's edge,
+// inter-intra blocks, intra block copies, unaligned positions).  One body
+// that takes the size at run time keeps the code inside the instruction cache,
+// which a body per transform size missed on almost every TU.
+template <class G, class S>
+__device__ __forceinline__ void run_tu(const G& g, S& s, const TuRec* rec, const IntraFrame& F, const SbCtx& c,
+                                       uint16_t* cache, const Tables& tb, const int32_t* __restrict__ pool) {
+    const TuHead t = rec->h;
+    const int tid = g.r, pl = t.plane, bd = F.bd, hbd = F.hbd, maxv = (1 << bd) - 1;
+    const int LW = t.dims & 15, LH = t.dims >> 4, W = 1 << LW, H = 1 << LH, Q = 1 << (LW + LH - 2);
+    const PlaneDev P = F.planes[pl];
+    const int sx = t.x, sy = t.y, cs = c.cs[pl], wlim = P.w - sx, hlim = P.h - sy;
+    uint16_t* tp = cache + t.coff;
+    uint8_t* dst = P.p + (size_t)sy * P.stride + ((size_t)sx << hbd);
+    constexpr int E = S::E;
+    // A[k] == AboveRow[k], Lc[k * ls] == LeftCol[k]
+    const uint16_t* A = tp - cs;
+    const uint16_t* Lc = tp - 1;
+    int ls = cs;
+    if (t.cls >= C_DC && t.cls <= C_FI && !(t.where & W_DIRECT)) {
+        // edge arrays (intra_predict_block_samples, cdf.rs:17030-17075)
+        const bool ha = t.bits & R_ABOVE, hl = t.bits & R_LEFT;
+        const int ea = t.ea, total = ea + 1 + t.el;
+        const int mid = 1 << (bd - 1);
+        for (int k = tid; k < total; k += G::N) {
+            const bool above = k <= ea;
+            const int i = above ? k - 1 : k - ea - 1;
+            int v;
+            // a missing row repeats the left column's first sample, a missing column the row's
+            const bool from_row = above ? ha : !hl;
+            const int xo = from_row ? (!above ? 0 : i < 0 ? (hl ? -1 : 0) : min(i, t.na - 1)) : -1;
+            const int yo = from_row ? -1 : above ? 0 : min(i, t.nl - 1);
+            if (!ha && !hl) v = above ? (i < 0 ? mid : mid - 1) : mid + 1;
+            else if (t.where & W_COPY) v = tp[yo * cs + xo];
+            else v = rdp(F, c, cache, pl, sy + yo, sx + xo);
+            s.raw[(above ? 4 : E + 4) + i] = (uint16_t)v;
+            if (k == 0) s.raw[E + 3] = (uint16_t)v;
+        }
+        A = s.raw + 4;
+        Lc = s.raw + E + 4;
+        ls = 1;
         g.sync();
-    } else if (t.mode == AV1G_INTRA_MODE_INTRABC) {
+        if (t.bits & R_EDGE) {
+            // corner filter, intra_edge_filter (cdf.rs:2760) or
+            // intra_edge_upsample (cdf.rs:2700) of both edges at once
+            const int nA = ea + 1, nT = nA + t.el + 1;
+            int fc = s.raw[3];
+            if (t.bits & R_CORNER) fc = (s.raw[E + 4] * 5 + fc * 6 + s.raw[4] * 5 + 8) >> 4;
+            for (int k = tid; k < nT; k += G::N) {
+                const bool left = k >= nA;
+                const int kk = left ? k - nA : k;  // position kk - 1
+                const uint16_t* R = s.raw + (left ? E + 3 : 3);
+                uint16_t* D = s.fin + (left ? E + 3 : 3);
+                if (t.bits & (left ? R_UPL : R_UPA)) {
+                    const int n = left ? t.el : ea;
+                    if (kk == 0) {
+                        D[-1] = R[0];
+                    } else {
+                        const int sum = -R[max(kk - 2, 0)] + 9 * R[kk - 1] + 9 * R[kk] - R[min(kk + 1, n)];
+                        D[2 * kk - 2] = (uint16_t)clip3(0, maxv, (sum + 8) >> 4);
+                        D[2 * kk - 1] = (uint16_t)min((int)R[kk], maxv);
+                    }
+                } else {
+                    const int st = left ? t.strength >> 4 : t.strength & 15, sz = left ? t.fl : t.fa;
+                    int v = kk ? R[kk] : fc;
+                    if (st && kk && kk < sz) {
+                        const int k0 = st == 3 ? 2 : 0, k1 = st == 2 ? 5 : 4, k2 = st == 1 ? 8 : st == 2 ? 6 : 4;
+                        auto tap = [&](int q) { return q <= 0 ? fc : (int)R[min(q, sz - 1)]; };
+                        v = (k0 * (tap(kk - 2) + tap(kk + 2)) + k1 * (tap(kk - 1) + tap(kk + 1)) + k2 * v + 8) >> 4;
+                    }
+                    D[kk] = (uint16_t)v;
+                }
+            }
+            A = s.fin + 4;
+            Lc = s.fin + E + 4;
+            g.sync();
+        }
+    }
+    int dc = 0;
+    if (t.cls == C_DC) {
+        // predict_intra_dc_pred (cdf.rs:1348); a missing edge has length 0
+        int part = 0;
+        for (int i = tid; i < t.ea + t.el; i += G::N) part += i < t.ea ? A[i] : Lc[(i - t.ea) * ls];
+        const unsigned n = t.ea + t.el, sum = gsum(g, s, part);
+        // the quotient by the reciprocal is exact: sum + n / 2 < 2^20, n <= 128
+        dc = n == 0 ? 1 << (bd - 1) : __umulhi(sum + (n >> 1), rec->recip);
+    } else if (t.cls == C_FI) {
+        // predict_intra_recursive (cdf.rs:2145): 4x2 cells, wavefront over
+        // i2 + j4, reading earlier cells back from the copy
+        const int W4 = W >> 2, H2 = H >> 1, o = tid & 7, i1 = o >> 2, j1 = o & 3;
+        const uint2 tw = *reinterpret_cast<const uint2*>(tb.fi[t.misc & 7][o]);
+        auto tap = [&](int i) { return (int)(int8_t)((i < 4 ? tw.x : tw.y) >> (8 * (i & 3))); };
+        for (int dd = 0; dd < W4 + H2 - 1; dd++) {
+            for (int bb = tid >> 3;; bb += G::N >> 3) {
+                const int i2 = max(0, dd - (W4 - 1)) + bb, j4 = dd - i2;
+                if (i2 >= H2 || j4 < 0) break;
+                const uint16_t* up = i2 == 0 ? A + (j4 << 2) : tp + ((i2 << 1) - 1) * cs + (j4 << 2);
+                const int ps = j4 == 0 ? ls : cs;
+                const uint16_t* lf = j4 == 0 ? Lc + (i2 << 1) * ls : tp + (i2 << 1) * cs + (j4 << 2) - 1;
+                int acc = tap(0) * (j4 == 0 && i2 > 0 ? lf[-ps] : up[-1]);
+#pragma unroll
+                for (int i = 1; i < 5; i++) acc += tap(i) * up[i - 1];
+                acc += tap(5) * lf[0] + tap(6) * lf[ps];
+                const int v = acc >= 0 ? (acc + 8) >> 4 : -(((-acc) + 8) >> 4);
+                tp[((i2 << 1) + i1) * cs + (j4 << 2) + j1] = (uint16_t)clip3(0, maxv, v);
+            }
+            g.sync();
+        }
+    } else if (t.cls == C_BC) {
         // predict_intrabc_leaf_into_curr_frame (cdf.rs:19235): BILINEAR
         // block_inter_prediction from the pre-filter plane at unit scale,
         // start = (x << 10) + (((2 * mv) >> ss) << 6) + 32, clamped to the
         // mi-padded plane (the reference's window clamp is the same set).
         // The whole block is predicted before any of it is stored.
         const int pss_x = pl ? F.ssx : 0, pss_y = pl ? F.ssy : 0;
-        const int stx = (sx << 10) + ((2 * t.mv[1]) >> pss_x) * 64 + 32;
-        const int sty = (sy << 10) + ((2 * t.mv[0]) >> pss_y) * 64 + 32;
-        const int r0 = bd == 12 ? 5 : 3, r1 = bd == 12 ? 9 : 11;
+        const int stx = (sx << 10) + ((2 * (int16_t)(t.map & 0xffff)) >> pss_x) * 64 + 32;
+        const int sty = (sy << 10) + ((2 * (int16_t)(t.map >> 16)) >> pss_y) * 64 + 32;
+        const int b0 = bd == 12 ? 5 : 3, b1 = bd == 12 ? 9 : 11;
         const int hph = (stx >> 6) & 15, vph = (sty >> 6) & 15;
+#pragma unroll 1
         for (int k = tid; k < W * H; k += G::N) {
-            int i = k >> LW, j = k & (W - 1);
-            int xi = ((stx >> 10) + j) - 3, yi = ((sty >> 10) + i) - 3;
+            const int i = k >> LW, j = k & (W - 1);
+            const int xi = ((stx >> 10) + j) - 3, yi = ((sty >> 10) + i) - 3;
             int acc = 0;
+#pragma unroll 1
             for (int tt = 0; tt < 8; tt++) {
-                int vc = c_subpel[3][vph][tt];
+                const int vc = c_subpel[3][vph][tt];
                 if (!vc) continue;
-                int yy = min(max(yi + tt, 0), P.h - 1);
+                const int yy = min(max(yi + tt, 0), P.h - 1);
                 int hsum = 0;
+#pragma unroll 1
                 for (int u = 0; u < 8; u++) {
-                    int hc = c_subpel[3][hph][u];
+                    const int hc = c_subpel[3][hph][u];
                     if (hc) hsum += hc * rdp(F, c, cache, pl, yy, min(max(xi + u, 0), P.w - 1));
                 }
-                acc += vc * ((hsum + ((1 << r0) >> 1)) >> r0);
+                acc += vc * ((hsum + ((1 << b0) >> 1)) >> b0);
             }
-            s.buf[k] = min(max((acc + (1 << (r1 - 1))) >> r1, 0), maxv);
+            s.buf[k] = (uint16_t)min(max((acc + (1 << (b1 - 1))) >> b1, 0), maxv);
         }
         g.sync();
-        for (int k = tid; k < W * H; k += G::N) tp[(k >> LW) * cs + (k & (W - 1))] = (uint16_t)s.buf[k];
+        for (int k = tid; k < W * H; k += G::N) tp[(k >> LW) * cs + (k & (W - 1))] = s.buf[k];
         g.sync();
     }
-    if ((t.flags & AV1G_INTRA_CFL) && pl > 0) {
+    int cfl_avg = 0;
+    if (t.bits & R_CFL) {
         // predict_chroma_from_luma_into_curr_frame (cdf.rs:17256-17340).  The
         // block's luma transforms may run past the mi-grid plane; their
         // samples there stay in the superblock's staged copy (the reference's
         // LumaOverhang side store, cdf.rs:15938, read at cdf.rs:17292-17305),
         // which spans the whole superblock.  Luma neither in the plane nor in
         // that copy reads as 0.
-        const PlaneDev& Y = F.planes[0];
         const int ssx = F.ssx, ssy = F.ssy;
-        const int cx = max((int)t.max_luma_w - (1 << ssx), 0), cy = max((int)t.max_luma_h - (1 << ssy), 0);
-        long long part = 0;
-        for (int k = tid; k < W * H; k += G::N) {
-            int i = k >> LW, j = k & (W - 1);
-            int ly = min((sy + i) << ssy, cy), lx = min((sx + j) << ssx, cx);
-            int acc = 0;
-            for (int ddy = 0; ddy <= ssy; ddy++)
-                for (int ddx = 0; ddx <= ssx; ddx++) {
-                    int yy = ly + ddy, xx = lx + ddx;
-                    const bool staged = (unsigned)(yy - c.y0[0]) < (unsigned)c.h[0] &&
-                                        (unsigned)(xx - c.x0[0]) < (unsigned)c.w[0];
-                    acc += (staged || (yy < Y.h && xx < Y.w)) ? rdp(F, c, cache, 0, yy, xx) : 0;
-                }
-            int v = acc << (3 - ssx - ssy);
-            s.buf[k] = v;
-            part += v;
-        }
-        long long sum = gsum(g, s, part);
-        long long half = 1LL << (LW + LH - 1);
-        long long avg = sum >= 0 ? (sum + half) >> (LW + LH) : -(((-sum) + half) >> (LW + LH));
-        for (int k = tid; k < W * H; k += G::N) {
-            int i = k >> LW, j = k & (W - 1);
-            if (sy + i >= P.h || sx + j >= P.w) continue;
-            long long d = (long long)t.cfl_alpha * (s.buf[k] - avg);
-            long long sc = d >= 0 ? (d + 32) >> 6 : -(((-d) + 32) >> 6);
-            uint16_t& px = tp[i * cs + j];
-            px = (uint16_t)min(max((long long)px + sc, 0LL), (long long)maxv);
-        }
-        g.sync();
-    }
-    if (has_res) {
-        // curr_frame_step3_merge (cdf.rs:17398-17470): Clip1(pred + residual);
-        // luma past the plane is merged too, in the staged copy only (the
-        // overhang chroma from luma reads)
+        int part = 0;
+        if (t.where & W_CFL) {
+            const uint16_t* Y = cache + c.off[0] - c.rect[0].y * c.cs[0] - c.rect[0].x;
+            const int ycs = c.cs[0];
+#pragma unroll 1
+            for (int q = tid; q < Q; q += G::N) {
+                const int i = q >> (LW - 2), j = (q << 2) & (W - 1);
+                const uint16_t* yp = Y + min((sy + i) << ssy, (int)t.cy) * ycs;
+                int v[4];
 #pragma unroll
-        for (int q = 0; q < (G::N == 32 ? KP : (W * H + G::N - 1) / G::N); q++) {
-            const int k = tid + q * G::N;
-            if (k >= W * H) break;
-            const int i = k >> LW, j = k & (W - 1);
-            if (pl != 0 && (sy + i >= P.h || sx + j >= P.w)) continue;
-            int v;
-            if constexpr (G::N == 32) v = rv[q];
-            else v = __ldg(rp + k);
-            uint16_t& px = tp[i * cs + j];
-            px = (uint16_t)min(max((int)px + v, 0), maxv);
+                for (int e = 0; e < 4; e++) {
+                    const uint16_t* p = yp + min((sx + j + e) << ssx, (int)t.cx);
+                    if (ssx) {
+                        uint32_t w = *reinterpret_cast<const uint32_t*>(p);  // two samples below 4096: no carry
+                        if (ssy) w += *reinterpret_cast<const uint32_t*>(p + ycs);
+                        v[e] = (int)((w & 0xffff) + (w >> 16)) << (2 - ssy);
+                    } else {
+                        v[e] = ssy ? (p[0] + p[ycs]) << 2 : p[0] << 3;
+                    }
+                    part += v[e];
+                }
+                *reinterpret_cast<uint2*>(s.buf + 4 * q) =
+                    make_uint2((uint32_t)v[0] | (uint32_t)v[1] << 16, (uint32_t)v[2] | (uint32_t)v[3] << 16);
+            }
+        } else {
+            const PlaneDev& Y = F.planes[0];
+            const int4 yr = c.rect[0];
+#pragma unroll 1
+            for (int k = tid; k < W * H; k += G::N) {
+                const int i = k >> LW, j = k & (W - 1);
+                const int ly = min((sy + i) << ssy, (int)t.cy), lx = min((sx + j) << ssx, (int)t.cx);
+                int acc = 0;
+                for (int ddy = 0; ddy <= ssy; ddy++)
+                    for (int ddx = 0; ddx <= ssx; ddx++) {
+                        const int yy = ly + ddy, xx = lx + ddx;
+                        const bool staged =
+                            (unsigned)(yy - yr.y) < (unsigned)yr.w && (unsigned)(xx - yr.x) < (unsigned)yr.z;
+                        acc += (staged || (yy < Y.h && xx < Y.w)) ? rdp(F, c, cache, 0, yy, xx) : 0;
+                    }
+                const int v = acc << (3 - ssx - ssy);  // at most 4 * 4095 * 2
+                s.buf[k] = (uint16_t)v;
+                part += v;
+            }
         }
+        const int sum = gsum(g, s, part);  // at most 4096 * 32760, never negative
+        cfl_avg = (int)(((unsigned)sum + (1u << (LW + LH - 1))) >> (LW + LH));
         g.sync();
     }
-    // the TU's final samples to HBM: other superblocks read them once this
-    // level is published
-    for (int k = tid; k < W * H; k += G::N) {
-        const int i = k >> LW, j = k & (W - 1);
-        if (sy + i < P.h && sx + j < P.w) st_px(P, hbd, sy + i, sx + j, tp[i * cs + j]);
-    }
-}
-
-__device__ void run_small(const WarpG& g, WScr& s, const IntraFrame& F, const SbCtx& c, uint16_t* cache,
-                          const av1g_intra_tu* rec, Pool pool) {
-    switch (rec->tx_size) {
-        case 0: intra_tu<0>(g, s, F, c, cache, rec, pool); break;
-        case 1: intra_tu<1>(g, s, F, c, cache, rec, pool); break;
-        case 2: intra_tu<2>(g, s, F, c, cache, rec, pool); break;
-        case 5: intra_tu<5>(g, s, F, c, cache, rec, pool); break;
-        case 6: intra_tu<6>(g, s, F, c, cache, rec, pool); break;
-        case 7: intra_tu<7>(g, s, F, c, cache, rec, pool); break;
-        case 8: intra_tu<8>(g, s, F, c, cache, rec, pool); break;
-        case 13: intra_tu<13>(g, s, F, c, cache, rec, pool); break;
-        case 14: intra_tu<14>(g, s, F, c, cache, rec, pool); break;
-        case 15: intra_tu<15>(g, s, F, c, cache, rec, pool); break;
-        default: intra_tu<16>(g, s, F, c, cache, rec, pool); break;
-    }
-}
-
-__device__ void run_large(const CtaG& g, CScr& s, const IntraFrame& F, const SbCtx& c, uint16_t* cache,
-                          const av1g_intra_tu* rec, Pool pool) {
-    switch (rec->tx_size) {
-        case 3: intra_tu<3>(g, s, F, c, cache, rec, pool); break;
-        case 4: intra_tu<4>(g, s, F, c, cache, rec, pool); break;
-        case 9: intra_tu<9>(g, s, F, c, cache, rec, pool); break;
-        case 10: intra_tu<10>(g, s, F, c, cache, rec, pool); break;
-        case 11: intra_tu<11>(g, s, F, c, cache, rec, pool); break;
-        case 12: intra_tu<12>(g, s, F, c, cache, rec, pool); break;
-        case 17: intra_tu<17>(g, s, F, c, cache, rec, pool); break;
-        default: intra_tu<18>(g, s, F, c, cache, rec, pool); break;
+    const int ii = t.misc >> 4;
+    const int4* rp = reinterpret_cast<const int4*>(pool + t.res);
+#pragma unroll 1
+    for (int q = tid; q < Q; q += G::N) {
+        const int i = q >> (LW - 2), j = (q << 2) & (W - 1);
+        int4 rv = make_int4(0, 0, 0, 0);
+        if (t.bits & R_RES) rv = __ldg(rp + q);
+        uint16_t* cp = tp + i * cs + j;
+        int v[4];
+        switch (t.cls) {
+            case C_DC:
+#pragma unroll
+                for (int e = 0; e < 4; e++) v[e] = dc;
+                break;
+            case C_H:
+#pragma unroll
+                for (int e = 0; e < 4; e++) v[e] = Lc[i * ls];
+                break;
+            case C_V:
+            case C_SMOOTH:
+            case C_SMOOTH_V:
+            case C_SMOOTH_H:
+            case C_PAETH: {
+                const uint2 aw = *reinterpret_cast<const uint2*>(A + j);
+                const int a[4] = {(int)(aw.x & 0xffff), (int)(aw.x >> 16), (int)(aw.y & 0xffff), (int)(aw.y >> 16)};
+                if (t.cls == C_V) {
+#pragma unroll
+                    for (int e = 0; e < 4; e++) v[e] = a[e];
+                    break;
+                }
+                const int l = Lc[i * ls];
+                if (t.cls == C_PAETH) {  // cdf.rs:2077
+                    const int corner = A[-1];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const int base = a[e] + l - corner;
+                        const int dl = abs(base - l), dt = abs(base - a[e]), dtl = abs(base - corner);
+                        v[e] = (dl <= dt && dl <= dtl) ? l : (dt <= dtl ? a[e] : corner);
+                    }
+                    break;
+                }
+                // SMOOTH (cdf.rs:2267), SMOOTH_V, SMOOTH_H
+                const uint32_t wx = *reinterpret_cast<const uint32_t*>(tb.sm + W - 4 + j);
+                const int wy = tb.sm[H - 4 + i], ar = A[W - 1], lb = Lc[(H - 1) * ls];
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int w = (wx >> (8 * e)) & 0xff;
+                    const int vv = wy * a[e] + (256 - wy) * lb, vh = w * l + (256 - w) * ar;
+                    v[e] = t.cls == C_SMOOTH ? (vv + vh + 256) >> 9 : ((t.cls == C_SMOOTH_V ? vv : vh) + 128) >> 8;
+                }
+                break;
+            }
+            case C_D1:
+            case C_D3: {
+                // predict_intra_directional (cdf.rs:2879-3010) along one edge
+                const bool d3 = t.cls == C_D3;
+                const uint16_t* edge = d3 ? Lc : A;
+                const int up = t.bits & (d3 ? R_UPL : R_UPA) ? 1 : 0, maxb = (W + H - 1) << up;
+                const int step = d3 ? t.dy : t.dx;
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int idx = ((d3 ? j + e : i) + 1) * step;
+                    const int base = (idx >> (6 - up)) + ((d3 ? i : j + e) << up);
+                    const int sh = ((idx << up) >> 1) & 0x1F;
+                    v[e] = base < maxb ? (edge[base] * (32 - sh) + edge[base + 1] * sh + 16) >> 5 : edge[maxb];
+                }
+                break;
+            }
+            case C_D2: {
+                const int ua = t.bits & R_UPA ? 1 : 0, ul = t.bits & R_UPL ? 1 : 0;
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int ix = ((j + e) << 6) - (i + 1) * t.dx, bx = ix >> (6 - ua);
+                    const int iy = (i << 6) - (j + e + 1) * t.dy, by = max(iy >> (6 - ul), -(1 << ul));
+                    const bool fa = bx >= -(1 << ua);
+                    const uint16_t* ed = fa ? A + bx : Lc + by;
+                    const int sh = ((fa ? ix << ua : iy << ul) >> 1) & 0x1F;
+                    v[e] = (ed[0] * (32 - sh) + ed[1] * sh + 16) >> 5;
+                }
+                break;
+            }
+            case C_PAL: {  // predict_palette (cdf.rs:11907); indices checked on the host
+                const uint8_t* m = F.maps + t.map + i * t.stride + j;
+#pragma unroll
+                for (int e = 0; e < 4; e++) v[e] = rec->colors[m[e] & 7];
+                break;
+            }
+            default:  // in the copy already: filter intra, intra block copy, no prediction
+#pragma unroll
+                for (int e = 0; e < 4; e++) v[e] = cp[e];
+                break;
+        }
+        const bool row_in = i < hlim;
+        if (ii) {
+            // the intra half of an inter-intra block is blended as it is stored
+            // (only inside the plane: the side plane has the plane's extent)
+#pragma unroll 1
+            for (int e = 0; e < 4; e++)
+                if (row_in && j + e < wlim) {
+                    const int w = interintra_px(F, t, ii, i, j + e, e == 0 ? v[0] : e == 1 ? v[1] : e == 2 ? v[2] : v[3],
+                                                ld_px(F.side[pl], hbd, sy + i, sx + j + e), maxv);
+                    if (e == 0) v[0] = w;
+                    else if (e == 1) v[1] = w;
+                    else if (e == 2) v[2] = w;
+                    else v[3] = w;
+                }
+        }
+        if (t.bits & R_CFL) {
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const int al = t.alpha * ((int)s.buf[4 * q + e] - cfl_avg);
+                const int sc = al >= 0 ? (al + 32) >> 6 : -(((-al) + 32) >> 6);
+                if (row_in && j + e < wlim) v[e] = min(max(v[e] + sc, 0), maxv);
+            }
+        }
+        if (t.bits & R_RES) {
+            // curr_frame_step3_merge (cdf.rs:17398-17470): Clip1(pred + residual);
+            // luma past the plane is merged too, in the staged copy only (the
+            // overhang chroma from luma reads)
+            const int r[4] = {rv.x, rv.y, rv.z, rv.w};
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+                if (pl == 0 || (row_in && j + e < wlim)) v[e] = min(max(v[e] + r[e], 0), maxv);
+        }
+        // the final samples to the copy and to HBM: other superblocks read
+        // them once this level is published.  Plane widths are multiples of
+        // four, so an aligned group lies wholly inside or outside the plane.
+        uint8_t* out = dst + (size_t)i * P.stride + (j << hbd);
+        if (t.where & W_ALIGNED) {
+            const uint2 pk = make_uint2((uint32_t)v[0] | (uint32_t)v[1] << 16, (uint32_t)v[2] | (uint32_t)v[3] << 16);
+            *reinterpret_cast<uint2*>(cp) = pk;
+            if (row_in && j < wlim) {
+                if (hbd) *reinterpret_cast<uint2*>(out) = pk;
+                else *reinterpret_cast<uint32_t*>(out) = __byte_perm(pk.x, pk.y, 0x6420);
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                cp[e] = (uint16_t)v[e];
+                if (row_in && j + e < wlim) {
+                    if (hbd) reinterpret_cast<uint16_t*>(out)[e] = (uint16_t)v[e];
+                    else out[e] = (uint8_t)v[e];
+                }
+            }
+        }
     }
 }
 
@@ -685,39 +1263,70 @@ __device__ __forceinline__ long long gtimer() {
     return t;
 }
 
-// The superblock copy <-> HBM, two samples per thread (plane widths are even,
-// superblock origins and row pitches keep the pairs aligned).
-template <bool LOAD>
-__device__ void move_sb(const IntraFrame& F, const SbCtx& c, uint16_t* cache) {
+// Four samples at column x of a row, as u16 pairs.
+__device__ __forceinline__ uint2 ld_quad(const uint8_t* row, int hbd, int x) {
+    if (hbd) return __ldcg(reinterpret_cast<const uint2*>(row + 2 * x));
+    const uint32_t u = __ldcg(reinterpret_cast<const uint32_t*>(row + x));
+    return make_uint2(__byte_perm(u, 0u, 0x4140), __byte_perm(u, 0u, 0x4342));
+}
+
+// HBM -> the superblock's area of the copy, four samples per thread (plane
+// widths, superblock origins and row pitches are multiples of four samples).
+__device__ void load_area(const IntraFrame& F, const SbCtx& c, uint16_t* cache) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int p = 0; p < F.np; p++) {
         const PlaneDev& P = F.planes[p];
-        const int rows = min(c.h[p], P.h - c.y0[p]), pairs = min(c.w[p], P.w - c.x0[p]) >> 1;
+        const int4 r = c.rect[p];
+        const int rows = min(r.w, P.h - r.y), quads = min(r.z, P.w - r.x) >> 2;
         uint16_t* cp = cache + c.off[p];
-        for (int r = warp; r < rows; r += kNW) {
-            uint8_t* row = P.p + (size_t)(c.y0[p] + r) * P.stride;
-            uint16_t* crow = cp + r * c.w[p];
-            for (int q = lane; q < pairs; q += 32) {
-                if (F.hbd) {
-                    uint32_t* g = reinterpret_cast<uint32_t*>(row) + (c.x0[p] >> 1) + q;
-                    if (LOAD) {
-                        const uint32_t v = *g;
-                        crow[2 * q] = (uint16_t)v;
-                        crow[2 * q + 1] = (uint16_t)(v >> 16);
-                    } else {
-                        *g = (uint32_t)crow[2 * q] | ((uint32_t)crow[2 * q + 1] << 16);
-                    }
-                } else {
-                    uint16_t* g = reinterpret_cast<uint16_t*>(row + c.x0[p]) + q;
-                    if (LOAD) {
-                        const uint16_t v = *g;
-                        crow[2 * q] = v & 0xff;
-                        crow[2 * q + 1] = v >> 8;
-                    } else {
-                        *g = (uint16_t)(crow[2 * q] | (crow[2 * q + 1] << 8));
-                    }
-                }
+        for (int k = warp; k < rows; k += kIT / 32) {
+            const uint8_t* row = P.p + (size_t)(r.y + k) * P.stride;
+            for (int q = lane; q < quads; q += 32)
+                *reinterpret_cast<uint2*>(cp + k * c.cs[p] + 4 * q) = ld_quad(row, F.hbd, r.x + 4 * q);
+        }
+    }
+}
+
+// HBM -> the copy's row above and column to the left, by n threads of rank r;
+// a thread's loads are in flight together.  What neighbours have not finished
+// yet is loaded too and loaded again once a wait on it is over; no TU reads it
+// before that.
+__device__ void load_border(const IntraFrame& F, const SbCtx& c, uint16_t* cache, int r, int n) {
+    constexpr int B = 4;
+    auto items = [&](int p) { return (4 + c.rect[p].z + intra_copy_ext(c.rect[p].z)) / 4 + c.rect[p].w; };
+    const int n0 = items(0), n1 = F.np > 1 ? items(1) : 0, total = n0 + 2 * n1;
+#pragma unroll 1
+    for (int base = r; base < total; base += B * n) {
+        uint2 v[B];
+        int at[B];  // where it goes; the low bit of a group of four's marks it
+#pragma unroll
+        for (int e = 0; e < B; e++) {
+            const int k = base + e * n;
+            at[e] = -1;
+            if (k >= total) continue;
+            const int p = k < n0 ? 0 : k < n0 + n1 ? 1 : 2, q = k - (p == 0 ? 0 : p == 1 ? n0 : n0 + n1);
+            const PlaneDev& P = F.planes[p];
+            const int4 a = c.rect[p];
+            const int groups = (4 + a.z + intra_copy_ext(a.z)) / 4;
+            if (q < groups) {
+                const int x = a.x - 4 + 4 * q, y = a.y - 1;
+                if (y < 0 || x < 0 || x >= P.w) continue;
+                v[e] = ld_quad(P.p + (size_t)y * P.stride, F.hbd, x);
+                at[e] = 2 * (c.off[p] - c.cs[p] - 4 + 4 * q) + 1;
+            } else {
+                const int x = a.x - 1, y = a.y + q - groups;
+                if (x < 0 || y >= P.h) continue;
+                const uint8_t* row = P.p + (size_t)y * P.stride;
+                v[e].x = F.hbd ? __ldcg(reinterpret_cast<const unsigned short*>(row) + x) : __ldcg(row + x);
+                at[e] = 2 * (c.off[p] + (q - groups) * c.cs[p] - 1);
             }
+        }
+#pragma unroll
+        for (int e = 0; e < B; e++) {
+            if (at[e] < 0) continue;
+            uint16_t* o = cache + (at[e] >> 1);
+            if (at[e] & 1) *reinterpret_cast<uint2*>(o) = v[e];
+            else *o = (uint16_t)v[e].x;
         }
     }
 }
@@ -729,20 +1338,33 @@ struct ResTask {
     int32_t out;
 };
 
-// Residual blocks of every intra TU of the batch, ahead of the wavefront:
-// they depend on the coefficients only.  Blocks [0, small_blocks) run the
-// small TUs one per warp; the others run the large TUs with the whole CTA.
-__global__ void __launch_bounds__(kT) intra_res_kernel(const IntraFrame* __restrict__ frames,
+// Ahead of the wavefront, what depends on the descriptors and coefficients
+// only: the TU records (blocks [0, prep_blocks), a superblock per warp) and the
+// residual blocks of every intra TU of the batch (the next small_blocks run
+// the small TUs one per warp, the others the large TUs with the whole CTA).
+__global__ void __launch_bounds__(kT) intra_pre_kernel(const IntraFrame* __restrict__ frames,
+                                                       const SbItem* __restrict__ items, int nitems, TuRec* tus,
                                                        const ResTask* __restrict__ small, int n_small,
                                                        const ResTask* __restrict__ large, int n_large,
-                                                       int32_t* __restrict__ res, int small_blocks) {
+                                                       int32_t* __restrict__ res, int prep_blocks, int small_blocks) {
     __shared__ union {
-        WScr w[kNW];
-        CScr c;
+        ResScr<kSmallPx> w[kNW];
+        ResScr<64 * 64> c;
     } u;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if ((int)blockIdx.x < small_blocks) {
-        for (int q = blockIdx.x * kNW + warp; q < n_small; q += small_blocks * kNW) {
+    if ((int)blockIdx.x < prep_blocks) {
+        for (int q = blockIdx.x * kNW + warp; q < nitems; q += prep_blocks * kNW) {
+            const SbItem it = items[q];
+            const IntraFrame& F = frames[it.frame];
+            for (int k = it.tu_first + lane; k < it.tu_end; k += 32) {
+                const av1g_intra_tu t = *reinterpret_cast<const av1g_intra_tu*>(tus + k);
+                TuRec r;
+                prep_tu(F, it.log2sb, t, r);
+                tus[k] = r;
+            }
+        }
+    } else if ((int)blockIdx.x < prep_blocks + small_blocks) {
+        for (int q = (blockIdx.x - prep_blocks) * kNW + warp; q < n_small; q += small_blocks * kNW) {
             const ResTask tk = small[q];
             const IntraFrame& F = frames[tk.frame];
             const WarpG g{lane};
@@ -762,7 +1384,8 @@ __global__ void __launch_bounds__(kT) intra_res_kernel(const IntraFrame* __restr
             }
         }
     } else {
-        for (int q = blockIdx.x - small_blocks; q < n_large; q += gridDim.x - small_blocks) {
+        const int first = prep_blocks + small_blocks;
+        for (int q = blockIdx.x - first; q < n_large; q += gridDim.x - first) {
             const ResTask tk = large[q];
             const IntraFrame& F = frames[tk.frame];
             const CtaG g{tid};
@@ -781,31 +1404,83 @@ __global__ void __launch_bounds__(kT) intra_res_kernel(const IntraFrame* __restr
     }
 }
 
-// Stages TU records [b, min(b + kTuWin, end)) into the window and returns
-// the window's end (all threads call; the bounds live in registers, the same
-// in every thread).
-__device__ __forceinline__ int stage_tus(av1g_intra_tu* win, const av1g_intra_tu* __restrict__ tus, int b, int end) {
-    const int e = min(b + kTuWin, end);
-    const uint4* src = reinterpret_cast<const uint4*>(tus + b);
-    uint4* dst = reinterpret_cast<uint4*>(win);
-    for (int q = threadIdx.x; q < (e - b) * 4; q += kT) dst[q] = __ldg(src + q);
-    return e;
+// The waits of a superblock, by one warp: polls the progress words its next
+// waits name, and after each that is over reloads the copy's border and lets
+// the workers on up to the level of the first wait that is not.  A wait that
+// runs out of time sets the frame's abort word; from then on the frame's
+// superblocks no longer wait (their samples are incomplete, and the host
+// reports the frame).
+__device__ void wait_warp(Shared& S, uint16_t* cache, const int4* __restrict__ waits, const SbItem& it, int* prog,
+                          int* abort_word, int lane) {
+    long long t0 = gtimer();
+    const long long bound = *(volatile long long*)&g_wait_ns;
+    int wq = 0;
+    while (wq < it.nwait) {
+        const int q = wq + lane;
+        bool over = false;
+        if (q < it.nwait) {
+            const int4 w = __ldg(waits + it.wait_first + q);
+            over = *(volatile int*)(prog + w.y) >= w.z;
+            if (over) ld_acquire(prog + w.y);
+        }
+        // the waits are in level order: only the ones before the first open one count
+        const unsigned open = __ballot_sync(0xffffffffu, !over);
+        const int n = open ? __ffs(open) - 1 : 32;
+        if (n > 0) {
+            wq += n;
+            __syncwarp();
+            load_border(S.fr, S.sb, cache, lane, 32);
+            __syncwarp();
+            __threadfence_block();
+            if (lane == 0) *(volatile int*)&S.ready = wq < it.nwait ? __ldg(waits + it.wait_first + wq).x : kNoWait;
+            t0 = gtimer();
+            continue;
+        }
+        int stop = 0;
+        if (lane == 0) {
+            stop = *(volatile int*)abort_word;
+            if (!stop && gtimer() - t0 > bound) {
+                atomicExch(abort_word, 1);
+                stop = 1;
+            }
+        }
+        if (__shfl_sync(0xffffffffu, stop, 0)) {
+            if (lane == 0) *(volatile int*)&S.ready = kNoWait;
+            return;
+        }
+        __nanosleep(20);
+    }
 }
 
-__global__ void __launch_bounds__(kT) intra_kernel(const IntraFrame* __restrict__ frames,
-                                                   const av1g_intra_tu* __restrict__ tus,
-                                                   const SbItem* __restrict__ items, const int2* __restrict__ lvs,
-                                                   const int4* __restrict__ waits, int* prog, int* ctl, int nitems,
-                                                   const int32_t* __restrict__ res) {
+// One persistent launch.  A CTA claims superblocks in claim order.  Its worker
+// warps run a superblock's levels, in three groups of four warps that take the
+// levels in turn: a group decodes its TUs (fast_decode) while the other two
+// run the levels before its own, and only the group of the next level waits for
+// the end of a level.  Another warp publishes finished levels (its fence waits for
+// their samples to reach L2 without holding up the next level), and another waits
+// for other superblocks' levels and brings the border samples in ahead of the
+// level that reads them.
+__global__ void __launch_bounds__(kIT, 1) intra_kernel(const IntraFrame* __restrict__ frames,
+                                                       const TuRec* __restrict__ tus,
+                                                       const SbItem* __restrict__ items, const int2* __restrict__ lvs,
+                                                       const int4* __restrict__ waits, int* prog, int* ctl, int nitems,
+                                                       const int32_t* __restrict__ res) {
     // ctl[0]: the claim counter; ctl[1 + f]: frame f's abort word
-    // dynamic shared memory: Shared | TU window | superblock copy
+    // dynamic shared memory: Shared | TU records | superblock copy
     extern __shared__ __align__(16) uint8_t dsm[];
     Shared& S = *reinterpret_cast<Shared*>(dsm);
-    av1g_intra_tu* win = reinterpret_cast<av1g_intra_tu*>(dsm + kSharedBytes);
-    uint16_t* cache = reinterpret_cast<uint16_t*>(dsm + kSharedBytes + kTuWin * sizeof(av1g_intra_tu));
+    TuRec* win = reinterpret_cast<TuRec*>(dsm + kSharedBytes);
+    uint16_t* cache = reinterpret_cast<uint16_t*>(dsm + kSharedBytes + kTuStage * sizeof(TuRec));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const IntraFrame& F = S.fr;
-    const Pool pool{res};
+    // the tables that lanes index by different entries: shared, not constant, memory
+    for (int q = tid; q < 5 * 8 * 8; q += kIT) {
+        const int m = q >> 6, o = (q >> 3) & 7, i = q & 7;
+        S.tb.fi[m][o][i] = i < 7 ? (int8_t)c_fi_taps[m][o][i] : (int8_t)0;
+    }
+    if (tid < 124)
+        S.tb.sm[tid] = tid < 4 ? c_sm4[tid] : tid < 12 ? c_sm8[tid - 4] : tid < 28 ? c_sm16[tid - 12]
+                     : tid < 60 ? c_sm32[tid - 28] : c_sm64[tid - 60];
     for (;;) {
         __syncthreads();
         if (tid == 0) S.idx = atomicAdd(&ctl[0], 1);
@@ -816,118 +1491,104 @@ __global__ void __launch_bounds__(kT) intra_kernel(const IntraFrame* __restrict_
         {
             const uint32_t* src = reinterpret_cast<const uint32_t*>(frames + it.frame);
             uint32_t* dst = reinterpret_cast<uint32_t*>(&S.fr);
-            for (int q = tid; q < (int)(sizeof(IntraFrame) / 4); q += kT) dst[q] = __ldg(src + q);
+            for (int q = tid; q < (int)(sizeof(IntraFrame) / 4); q += kIT) dst[q] = __ldg(src + q);
         }
         __syncthreads();
-        if (tid == 0) {
-            int off = 0;
-            for (int p = 0; p < 3; p++) {
-                const int ssx = p ? F.ssx : 0, ssy = p ? F.ssy : 0;
-                S.sb.x0[p] = it.x0 >> ssx;
-                S.sb.y0[p] = it.y0 >> ssy;
-                S.sb.w[p] = (1 << it.log2sb) >> ssx;
-                S.sb.h[p] = (1 << it.log2sb) >> ssy;
-                S.sb.off[p] = off;
-                off += p < F.np ? S.sb.w[p] * S.sb.h[p] : 0;
-            }
-            S.abort_seen = 0;
+        if (tid < 3) {
+            const int p = tid, ssx = p ? F.ssx : 0, ssy = p ? F.ssy : 0;
+            S.sb.rect[p] = make_int4(it.x0 >> ssx, it.y0 >> ssy, (1 << it.log2sb) >> ssx, (1 << it.log2sb) >> ssy);
+            S.sb.cs[p] = copy_pitch(it.log2sb, ssx);
+            S.sb.off[p] = copy_off(it.log2sb, F.ssx, F.ssy, p);
+        }
+        if (tid == 3) {
+            S.done = 0;
+            S.ready = it.nwait > 0 ? __ldg(waits + it.wait_first).x : kNoWait;
         }
         __syncthreads();
         // the superblock's own area is written only by its own TUs, and its
         // TU records are inputs: stage both before any wait
-        move_sb<true>(F, S.sb, cache);
-        int tw0 = it.tu_first;
-        int tw1 = stage_tus(win, tus, tw0, it.tu_end);
-        // the waits, by level (staged when few; the level of the next one in a register)
-        const int4* wsrc = waits + it.wait_first;
-        if (it.nwait <= kWaitWin) {
-            for (int q = tid; q < it.nwait; q += kT) S.wv[q] = __ldg(wsrc + q);
-            wsrc = S.wv;
+        load_area(F, S.sb, cache);
+        load_border(F, S.sb, cache, tid, kIT);
+        {
+            const uint4* src = reinterpret_cast<const uint4*>(tus + it.tu_first);
+            uint4* dst = reinterpret_cast<uint4*>(win);
+            const int n = min(it.tu_end - it.tu_first, kTuStage) * 4;
+            for (int q = tid; q < n; q += kIT) dst[q] = __ldg(src + q);
         }
-        int wq = 0;
+        for (int q = tid; q <= it.nlv && q < kLvStage; q += kIT) S.lv[q] = __ldg(lvs + it.lv_first + q);
         __syncthreads();
-        int next_wait = it.nwait > 0 ? wsrc[0].x : 0x7fffffff;
-        for (int L0 = 0; L0 < it.nlv; L0 += kLvChunk) {
-            const int n = min(kLvChunk, it.nlv - L0);
-            __syncthreads();
-            for (int q = tid; q <= n; q += kT) S.lv[q] = lvs[it.lv_first + L0 + q];
-            __syncthreads();
-            for (int L = 0; L < n; L++) {
-                const int lg = L0 + L;
-                if (next_wait <= lg) {
-                    // the levels of other superblocks this level reads: poll
-                    // with volatile loads, then an acquire load orders the
-                    // reads after the progress seen
-                    const int w0 = wq;
-                    while (wq < it.nwait && wsrc[wq].x <= lg) wq++;
-                    next_wait = wq < it.nwait ? wsrc[wq].x : 0x7fffffff;
-                    int* abort_word = ctl + 1 + it.frame;
-                    const long long bound = *(volatile long long*)&g_wait_ns;
-                    for (int q = w0 + tid; q < wq; q += kT) {
-                        const int4 w = wsrc[q];
-                        const volatile int* f = prog + w.y;
-                        if (*f < w.z) {
-                            const long long t0 = gtimer();
-                            while (*f < w.z) {
-                                if (*(volatile int*)abort_word) break;
-                                if (gtimer() - t0 > bound) {
-                                    atomicExch(abort_word, 1);
-                                    break;
-                                }
-                                __nanosleep(64);
-                            }
-                        }
-                        ld_acquire(prog + w.y);
+        if (warp == kWW) {
+            if (lane == 0)
+                for (int last = 0; last < it.nlv;) {
+                    const int done = *(volatile int*)&S.done;
+                    if (done == last) {
+                        __nanosleep(20);
+                        continue;
                     }
-                    __syncthreads();
-                    if (tid == 0 && *(volatile int*)abort_word) S.abort_seen = 1;
-                    __syncthreads();
-                }
-                const bool publish = S.lv[L].y & kLevelPublished;
-                if (!S.abort_seen) {
-                    const int b = S.lv[L].x, m = S.lv[L].y & ~kLevelPublished, e = S.lv[L + 1].x;
-                    if (e > tw1 && b > tw0) {  // slide the window to this level
-                        tw0 = b;
-                        tw1 = stage_tus(win, tus, b, it.tu_end);
-                        __syncthreads();
-                    }
-                    for (int k = b + warp; k < m; k += kNW) {
-                        WScr& ws = S.s.w[warp];
-                        const av1g_intra_tu* rec = win + (k - tw0);
-                        if (k >= tw1) {  // a level wider than the window
-                            if (lane < 16)
-                                reinterpret_cast<uint32_t*>(&ws.tu)[lane] =
-                                    __ldg(reinterpret_cast<const uint32_t*>(tus + k) + lane);
-                            __syncwarp();
-                            rec = &ws.tu;
-                        }
-                        run_small(WarpG{lane}, ws, F, S.sb, cache, rec, pool);
-                        __syncwarp();
-                    }
-                    if (m < e) {
-                        __syncthreads();
-                        for (int k = m; k < e; k++) {
-                            const av1g_intra_tu* rec = win + (k - tw0);
-                            if (k >= tw1) {
-                                if (tid < 16)
-                                    reinterpret_cast<uint32_t*>(&S.s.c.tu)[tid] =
-                                        __ldg(reinterpret_cast<const uint32_t*>(tus + k) + tid);
-                                __syncthreads();
-                                rec = &S.s.c.tu;
-                            }
-                            run_large(CtaG{tid}, S.s.c, F, S.sb, cache, rec, pool);
-                            __syncthreads();
-                        }
-                    }
-                }
-                __syncthreads();
-                // publish "lg + 1 levels done" when another superblock waits
-                // for it, from the last warp (the first warp starts the next level)
-                if (publish && tid == kT - 32) {
                     __threadfence();
-                    atomicExch(prog + idx, lg + 1);
+                    atomicExch(prog + idx, done);
+                    last = done;
+                }
+            continue;
+        }
+        if (warp == kWW + 1) {
+            wait_warp(S, cache, waits, it, prog, ctl + 1 + it.frame, lane);
+            continue;
+        }
+        const int grp = warp / kGW, wi = warp % kGW;
+        auto level = [&](int q) { return q < kLvStage ? S.lv[q] : __ldg(lvs + it.lv_first + q); };
+        auto record = [&](int k) { return k - it.tu_first < kTuStage ? win + (k - it.tu_first) : tus + k; };
+        int ready = 0;
+        int lg = grp;
+        for (; lg <= it.nlv; lg += kGroups) {
+            const int2 prev = lg > 0 ? level(lg - 1) : make_int2(0, 0);
+            int b = 0, m = 0, e = 0;
+            Prog d;
+            bool fast = false;
+            if (lg < it.nlv) {
+                const int2 cur = level(lg);
+                b = cur.x;
+                m = cur.y & ~kLevelPublished;
+                e = level(lg + 1).x;
+                if (b + wi < m) {
+                    const TuRec* rec = record(b + wi);
+                    fast = rec->h.where & W_FAST;
+                    if (fast) fast_decode(d, rec, F, S.sb, cache, res, lane);
                 }
             }
+            if (lg > 0) {
+                bar_sync(1 + (lg - 1) % kGroups, 2 * kGT);
+                // "lg levels done", when another superblock waits for it or
+                // the superblock is finished
+                if (wi == 0 && lane == 0 && ((prev.y & kLevelPublished) || lg == it.nlv)) {
+                    __threadfence_block();
+                    *(volatile int*)&S.done = lg;
+                }
+            }
+            if (lg == it.nlv) break;
+            if (ready <= lg) {
+                while ((ready = *(volatile int*)&S.ready) <= lg) {}
+                __threadfence_block();
+            }
+            WScr& ws = S.s[grp].w[wi];
+            for (int k = b + wi; k < m; k += kGW) {
+                if (k > b + wi) {
+                    const TuRec* rec = record(k);
+                    fast = rec->h.where & W_FAST;
+                    if (fast) fast_decode(d, rec, F, S.sb, cache, res, lane);
+                }
+                if (fast) fast_run(d, ws, F, S.sb, cache, S.tb, lane);
+                else run_tu(WarpG{lane}, ws, record(k), F, S.sb, cache, S.tb, res);
+                __syncwarp();
+            }
+            if (m < e) {
+                const WorkG g{tid - grp * kGT, 4 + grp};
+                for (int k = m; k < e; k++) {
+                    if (k > b) g.sync();
+                    run_tu(g, S.s[grp].c, record(k), F, S.sb, cache, S.tb, res);
+                }
+            }
+            bar_arrive(1 + lg % kGroups, 2 * kGT);
         }
     }
 }
@@ -956,7 +1617,8 @@ void plan_fault_wait(IntraPlan& plan, int f) {
 
 // The most dynamic shared memory any launch asks for: the fixed part, the TU
 // window and the largest superblock copy (128x128, three full planes, u16).
-constexpr size_t kMaxDynSmem = kSharedBytes + kTuWin * sizeof(av1g_intra_tu) + 3 * 128 * 128 * sizeof(uint16_t);
+constexpr size_t kMaxDynSmem =
+    kSharedBytes + kTuStage * sizeof(TuRec) + 3 * intra_copy_samples(128, 128) * sizeof(uint16_t);
 static_assert(kMaxDynSmem <= 227 * 1024, "intra_kernel's shared memory exceeds an SM's");
 
 // The kernel's dynamic shared memory limit is a per-device attribute that
@@ -1045,27 +1707,29 @@ av1g_status intra_run_status(const av1g_intra_job* jobs, int n, cudaStream_t st,
     int32_t* dres = (int32_t*)(dev_buf + off_res);
     int sms = 0;
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess && (!rs.empty() || !rl.empty())) {
+    if (e == cudaSuccess) {
+        const int pb_blocks = (int)std::min<long long>(((long long)nitems + kNW - 1) / kNW, 8LL * sms);
         const int sb_blocks = (int)std::min<long long>(((long long)rs.size() + kNW - 1) / kNW, 16LL * sms);
         const int lb_blocks = (int)std::min<long long>((long long)rl.size(), 4LL * sms);
-        intra_res_kernel<<<sb_blocks + lb_blocks, kT, 0, st>>>(dframes, (const ResTask*)(dev_buf + off_rs), (int)rs.size(),
-                                                               (const ResTask*)(dev_buf + off_rl), (int)rl.size(), dres,
-                                                               sb_blocks);
+        intra_pre_kernel<<<pb_blocks + sb_blocks + lb_blocks, kT, 0, st>>>(
+            dframes, (const SbItem*)(dev_buf + off_items), nitems, (TuRec*)(dev_buf + off_tus),
+            (const ResTask*)(dev_buf + off_rs), (int)rs.size(), (const ResTask*)(dev_buf + off_rl), (int)rl.size(), dres,
+            pb_blocks, sb_blocks);
         e = cudaGetLastError();
     }
-    const size_t smem = kSharedBytes + kTuWin * sizeof(av1g_intra_tu) + plan.cache_bytes;
+    const size_t smem = kSharedBytes + kTuStage * sizeof(TuRec) + plan.cache_bytes;
     if (e == cudaSuccess && smem > kMaxDynSmem) e = cudaErrorInvalidValue;  // cannot happen: cache_bytes is bounded
     if (e == cudaSuccess) e = ensure_intra_smem_limit(dev);
     int per_sm = 0;
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, intra_kernel, kT, smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, intra_kernel, kIT, smem);
     if (e == cudaSuccess) {
         // as many CTAs as the wavefront can keep busy (the superblocks of
         // one depth, twice over since level-granular waits let the next depth
         // start early), not the whole GPU: idle CTAs would only poll while
         // other streams' kernels wait for SMs
         const int grid = std::max(1, std::min({nitems, std::max(per_sm, 1) * sms, 2 * plan.width + 2}));
-        intra_kernel<<<grid, kT, smem, st>>>(
-            dframes, (const av1g_intra_tu*)(dev_buf + off_tus), (const SbItem*)(dev_buf + off_items),
+        intra_kernel<<<grid, kIT, smem, st>>>(
+            dframes, (const TuRec*)(dev_buf + off_tus), (const SbItem*)(dev_buf + off_items),
             (const int2*)(dev_buf + off_lv), (const int4*)(dev_buf + off_waits), (int*)(dev_buf + off_done),
             (int*)(dev_buf + off_ctl), nitems, dres);
         e = cudaGetLastError();

@@ -100,8 +100,8 @@ av1g_status intra_plan(const av1g_intra_job* jobs, int n, IntraPlan& plan, std::
         const int sb = j.sb_size, log2sb = sb == 128 ? 7 : 6;
         const int ssx = h.subsampling_x, ssy = h.subsampling_y;
         {
-            size_t cb = (size_t)sb * sb;
-            if (h.num_planes > 1) cb += 2 * (size_t)(sb >> ssx) * (sb >> ssy);
+            size_t cb = intra_copy_samples(sb, sb);
+            if (h.num_planes > 1) cb += 2 * (size_t)intra_copy_samples(sb >> ssx, sb >> ssy);
             plan.cache_bytes = std::max(plan.cache_bytes, cb * sizeof(uint16_t));
         }
         plan.map_base[i] = plan.maps.size();

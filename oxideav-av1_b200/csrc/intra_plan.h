@@ -36,6 +36,12 @@ struct SbItem {
 
 // TUs of at most this many samples run on one warp; larger ones on the CTA.
 constexpr int kIntraSmallPx = 256;
+// A superblock's copy in shared memory, per plane of w x h samples: one row
+// above, which runs on ext samples past the right edge (the largest above-right
+// edge), and one column to the left in a group of four.
+constexpr __host__ __device__ int intra_copy_ext(int w) { return w < 64 ? w : 64; }
+constexpr __host__ __device__ int intra_copy_pitch(int w) { return 4 + w + intra_copy_ext(w); }
+constexpr __host__ __device__ int intra_copy_samples(int w, int h) { return intra_copy_pitch(w) * (h + 1); }
 // Level-table flag (in .y): other superblocks wait for this level.
 constexpr int kLevelPublished = 1 << 30;
 
