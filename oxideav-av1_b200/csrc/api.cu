@@ -336,7 +336,7 @@ av1g_status run(const av1g_frame_job* jobs, int n, int stage_mask, int mode, voi
     if (st != AV1G_OK) return st;
     cudaStream_t s = (cudaStream_t)stream;
     uint8_t* dev = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&dev, P.total_bytes, s);
+    cudaError_t e = workspace_alloc(&dev, P.total_bytes, s);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMallocAsync");
     bind(P, dev);
     // the prefix is 256-byte aligned; one or two launches carry a small one
@@ -550,7 +550,7 @@ av1g_status av1g_autotune_postfilter(const av1g_frame_job* jobs, int32_t n, void
     const int hbd = P.b.frames[0].hbd;
     cudaStream_t s = (cudaStream_t)stream;
     uint8_t* dev = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&dev, P.total_bytes, s);
+    cudaError_t e = workspace_alloc(&dev, P.total_bytes, s);
     if (e != cudaSuccess) return cuda_fail(e, "cudaMallocAsync");
     bind(P, dev);
     e = cudaMemcpyAsync(dev, P.host.data(), P.off_scratch, cudaMemcpyHostToDevice, s);

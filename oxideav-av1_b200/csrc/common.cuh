@@ -81,6 +81,11 @@ __device__ __forceinline__ long long round2ll(long long x, int n) {
 }
 __device__ __forceinline__ int floor_log2u(unsigned x) { return x ? 31 - __clz(x) : 0; }
 
+// A call's workspace, stream-ordered (freed with cudaFreeAsync on its stream).
+// The device's default pool keeps up to kWorkspaceKeep bytes of what is freed.
+constexpr unsigned long long kWorkspaceKeep = 256ull << 20;
+cudaError_t workspace_alloc(uint8_t** p, size_t n, cudaStream_t s);
+
 // Enqueues a host-to-device copy of n bytes through a pinned staging block
 // (returns once enqueued; the host bytes may be reused immediately).
 cudaError_t upload(void* dev, const void* host, size_t n, cudaStream_t s);

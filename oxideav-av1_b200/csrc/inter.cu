@@ -757,7 +757,7 @@ av1g_status inter_run(const av1g_inter_job* jobs, int n, cudaStream_t st, std::s
         bytes = al(bytes + (size_t)frames[i].mask_stride * (jobs[i].planes[0].height + kMaskMargin));
     }
     uint8_t* dev = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&dev, bytes, st);
+    cudaError_t e = workspace_alloc(&dev, bytes, st);
     if (e != cudaSuccess) {
         err = std::string("cudaMallocAsync: ") + cudaGetErrorString(e);
         return AV1G_EDEVICE;

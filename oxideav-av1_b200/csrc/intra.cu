@@ -1686,7 +1686,7 @@ av1g_status intra_run_status(const av1g_intra_job* jobs, int n, cudaStream_t st,
     const size_t off_res = al(bytes);
     const size_t total = off_res + sizeof(int32_t) * (size_t)res_ints;
     uint8_t* dev_buf = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&dev_buf, total, st);
+    cudaError_t e = workspace_alloc(&dev_buf, total, st);
     if (e != cudaSuccess) {
         err = std::string("cudaMallocAsync: ") + cudaGetErrorString(e);
         return AV1G_EDEVICE;

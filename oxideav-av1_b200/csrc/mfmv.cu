@@ -239,7 +239,7 @@ av1g_status mf_store_run(const av1g_mf_store_job* jobs, int n, cudaStream_t s, s
     const size_t off_starts = align256(sizeof(StoreDev) * n);
     const size_t bytes = off_starts + sizeof(int32_t) * (n + 1);
     uint8_t* buf = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&buf, bytes, s);
+    cudaError_t e = workspace_alloc(&buf, bytes, s);
     if (e != cudaSuccess) {
         err = std::string("cudaMallocAsync: ") + cudaGetErrorString(e);
         return AV1G_EDEVICE;
@@ -353,7 +353,7 @@ av1g_status mf_project_run(const av1g_mf_project_job* jobs, int n, cudaStream_t 
     const size_t off_win = align256(off_cstart + sizeof(int32_t) * (npass + 1));
     const size_t bytes = off_win + sizeof(unsigned long long) * (size_t)positions;
     uint8_t* buf = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&buf, bytes, s);
+    cudaError_t e = workspace_alloc(&buf, bytes, s);
     if (e != cudaSuccess) {
         err = std::string("cudaMallocAsync: ") + cudaGetErrorString(e);
         return AV1G_EDEVICE;

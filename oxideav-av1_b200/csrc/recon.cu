@@ -150,7 +150,7 @@ av1g_status recon_run(const av1g_recon_job* jobs, int n, cudaStream_t s, std::st
     size_t off_tasks = (off_tus + sizeof(TuDev) * total + 255) & ~(size_t)255;
     size_t bytes = off_tasks + sizeof(Task) * tasks.size();
     uint8_t* dev = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&dev, bytes, s);
+    cudaError_t e = workspace_alloc(&dev, bytes, s);
     if (e != cudaSuccess) {
         err = std::string("cudaMallocAsync: ") + cudaGetErrorString(e);
         return AV1G_EDEVICE;

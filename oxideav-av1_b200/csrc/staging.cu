@@ -10,6 +10,7 @@
 // has completed.  Idle blocks wait in power-of-two capacity classes; blocks in
 // flight queue in enqueue order and only the oldest few are polled per call,
 // so an upload costs a handful of event queries however large the pool grows.
+#include <atomic>
 #include <cstring>
 #include <deque>
 #include <functional>
@@ -64,6 +65,32 @@ cudaError_t reap() {
 }
 
 }  // namespace
+
+// cudaMallocAsync with a pool that keeps its memory.  The default pool's
+// release threshold is 0, so whenever the caller synchronises it unmaps all that
+// is free, and the next call maps it again: 0.3 to 3 ms of host time per
+// allocation on a B200 box, paid by every entry point that synchronises (and by
+// every caller that waits for a result).  The threshold is raised once per device, to a
+// bound that holds a 4K key frame's workspace, and only where it is still 0: one
+// that the application or a serving engine has set stands.  The pool is the
+// device's own, so the application can trim it (cudaMemPoolTrimTo).
+cudaError_t workspace_alloc(uint8_t** p, size_t n, cudaStream_t s) {
+    static std::atomic<bool> seen[64];
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    if (device < 64 && !seen[device].load(std::memory_order_acquire)) {
+        cudaMemPool_t pool;
+        uint64_t keep = 0;
+        if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess &&
+            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess && keep == 0) {
+            keep = kWorkspaceKeep;
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        }
+        seen[device].store(true, std::memory_order_release);
+    }
+    return cudaMallocAsync(reinterpret_cast<void**>(p), n, s);
+}
 
 cudaError_t upload_with(void* dev, size_t n, cudaStream_t s, const std::function<void(uint8_t*)>& fill) {
     if (n == 0) return cudaSuccess;

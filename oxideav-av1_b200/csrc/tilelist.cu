@@ -155,7 +155,7 @@ av1g_status tile_list_run(const av1g_tile_list_job* jobs, int n, cudaStream_t s,
     const size_t off_st = (off_ent + sizeof(EntryDev) * ed.size() + 255) & ~(size_t)255;
     const size_t bytes = off_st + sizeof(int32_t) * (n + 1);
     uint8_t* buf = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&buf, bytes, s);
+    cudaError_t e = workspace_alloc(&buf, bytes, s);
     if (e != cudaSuccess) {
         err = std::string("cudaMallocAsync: ") + cudaGetErrorString(e);
         return AV1G_EDEVICE;
