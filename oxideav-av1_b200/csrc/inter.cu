@@ -28,6 +28,7 @@
 
 #include "av1_spec_tables.h"
 #include "common.cuh"
+#include "host_pool.h"
 #include "wedge.cuh"
 
 namespace av1g {
@@ -674,28 +675,40 @@ uint32_t tiles_of(const Call& c) { return (uint32_t)((c.w + 7) >> 3) * (uint32_t
 
 av1g_status inter_run(const av1g_inter_job* jobs, int n, cudaStream_t st, std::string& err) {
     std::vector<InterFrame> frames(n);
-    std::vector<Call> a, b;
-    std::vector<WarpRec> warps;
-    std::vector<Seg> segs;
     std::vector<int> diff_frames;
-    {
-        size_t np = 0;
-        for (int i = 0; i < n; i++) np += jobs[i].num_preds > 0 ? (size_t)jobs[i].num_preds : 0;
-        a.reserve(np);
-    }
+    // the calls are built by runs of one job, which helper threads share
+    // (host_pool.h); a run's lists are joined to the others' as they are copied
+    struct Run {
+        int job, k0, k1;
+        av1g_status rc = AV1G_OK;
+        std::string err;
+        std::vector<Call> a, b;
+        std::vector<WarpRec> warps;
+        std::vector<Seg> segs;
+        std::vector<uint32_t> sa, sb;  // tiles before each call of a / b, within the run
+        uint32_t tiles_a = 0, tiles_b = 0;
+        size_t at_a = 0, at_b = 0, at_warp = 0, at_seg = 0;  // where its lists start
+        uint32_t tile_a = 0, tile_b = 0;
+        bool any_diff = false;
+    };
+    std::vector<Run> runs;
+    long long total = 0;
+    av1g_status bad_frame = AV1G_OK;
     for (int i = 0; i < n; i++) {
         const av1g_inter_job& j = jobs[i];
         if (!j.hdr || !j.refs || j.num_preds < 0 || (j.num_preds > 0 && !j.preds) || j.num_neighbours < 0 ||
             (j.num_neighbours > 0 && !j.neighbours) || j.num_warps < 0 || (j.num_warps > 0 && !j.warps)) {
             err = "inter job " + std::to_string(i) + ": missing header, references or lists";
-            return AV1G_EINVAL;
+            bad_frame = AV1G_EINVAL;
+            break;
         }
         const av1g_frame_header& h = *j.hdr;
         if ((h.bit_depth != 8 && h.bit_depth != 10 && h.bit_depth != 12) || h.frame_width <= 0 ||
             h.frame_height <= 0 || h.frame_width > 65535 || h.frame_height > 65535 || h.subsampling_x > 1 ||
             h.subsampling_y > 1 || h.num_planes < 1 || h.num_planes > 3) {
             err = "inter job " + std::to_string(i) + ": bit depth, subsampling or frame size";
-            return AV1G_EINVAL;
+            bad_frame = AV1G_EINVAL;
+            break;
         }
         InterFrame& F = frames[i];
         memset(&F, 0, sizeof F);
@@ -706,7 +719,8 @@ av1g_status inter_run(const av1g_inter_job* jobs, int n, cudaStream_t st, std::s
             if (!pl.data || pl.width <= 0 || pl.height <= 0 || pl.stride < pl.width * (F.hbd ? 2 : 1) ||
                 (pl.stride & 15)) {
                 err = "inter job " + std::to_string(i) + ": plane " + std::to_string(p);
-                return AV1G_EINVAL;
+                bad_frame = AV1G_EINVAL;
+                break;
             }
             F.planes[p] = PlaneDev{(uint8_t*)pl.data, pl.stride, pl.width, pl.height};
             const av1g_plane& sp = j.interintra_out[p];
@@ -714,7 +728,8 @@ av1g_status inter_run(const av1g_inter_job* jobs, int n, cudaStream_t st, std::s
                 if (sp.width < pl.width || sp.height < pl.height || sp.stride < pl.width * (F.hbd ? 2 : 1) ||
                     (sp.stride & 15) || ((uintptr_t)sp.data & 15)) {
                     err = "inter job " + std::to_string(i) + ": inter-intra side plane " + std::to_string(p);
-                    return AV1G_EINVAL;
+                    bad_frame = AV1G_EINVAL;
+                    break;
                 }
                 F.side[p] = PlaneDev{(uint8_t*)sp.data, sp.stride, pl.width, pl.height};
             }
@@ -725,30 +740,79 @@ av1g_status inter_run(const av1g_inter_job* jobs, int n, cudaStream_t st, std::s
                                         ((R.upscaled_width + sx) >> sx) - 1, ((R.frame_height + sy) >> sy) - 1};
             }
         }
-        Builder B{j, i, h.subsampling_x, h.subsampling_y, F.hbd, a, b, warps, segs, err};
-        B.init();
-        for (int k = 0; k < j.num_preds; k++)
-            if (!B.add(k)) return AV1G_EINVAL;
-        if (B.any_diff) {
-            F.mask_stride = ((j.planes[0].width + kMaskMargin) + 15) & ~15;
-            diff_frames.push_back(i);
+        if (bad_frame != AV1G_OK) break;
+        const int parts = parallel_parts(j.num_preds, 1024);
+        total += j.num_preds;
+        for (int u = 0; u < parts; u++) {
+            runs.emplace_back();
+            Run& r = runs.back();
+            r.job = i;
+            r.k0 = (int)((long long)j.num_preds * u / parts);
+            r.k1 = (int)((long long)j.num_preds * (u + 1) / parts);
         }
     }
-    if (a.empty() && b.empty()) return AV1G_OK;
-
-    std::vector<uint32_t> sa(a.size() + 1, 0), sb(b.size() + 1, 0);
-    for (size_t k = 0; k < a.size(); k++) sa[k + 1] = sa[k] + tiles_of(a[k]);
-    for (size_t k = 0; k < b.size(); k++) sb[k + 1] = sb[k] + tiles_of(b[k]);
+    parallel_for((int)runs.size(), total, [&](int u) {
+        Run& r = runs[u];
+        const av1g_inter_job& j = jobs[r.job];
+        r.a.reserve(r.k1 - r.k0);
+        Builder B{j, r.job, j.hdr->subsampling_x, j.hdr->subsampling_y, frames[r.job].hbd, r.a, r.b, r.warps, r.segs,
+                  r.err};
+        B.init();
+        for (int k = r.k0; k < r.k1; k++)
+            if (!B.add(k)) {
+                r.rc = AV1G_EINVAL;
+                return;
+            }
+        r.any_diff = B.any_diff;
+        r.sa.resize(r.a.size());
+        r.sb.resize(r.b.size());
+        for (size_t k = 0; k < r.a.size(); k++) {
+            r.sa[k] = r.tiles_a;
+            r.tiles_a += tiles_of(r.a[k]);
+        }
+        for (size_t k = 0; k < r.b.size(); k++) {
+            r.sb[k] = r.tiles_b;
+            r.tiles_b += tiles_of(r.b[k]);
+        }
+    });
+    // the first error in call order, then a bad frame's (its job comes after the runs)
+    for (const Run& r : runs)
+        if (r.rc != AV1G_OK) {
+            err = r.err;
+            return r.rc;
+        }
+    if (bad_frame != AV1G_OK) return bad_frame;
+    size_t n_a = 0, n_b = 0, n_warp = 0, n_seg = 0;
+    uint32_t tiles_a = 0, tiles_b = 0;
+    for (Run& r : runs) {
+        r.at_a = n_a;
+        r.at_b = n_b;
+        r.at_warp = n_warp;
+        r.at_seg = n_seg;
+        r.tile_a = tiles_a;
+        r.tile_b = tiles_b;
+        n_a += r.a.size();
+        n_b += r.b.size();
+        n_warp += r.warps.size();
+        n_seg += r.segs.size();
+        tiles_a += r.tiles_a;
+        tiles_b += r.tiles_b;
+        if (r.any_diff && (diff_frames.empty() || diff_frames.back() != r.job)) {
+            frames[r.job].mask_stride = ((jobs[r.job].planes[0].width + kMaskMargin) + 15) & ~15;
+            diff_frames.push_back(r.job);
+        }
+    }
+    if (n_a == 0 && n_b == 0) return AV1G_OK;
 
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
     size_t o_frames = 0;
     size_t o_a = al(o_frames + sizeof(InterFrame) * n);
-    size_t o_b = al(o_a + sizeof(Call) * a.size());
-    size_t o_sa = al(o_b + sizeof(Call) * b.size());
-    size_t o_sb = al(o_sa + sizeof(uint32_t) * sa.size());
-    size_t o_w = al(o_sb + sizeof(uint32_t) * sb.size());
-    size_t o_s = al(o_w + sizeof(WarpRec) * warps.size());
-    size_t o_m = al(o_s + sizeof(Seg) * segs.size());
+    size_t o_b = al(o_a + sizeof(Call) * n_a);
+    size_t o_sa = al(o_b + sizeof(Call) * n_b);
+    size_t o_sb = al(o_sa + sizeof(uint32_t) * (n_a + 1));
+    size_t o_w = al(o_sb + sizeof(uint32_t) * (n_b + 1));
+    size_t o_s = al(o_w + sizeof(WarpRec) * n_warp);
+    size_t o_m = al(o_s + sizeof(Seg) * n_seg);
     size_t host_bytes = o_m;
     std::vector<size_t> mask_off(n, 0);
     size_t bytes = o_m;
@@ -765,27 +829,45 @@ av1g_status inter_run(const av1g_inter_job* jobs, int n, cudaStream_t st, std::s
     for (int i : diff_frames) frames[i].mask = dev + mask_off[i];
     e = upload_with(dev, host_bytes, st, [&](uint8_t* host) {
         memcpy(host + o_frames, frames.data(), sizeof(InterFrame) * n);
-        if (!a.empty()) memcpy(host + o_a, a.data(), sizeof(Call) * a.size());
-        if (!b.empty()) memcpy(host + o_b, b.data(), sizeof(Call) * b.size());
-        memcpy(host + o_sa, sa.data(), sizeof(uint32_t) * sa.size());
-        memcpy(host + o_sb, sb.data(), sizeof(uint32_t) * sb.size());
-        if (!warps.empty()) memcpy(host + o_w, warps.data(), sizeof(WarpRec) * warps.size());
-        if (!segs.empty()) memcpy(host + o_s, segs.data(), sizeof(Seg) * segs.size());
+        uint32_t* sa = reinterpret_cast<uint32_t*>(host + o_sa);
+        uint32_t* sb = reinterpret_cast<uint32_t*>(host + o_sb);
+        sa[n_a] = tiles_a;
+        sb[n_b] = tiles_b;
+        parallel_for((int)runs.size(), total, [&](int u) {
+            const Run& r = runs[u];
+            auto put = [&](const std::vector<Call>& from, size_t o, size_t at, const std::vector<uint32_t>& tiles,
+                           uint32_t* starts, uint32_t first) {
+                Call* dst = reinterpret_cast<Call*>(host + o) + at;
+                for (size_t k = 0; k < from.size(); k++) {
+                    Call c = from[k];
+                    for (int l = 0; l < c.nref; l++)
+                        if (c.ref[l].warp) c.ref[l].sx += (int32_t)r.at_warp;
+                    c.seg_first += (uint32_t)r.at_seg;
+                    dst[k] = c;
+                    starts[at + k] = first + tiles[k];
+                }
+            };
+            put(r.a, o_a, r.at_a, r.sa, sa, r.tile_a);
+            put(r.b, o_b, r.at_b, r.sb, sb, r.tile_b);
+            if (!r.warps.empty())
+                memcpy(host + o_w + sizeof(WarpRec) * r.at_warp, r.warps.data(), sizeof(WarpRec) * r.warps.size());
+            if (!r.segs.empty()) memcpy(host + o_s + sizeof(Seg) * r.at_seg, r.segs.data(), sizeof(Seg) * r.segs.size());
+        });
     });
     if (e == cudaSuccess && bytes > host_bytes) e = cudaMemsetAsync(dev + host_bytes, 0, bytes - host_bytes, st);
     const InterFrame* df = (const InterFrame*)(dev + o_frames);
     const WarpRec* dw = (const WarpRec*)(dev + o_w);
     const Seg* ds = (const Seg*)(dev + o_s);
-    if (e == cudaSuccess && sa.back()) {
-        unsigned grid = (sa.back() + kWarps - 1) / kWarps;
+    if (e == cudaSuccess && tiles_a) {
+        unsigned grid = (tiles_a + kWarps - 1) / kWarps;
         inter_kernel<<<grid, kWarps * 32, 0, st>>>(df, (const Call*)(dev + o_a), (const uint32_t*)(dev + o_sa),
-                                                  (int)a.size(), sa.back(), dw, ds);
+                                                  (int)n_a, tiles_a, dw, ds);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess && sb.back()) {
-        unsigned grid = (sb.back() + kWarps - 1) / kWarps;
+    if (e == cudaSuccess && tiles_b) {
+        unsigned grid = (tiles_b + kWarps - 1) / kWarps;
         inter_kernel<<<grid, kWarps * 32, 0, st>>>(df, (const Call*)(dev + o_b), (const uint32_t*)(dev + o_sb),
-                                                  (int)b.size(), sb.back(), dw, ds);
+                                                  (int)n_b, tiles_b, dw, ds);
         e = cudaGetLastError();
     }
     cudaFreeAsync(dev, st);

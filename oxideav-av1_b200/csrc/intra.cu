@@ -45,6 +45,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "host_pool.h"
 #include "intra_plan.h"
 #include "itx.cuh"
 #include "wedge.cuh"
@@ -1656,32 +1657,57 @@ av1g_status intra_run_status(const av1g_intra_job* jobs, int n, cudaStream_t st,
         for (int i = 0; i < n; i++)
             if (jobs[i].hdr->frame_width == fw) plan_fault_wait(plan, i);
     const int nitems = (int)plan.items.size();
-    // residual tasks; each TU's device record points at its residual block
-    std::vector<ResTask> rs, rl;
-    long long res_ints = 0;
-    for (const SbItem& it : plan.items)
-        for (int k = it.tu_first; k < it.tu_end; k++) {
-            av1g_intra_tu& t = plan.tus[k];
-            if (!(t.flags & AV1G_INTRA_RESIDUAL)) continue;
-            const int px = kTxW[t.tx_size] * kTxH[t.tx_size];
-            (px > kSmallPx ? rl : rs).push_back(ResTask{t.res, it.frame, (int32_t)res_ints});
-            t.res.coeff_offset = (uint32_t)res_ints;
-            res_ints += px;
-        }
+    // residual tasks, counted by part of the superblocks: each TU's device
+    // record will point at its residual block
+    const int parts = std::min(nitems, parallel_parts((long long)plan.ntus, 4096));
+    struct Count {
+        size_t small = 0, large = 0;
+        long long ints = 0;
+    };
+    std::vector<Count> at(parts + 1);
+    auto span = [&](int u, int& i0, int& i1) {
+        i0 = (int)((long long)nitems * u / parts);
+        i1 = (int)((long long)nitems * (u + 1) / parts);
+    };
+    // TU k of a superblock's range, in decode order (its records take the same range)
+    auto source = [&](const SbItem& it, int k) -> const av1g_intra_tu& {
+        return jobs[it.frame].tus[k - plan.tu_base[it.frame]];
+    };
+    parallel_for(parts, (long long)plan.ntus, [&](int u) {
+        Count c;
+        int i0, i1;
+        span(u, i0, i1);
+        for (int i = i0; i < i1; i++)
+            for (int k = plan.items[i].tu_first; k < plan.items[i].tu_end; k++) {
+                const av1g_intra_tu& t = source(plan.items[i], k);
+                if (!(t.flags & AV1G_INTRA_RESIDUAL)) continue;
+                const int px = kTxW[t.tx_size] * kTxH[t.tx_size];
+                (px > kSmallPx ? c.large : c.small)++;
+                c.ints += px;
+            }
+        at[u + 1] = c;
+    });
+    for (int u = 0; u < parts; u++) {
+        at[u + 1].small += at[u].small;
+        at[u + 1].large += at[u].large;
+        at[u + 1].ints += at[u].ints;
+    }
+    const size_t n_rs = at[parts].small, n_rl = at[parts].large;
+    const long long res_ints = at[parts].ints;
     if (res_ints >= (1LL << 31)) {
         err = "intra batch: more than 2^31 residual samples";
         return AV1G_EINVAL;
     }
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const size_t off_tus = al(sizeof(IntraFrame) * n);
-    const size_t off_items = al(off_tus + sizeof(av1g_intra_tu) * plan.tus.size());
+    const size_t off_items = al(off_tus + sizeof(av1g_intra_tu) * plan.ntus);
     const size_t off_lv = al(off_items + sizeof(SbItem) * plan.items.size());
     const size_t off_waits = al(off_lv + sizeof(int2) * plan.lvtab.size());
     const size_t off_done = al(off_waits + sizeof(int4) * plan.waits.size());
     const size_t off_ctl = al(off_done + sizeof(int) * plan.items.size());
     const size_t off_rs = al(off_ctl + (1 + (size_t)n) * sizeof(int));
-    const size_t off_rl = al(off_rs + sizeof(ResTask) * rs.size());
-    const size_t off_maps = al(off_rl + sizeof(ResTask) * rl.size());
+    const size_t off_rl = al(off_rs + sizeof(ResTask) * n_rs);
+    const size_t off_maps = al(off_rl + sizeof(ResTask) * n_rl);
     const size_t bytes = off_maps + plan.maps.size();  // uploaded
     const size_t off_res = al(bytes);
     const size_t total = off_res + sizeof(int32_t) * (size_t)res_ints;
@@ -1694,13 +1720,32 @@ av1g_status intra_run_status(const av1g_intra_job* jobs, int n, cudaStream_t st,
     for (int i = 0; i < n; i++) plan.frames[i].maps = dev_buf + off_maps + plan.map_base[i];
     e = upload_with(dev_buf, bytes, st, [&](uint8_t* host) {
         memcpy(host, plan.frames.data(), sizeof(IntraFrame) * n);
-        memcpy(host + off_tus, plan.tus.data(), sizeof(av1g_intra_tu) * plan.tus.size());
+        av1g_intra_tu* tus = reinterpret_cast<av1g_intra_tu*>(host + off_tus);
+        ResTask* small = reinterpret_cast<ResTask*>(host + off_rs);
+        ResTask* large = reinterpret_cast<ResTask*>(host + off_rl);
+        parallel_for(parts, (long long)plan.ntus, [&](int u) {
+            Count c = at[u];
+            int i0, i1;
+            span(u, i0, i1);
+            for (int i = i0; i < i1; i++) {
+                const SbItem& it = plan.items[i];
+                for (int k = it.tu_first; k < it.tu_end; k++) {
+                    const av1g_intra_tu& t = source(it, k);
+                    av1g_intra_tu& r = tus[plan.order[k]];
+                    r = t;
+                    if (t.interintra) r.palette_map = plan.wedge[k];
+                    if (!(t.flags & AV1G_INTRA_RESIDUAL)) continue;
+                    const int px = kTxW[t.tx_size] * kTxH[t.tx_size];
+                    (px > kSmallPx ? large[c.large++] : small[c.small++]) = ResTask{t.res, it.frame, (int32_t)c.ints};
+                    r.res.coeff_offset = (uint32_t)c.ints;
+                    c.ints += px;
+                }
+            }
+        });
         memcpy(host + off_items, plan.items.data(), sizeof(SbItem) * plan.items.size());
         memcpy(host + off_lv, plan.lvtab.data(), sizeof(int2) * plan.lvtab.size());
         if (!plan.waits.empty()) memcpy(host + off_waits, plan.waits.data(), sizeof(int4) * plan.waits.size());
         memset(host + off_done, 0, off_rs - off_done);  // progress, claim counter, abort flag
-        if (!rs.empty()) memcpy(host + off_rs, rs.data(), sizeof(ResTask) * rs.size());
-        if (!rl.empty()) memcpy(host + off_rl, rl.data(), sizeof(ResTask) * rl.size());
         if (!plan.maps.empty()) memcpy(host + off_maps, plan.maps.data(), plan.maps.size());
     });
     const IntraFrame* dframes = (const IntraFrame*)dev_buf;
@@ -1709,11 +1754,11 @@ av1g_status intra_run_status(const av1g_intra_job* jobs, int n, cudaStream_t st,
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess) {
         const int pb_blocks = (int)std::min<long long>(((long long)nitems + kNW - 1) / kNW, 8LL * sms);
-        const int sb_blocks = (int)std::min<long long>(((long long)rs.size() + kNW - 1) / kNW, 16LL * sms);
-        const int lb_blocks = (int)std::min<long long>((long long)rl.size(), 4LL * sms);
+        const int sb_blocks = (int)std::min<long long>(((long long)n_rs + kNW - 1) / kNW, 16LL * sms);
+        const int lb_blocks = (int)std::min<long long>((long long)n_rl, 4LL * sms);
         intra_pre_kernel<<<pb_blocks + sb_blocks + lb_blocks, kT, 0, st>>>(
             dframes, (const SbItem*)(dev_buf + off_items), nitems, (TuRec*)(dev_buf + off_tus),
-            (const ResTask*)(dev_buf + off_rs), (int)rs.size(), (const ResTask*)(dev_buf + off_rl), (int)rl.size(), dres,
+            (const ResTask*)(dev_buf + off_rs), (int)n_rs, (const ResTask*)(dev_buf + off_rl), (int)n_rl, dres,
             pb_blocks, sb_blocks);
         e = cudaGetLastError();
     }
@@ -1758,7 +1803,7 @@ extern "C" av1g_status av1g_intra_plan_stats_get(const av1g_intra_job* jobs, int
     std::string err;
     av1g_status rc = av1g::intra_plan(jobs, n, plan, err);
     if (rc != AV1G_OK) return rc;
-    *out = av1g_intra_plan_stats{(int32_t)plan.items.size(), (int32_t)plan.tus.size(), (int32_t)plan.waits.size(),
+    *out = av1g_intra_plan_stats{(int32_t)plan.items.size(), (int32_t)plan.ntus, (int32_t)plan.waits.size(),
                                  plan.depth, plan.width, 0};
     return AV1G_OK;
 }

@@ -4,6 +4,7 @@
 #pragma once
 
 #include <cstdint>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -49,7 +50,13 @@ struct IntraPlan {
     std::vector<IntraFrame> frames;     // maps still relative: map_base[frame]
     std::vector<size_t> map_base;
     std::vector<uint8_t> maps;          // palette colour indices of all jobs
-    std::vector<av1g_intra_tu> tus;     // per superblock, in level order (small before large)
+    // TU u of the batch (jobs in order, their TUs in decode order) is record
+    // order[u] of the launch: per superblock in level order, small before large.
+    // tu_base[i]: job i's first; wedge[u]: the window of an inter-intra wedge
+    size_t ntus = 0;
+    std::vector<size_t> tu_base;
+    std::unique_ptr<uint32_t[]> order;
+    std::vector<uint32_t> wedge;
     std::vector<int2> lvtab;
     std::vector<SbItem> items;          // claim order: a topological order of the waits
     std::vector<int4> waits;            // before level x, superblock y has finished z levels

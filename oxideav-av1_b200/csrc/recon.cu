@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "host_pool.h"
 #include "itx.cuh"
 
 namespace av1g {
@@ -97,9 +98,15 @@ av1g_status recon_run(const av1g_recon_job* jobs, int n, cudaStream_t s, std::st
     size_t total = 0;
     for (int i = 0; i < n; i++) total += jobs[i].num_tus > 0 ? jobs[i].num_tus : 0;
     // TUs bucketed by (size, type) so the threads of a warp run one butterfly
-    // network: a counting sort, stable in (job, decode order)
+    // network: a counting sort, stable in (job, decode order), whose two passes
+    // helper threads share by runs of TUs of one job (host_pool.h)
     constexpr int kKeys = 19 * 16;
     std::vector<uint32_t> count(kKeys + 1, 0);
+    struct Run {
+        int job, k0, k1, bad;
+        uint32_t at[kKeys];
+    };
+    std::vector<Run> runs;
     for (int i = 0; i < n; i++) {
         const av1g_recon_job& j = jobs[i];
         if (!j.hdr || !j.quant || (j.num_tus > 0 && (!j.tus || !j.coeffs)) || j.num_tus < 0) {
@@ -127,17 +134,40 @@ av1g_status recon_run(const av1g_recon_job* jobs, int n, cudaStream_t s, std::st
             }
             F.planes[p] = PlaneDev{(uint8_t*)pl.data, pl.stride, pw, ph};
         }
-        for (int k = 0; k < j.num_tus; k++) {
-            const av1g_tu& t = j.tus[k];
-            if (t.tx_size >= 19 || t.tx_type >= 16 || t.plane >= h.num_planes) {
-                err = "recon job " + std::to_string(i) + ": TU " + std::to_string(k) + " has an invalid size/type/plane";
-                return AV1G_EINVAL;
-            }
-            count[t.tx_size * 16 + t.tx_type + 1]++;
-        }
+        const int parts = parallel_parts(j.num_tus, 4096);
+        for (int u = 0; u < parts; u++)
+            runs.push_back(Run{i, (int)((long long)j.num_tus * u / parts), (int)((long long)j.num_tus * (u + 1) / parts),
+                               -1, {}});
     }
+    parallel_for((int)runs.size(), (long long)total, [&](int u) {
+        Run& r = runs[u];
+        const av1g_recon_job& j = jobs[r.job];
+        for (int k = r.k0; k < r.k1; k++) {
+            const av1g_tu& t = j.tus[k];
+            if (t.tx_size >= 19 || t.tx_type >= 16 || t.plane >= j.hdr->num_planes) {
+                r.bad = k;
+                return;
+            }
+            r.at[t.tx_size * 16 + t.tx_type]++;
+        }
+    });
+    for (const Run& r : runs)
+        if (r.bad >= 0) {
+            err = "recon job " + std::to_string(r.job) + ": TU " + std::to_string(r.bad) +
+                  " has an invalid size/type/plane";
+            return AV1G_EINVAL;
+        }
     if (total == 0) return AV1G_OK;
-    for (int k = 1; k <= kKeys; k++) count[k] += count[k - 1];  // count[key]: TUs with a smaller key
+    // count[key]: TUs with a smaller key; a run's at[key]: where its own go
+    for (int k = 0; k < kKeys; k++) {
+        uint32_t next = count[k];
+        for (Run& r : runs) {
+            const uint32_t len = r.at[k];
+            r.at[k] = next;
+            next += len;
+        }
+        count[k + 1] = next;
+    }
     // tasks: runs of at most slots_for(tx) TUs of one size; keys are
     // size-major, so the TUs of size tx are [count[16 tx], count[16 tx + 16])
     std::vector<Task> tasks;
@@ -160,11 +190,13 @@ av1g_status recon_run(const av1g_recon_job* jobs, int n, cudaStream_t s, std::st
     e = upload_with(dev, bytes, s, [&](uint8_t* host) {
         memcpy(host, frames.data(), sizeof(ReconFrame) * n);
         TuDev* dst = reinterpret_cast<TuDev*>(host + off_tus);
-        for (int i = 0; i < n; i++)
-            for (int k = 0; k < jobs[i].num_tus; k++) {
-                const av1g_tu& t = jobs[i].tus[k];
-                dst[count[t.tx_size * 16 + t.tx_type]++] = TuDev{t, i};
+        parallel_for((int)runs.size(), (long long)total, [&](int u) {
+            Run& r = runs[u];
+            for (int k = r.k0; k < r.k1; k++) {
+                const av1g_tu& t = jobs[r.job].tus[k];
+                dst[r.at[t.tx_size * 16 + t.tx_type]++] = TuDev{t, r.job};
             }
+        });
         memcpy(host + off_tasks, tasks.data(), sizeof(Task) * tasks.size());
     });
     if (e == cudaSuccess) {
