@@ -14,7 +14,10 @@
 //    seven precomputed matrix-vector products.  The auto-regressive filter
 //    (lag <= 3) reads only earlier rows and earlier samples of the same row,
 //    so samples with equal x + 4y are independent and one warp sweeps the
-//    template in ~350 wavefront steps.
+//    template in ~370 wavefront steps, the two chroma templates' warps a little
+//    behind the luma one's.  The chain of those steps bounds the kernel: 56 us
+//    for any batch of frames (190 us for twelve 4:4:4 frames, 171 us for four
+//    4:2:0 ones with all taps read from shared memory and chroma after luma).
 //  * grain_blend_kernel — every thread owns one chroma-resolution position
 //    and the (1 << ssx) x (1 << ssy) luma samples it covers.  The noise value
 //    of a sample is evaluated in closed form from the template, the random
@@ -28,7 +31,7 @@
 
 namespace av1g {
 
-__constant__ AV1T_GAUSSIAN_SEQUENCE_TYPE c_gauss AV1T_GAUSSIAN_SEQUENCE_DIMS = AV1T_GAUSSIAN_SEQUENCE_INIT;
+__device__ const AV1T_GAUSSIAN_SEQUENCE_TYPE g_gauss AV1T_GAUSSIAN_SEQUENCE_DIMS = AV1T_GAUSSIAN_SEQUENCE_INIT;
 
 namespace {
 
@@ -79,92 +82,175 @@ __device__ __forceinline__ uint16_t row_state(uint16_t seed, int row, int wi) {
 
 __device__ __forceinline__ int r2(int x, int n) { return n ? (x + (1 << (n - 1))) >> n : x; }
 
-// scaling_lookup_fill (film_grain.rs:490-540)
-__device__ void scaling_fill(uint8_t* t, int np, const uint8_t* xv, const uint8_t* yv) {
-    if (np == 0) {
-        for (int v = 0; v < 256; v++) t[v] = 0;
-        return;
-    }
-    for (int v = 0; v < xv[0]; v++) t[v] = yv[0];
+// scaling_lookup_fill (film_grain.rs:490-540) at one value: the first point's
+// scaling below it, the last one's from it on, and between two points the
+// interpolation of the last segment (of positive length) that holds the value
+__device__ int scaling_at(int v, int np, const uint8_t* xv, const uint8_t* yv) {
+    if (np == 0) return 0;
+    if (v >= xv[np - 1]) return yv[np - 1];
+    int r = v < xv[0] ? yv[0] : 0;
     for (int i = 0; i + 1 < np; i++) {
-        int dx = xv[i + 1] - xv[i], dy = yv[i + 1] - yv[i];
-        if (dx <= 0) continue;
-        int delta = dy * ((65536 + (dx >> 1)) / dx);
-        for (int x = 0; x < dx; x++) {
-            int idx = xv[i] + x;
-            if (idx < 256) t[idx] = (uint8_t)clip3(0, 255, yv[i] + ((x * delta + 32768) >> 16));
-        }
+        const int dx = xv[i + 1] - xv[i], x = v - xv[i];
+        if (dx <= 0 || x < 0 || x >= dx) continue;
+        const int delta = (yv[i + 1] - yv[i]) * ((65536 + (dx >> 1)) / dx);
+        r = clip3(0, 255, yv[i] + ((x * delta + 32768) >> 16));
     }
-    for (int v = xv[np - 1]; v < 256; v++) t[v] = yv[np - 1];
+    return r;
 }
 
-// AR filter of one template by one warp: wavefront over t = x + 4y, the
-// coefficients (minus 128) held in registers.
-template <int LAG>
-__device__ void ar_luma(int16_t* L, const av1g_film_grain& fg, int gmin, int gmax) {
-    constexpr int NC = 2 * LAG * (LAG + 1);
-    int c[NC > 0 ? NC : 1];
-#pragma unroll
-    for (int i = 0; i < NC; i++) c[i] = fg.ar_coeffs_y_plus_128[i] - 128;
-    const int shift = fg.ar_coeff_shift, lane = threadIdx.x & 31;
-    for (int T = 3 + 4 * 3; T <= (LW - 4) + 4 * (LH - 1); T++) {
-        const int ylo = max(3, (T - (LW - 4) + 3) >> 2), yhi = min(LH - 1, (T - 3) >> 2);
-        const int y = ylo + lane;
-        if (y <= yhi) {
-            const int x = T - 4 * y;
-            int s = 0;
-#pragma unroll
-            for (int dr = -LAG; dr <= 0; dr++)
-#pragma unroll
-                for (int dc = -LAG; dc <= LAG; dc++) {
-                    const int pos = (dr + LAG) * (2 * LAG + 1) + dc + LAG;
-                    if (pos < NC) s += L[(y + dr) * LW + x + dc] * c[pos];
-                }
-            L[y * LW + x] = (int16_t)clip3(gmin, gmax, L[y * LW + x] + r2(s, shift));
-        }
-        __syncwarp();
-    }
-}
-
-template <int LAG>
-__device__ void ar_chroma(int16_t* C, const int16_t* L, const uint8_t* coef, const av1g_film_grain& fg, int cw,
-                          int ch, int ssx, int ssy, int gmin, int gmax) {
-    constexpr int NC = 2 * LAG * (LAG + 1);  // the last coefficient weighs the co-located luma
+// AR filter of a w x h template by one warp, in place: a wavefront over
+// T = x + 4y in which lane y % 32 walks row y (a row takes w <= 82 steps and
+// starts four steps after the row above, so a lane is done with row y before
+// row y + 32 starts).  A sample's neighbours stay in registers: the three
+// samples to its left, and for each of the LAG rows above a window of 2 LAG + 1
+// samples that takes in one more per step, shuffled from the lane of the row
+// above: its last output is row y - 1 at x + 3, and its own windows hold row
+// y - 2 and y - 3 there.  So a step's chain is a shuffle and a row's
+// multiplications, 240 cycles at lag 3; reading all taps from shared memory at
+// each step took 600.  The filter leaves the first three rows and
+// the outer three columns as they are; they pass through the same chain unchanged.
+//
+// The chroma warps follow the luma warp through `prog`, the luma steps whose
+// samples are in shared memory: chroma step T weighs luma samples of at most
+// luma step 2 T with 4:2:0, T + w with 4:2:2 and T with 4:4:4.
+// SS: -1 the luma template, else a chroma template, subsampled in SS directions.
+template <int LAG, int SS>
+__device__ void ar_filter(int16_t* C, const int16_t* L, const uint8_t* coef, const av1g_film_grain& fg, int gmin,
+                          int gmax, volatile int* prog) {
+    constexpr bool CHROMA = SS >= 0;
+    constexpr int ssx = SS >= 1, ssy = SS == 2;
+    constexpr int w = ssx ? 44 : LW, h = ssy ? 38 : LH;
+    constexpr int NC = 2 * LAG * (LAG + 1);  // of chroma, coefficient NC weighs the co-located luma
+    constexpr int WN = 2 * LAG + 1, R = LAG > 0 ? LAG : 1, D = LAG > 0 ? 3 - LAG : 0;
     int c[NC + 1];
 #pragma unroll
-    for (int i = 0; i <= NC; i++) c[i] = coef[i] - 128;
-    const bool luma = fg.num_y_points > 0;
-    const int shift = fg.ar_coeff_shift, lane = threadIdx.x & 31;
-    for (int T = 3 + 4 * 3; T <= (cw - 4) + 4 * (ch - 1); T++) {
-        const int ylo = max(3, (T - (cw - 4) + 3) >> 2), yhi = min(ch - 1, (T - 3) >> 2);
-        for (int y = ylo + lane; y <= yhi; y += 32) {
-            const int x = T - 4 * y;
-            int s = 0;
+    for (int i = 0; i < NC; i++) c[i] = coef[i] - 128;
+    c[NC] = CHROMA ? coef[NC] - 128 : 0;
+    const bool luma = CHROMA && fg.num_y_points > 0;
+    const int shift = fg.ar_coeff_shift, half = shift ? 1 << (shift - 1) : 0, lane = threadIdx.x & 31;
+    int win[R][WN];  // win[r][k]: row y - 1 - r at x - LAG + k
+    int left[R];     // left[k]: this row at x - 1 - k
+    // The newest sample of each window comes from the lane above, whose last
+    // step was x + 3 of row y - 1: its output there, and the middle of its windows
+    // (rows y - 2 and y - 3 there).  LAG < 3 windows end at x + LAG and take that
+    // sample D = 3 - LAG steps later.
+    int keep[R][D + 1];  // arrived, not yet in the window
 #pragma unroll
-            for (int dr = -LAG; dr <= 0; dr++)
+    for (int r = 0; r < R; r++) {
+        left[r] = 0;
 #pragma unroll
-                for (int dc = -LAG; dc <= LAG; dc++) {
-                    const int pos = (dr + LAG) * (2 * LAG + 1) + dc + LAG;
-                    if (pos < NC) s += C[(y + dr) * cw + x + dc] * c[pos];
-                }
-            if (luma) {
-                const int lx = ((x - 3) << ssx) + 3, ly = ((y - 3) << ssy) + 3;
-                int l = 0;
-                for (int i = 0; i <= ssy; i++)
-                    for (int j = 0; j <= ssx; j++) l += L[(ly + i) * LW + lx + j];
-                s += r2(l, ssx + ssy) * c[NC];
+        for (int k = 0; k < WN; k++) win[r][k] = 0;
+#pragma unroll
+        for (int k = 0; k < D; k++) keep[r][k] = 0;
+    }
+    constexpr int last = w - 1 + 4 * (h - 1);
+    int out = 0, y = lane, x = -4 * lane, seen = 0;
+    // the step's noise and the luma around it, read one step ahead
+    int g = 0, l[4] = {0, 0, 0, 0};
+    // (outside the template some sample is read that nothing uses: no branch)
+    auto fetch = [&](int yy, int xx) {
+        const int yi = min(yy, h - 1), xi = max(xx, 0);
+        g = C[yi * w + xi];
+        if (CHROMA) {
+            const int yl = max(yi, 3), xl = min(max(xi, 3), w - 4);
+            const int16_t* p = L + (ssy ? 2 * yl - 3 : yl) * LW + (ssx ? 2 * xl - 3 : xl);
+            l[0] = p[0];
+            if (ssx) l[1] = p[1];
+            if (ssy) {
+                l[2] = p[LW];
+                l[3] = p[LW + 1];
             }
-            C[y * cw + x] = (int16_t)clip3(gmin, gmax, C[y * cw + x] + r2(s, shift));
         }
+    };
+    fetch(y, x);
+    // seven steps per round: a window's samples come round to the same registers
+#pragma unroll 7
+    for (int T = 0; T <= last; T++) {
+        const int gc = g;
+        const int lc = !luma ? 0 : (SS == 2 ? (l[0] + l[1] + l[2] + l[3] + 2) >> 2 : SS == 1 ? (l[0] + l[1] + 1) >> 1 : l[0]) * c[NC];
+        if (luma) {
+            const int need = min(ssy ? 2 * (T + 1) : ssx ? T + 1 + w : T + 1, LW - 1 + 4 * (LH - 1));
+            if (seen <= need) {
+                while ((seen = *prog) <= need) {}
+                __threadfence_block();
+            }
+        }
+        // the lane's next step: the next sample, or its next row once that starts
+        const bool end = x + 1 >= w;
+        const int yn = end ? y + 32 : y, xn = end ? T + 1 - 4 * (y + 32) : x + 1;
+        fetch(yn, xn);
+        const bool filt = y >= 3 && x >= 3 && x < w - 3;
+        int s = lc + half;
+        if constexpr (LAG > 0) {
+            int in[R];
+            in[0] = __shfl_sync(0xffffffffu, out, (lane + 31) & 31);
+#pragma unroll
+            for (int r = 1; r < LAG; r++) in[r] = __shfl_sync(0xffffffffu, win[r - 1][LAG], (lane + 31) & 31);
+#pragma unroll
+            for (int r = 0; r < LAG; r++) {
+#pragma unroll
+                for (int k = 0; k + 1 < WN; k++) win[r][k] = win[r][k + 1];
+                if constexpr (D == 0) {
+                    win[r][WN - 1] = in[r];
+                } else {
+                    win[r][WN - 1] = keep[r][0];
+#pragma unroll
+                    for (int k = 0; k + 1 < D; k++) keep[r][k] = keep[r][k + 1];
+                    keep[r][D - 1] = in[r];
+                }
+            }
+            // a chain of multiplications per row; the left samples end the last
+#pragma unroll
+            for (int r = LAG - 1; r >= 0; r--) {
+                int q = 0;
+#pragma unroll
+                for (int k = 0; k < WN; k++) q += win[r][k] * c[(LAG - 1 - r) * WN + k];
+                s += q;
+            }
+#pragma unroll
+            for (int k = LAG - 1; k >= 0; k--) s += left[k] * c[LAG * WN + LAG - 1 - k];
+        }
+        out = filt ? clip3(gmin, gmax, gc + (s >> shift)) : gc;
+        if constexpr (LAG > 0) {
+#pragma unroll
+            for (int k = LAG - 1; k > 0; k--) left[k] = left[k - 1];
+            left[0] = out;
+        }
+        if (x >= 0 && y < h) C[y * w + x] = (int16_t)out;
+        if (!CHROMA && (T & 3) == 3) {
+            __threadfence_block();
+            __syncwarp();
+            if (lane == 0) *prog = T + 1;
+        }
+        x = xn;
+        y = yn;
+    }
+    if (!CHROMA) {
+        __threadfence_block();
         __syncwarp();
+        if (lane == 0) *prog = last + 1;
     }
 }
 
-__global__ void __launch_bounds__(128) grain_template_kernel(const FrameDev* __restrict__ frames,
+template <int SS>
+__device__ void ar_filter_lag(int16_t* C, const int16_t* L, const uint8_t* coef, const av1g_film_grain& fg, int gmin,
+                              int gmax, volatile int* prog) {
+    switch (fg.ar_coeff_lag) {
+        case 0: ar_filter<0, SS>(C, L, coef, fg, gmin, gmax, prog); break;
+        case 1: ar_filter<1, SS>(C, L, coef, fg, gmin, gmax, prog); break;
+        case 2: ar_filter<2, SS>(C, L, coef, fg, gmin, gmax, prog); break;
+        default: ar_filter<3, SS>(C, L, coef, fg, gmin, gmax, prog); break;
+    }
+}
+
+constexpr int kTmplThreads = 256;
+
+__global__ void __launch_bounds__(kTmplThreads) grain_template_kernel(const FrameDev* __restrict__ frames,
                                                              const int32_t* __restrict__ starts, int n, int total) {
     __shared__ int16_t T[3][LH * LW];
+    __shared__ int prog;
     __shared__ int16_t gauss[2048];  // the lanes draw different entries: shared, not constant, memory
-    for (int i = threadIdx.x; i < 2048; i += blockDim.x) gauss[i] = (int16_t)c_gauss[i];
+    for (int i = threadIdx.x; i < 2048; i += blockDim.x) gauss[i] = (int16_t)__ldg(&g_gauss[i]);
     for (int t = blockIdx.x; t < total; t += gridDim.x) {
         int f = find_frame(starts, n, t);
         const FrameDev& F = frames[f];
@@ -174,17 +260,17 @@ __global__ void __launch_bounds__(128) grain_template_kernel(const FrameDev* __r
         const int shift = 12 - bd + fg.grain_scale_shift;
         const int cw = ssx ? 44 : 82, ch = ssy ? 38 : 73;
         __syncthreads();
-        if (threadIdx.x < 3) {
-            int p = threadIdx.x;
-            uint8_t* lut = F.grain_lut + p * 256;
+        for (int i = threadIdx.x; i < 3 * 256; i += blockDim.x) {
+            const int p = i >> 8, v = i & 255;
+            int r = 0;
             if (p < F.h.num_planes) {
-                if (p == 0 || fg.chroma_scaling_from_luma) scaling_fill(lut, fg.num_y_points, fg.point_y_value, fg.point_y_scaling);
-                else if (p == 1) scaling_fill(lut, fg.num_cb_points, fg.point_cb_value, fg.point_cb_scaling);
-                else scaling_fill(lut, fg.num_cr_points, fg.point_cr_value, fg.point_cr_scaling);
-            } else {
-                for (int v = 0; v < 256; v++) lut[v] = 0;
+                if (p == 0 || fg.chroma_scaling_from_luma) r = scaling_at(v, fg.num_y_points, fg.point_y_value, fg.point_y_scaling);
+                else if (p == 1) r = scaling_at(v, fg.num_cb_points, fg.point_cb_value, fg.point_cb_scaling);
+                else r = scaling_at(v, fg.num_cr_points, fg.point_cr_value, fg.point_cr_scaling);
             }
+            F.grain_lut[i] = (uint8_t)r;
         }
+        if (threadIdx.x == 0) prog = 0;
         // white noise (generate_grain, film_grain.rs:245-300)
         for (int job = threadIdx.x; job < LH + 2 * ch; job += blockDim.x) {
             int p = job < LH ? 0 : (job < LH + ch ? 1 : 2);
@@ -206,25 +292,29 @@ __global__ void __launch_bounds__(128) grain_template_kernel(const FrameDev* __r
             }
         }
         __syncthreads();
-        if (fg.num_y_points > 0 && threadIdx.x < 32) {
-            switch (fg.ar_coeff_lag) {
-                case 0: ar_luma<0>(T[0], fg, gmin, gmax); break;
-                case 1: ar_luma<1>(T[0], fg, gmin, gmax); break;
-                case 2: ar_luma<2>(T[0], fg, gmin, gmax); break;
-                default: ar_luma<3>(T[0], fg, gmin, gmax); break;
+        const int warp = threadIdx.x >> 5;
+        if (warp == 0) {
+            if (fg.num_y_points > 0)
+                ar_filter_lag<-1>(T[0], nullptr, fg.ar_coeffs_y_plus_128, fg, gmin, gmax, &prog);
+        } else if (warp < 3) {
+            if (fg.chroma_scaling_from_luma || fg.num_cb_points > 0 || fg.num_cr_points > 0) {
+                const uint8_t* cf = warp == 1 ? fg.ar_coeffs_cb_plus_128 : fg.ar_coeffs_cr_plus_128;
+                if (ssy) ar_filter_lag<2>(T[warp], T[0], cf, fg, gmin, gmax, &prog);
+                else if (ssx) ar_filter_lag<1>(T[warp], T[0], cf, fg, gmin, gmax, &prog);
+                else ar_filter_lag<0>(T[warp], T[0], cf, fg, gmin, gmax, &prog);
             }
-        }
-        __syncthreads();
-        if (fg.chroma_scaling_from_luma || fg.num_cb_points > 0 || fg.num_cr_points > 0) {
-            int warp = threadIdx.x >> 5;
-            if (warp < 2) {
-                int16_t* C = T[1 + warp];
-                const uint8_t* cf = warp == 0 ? fg.ar_coeffs_cb_plus_128 : fg.ar_coeffs_cr_plus_128;
-                switch (fg.ar_coeff_lag) {
-                    case 0: ar_chroma<0>(C, T[0], cf, fg, cw, ch, ssx, ssy, gmin, gmax); break;
-                    case 1: ar_chroma<1>(C, T[0], cf, fg, cw, ch, ssx, ssy, gmin, gmax); break;
-                    case 2: ar_chroma<2>(C, T[0], cf, fg, cw, ch, ssx, ssy, gmin, gmax); break;
-                    default: ar_chroma<3>(C, T[0], cf, fg, cw, ch, ssx, ssy, gmin, gmax); break;
+        } else {
+            // meanwhile the per-stripe block offsets (add_noise_synthesis,
+            // film_grain.rs:604-615)
+            const int h = F.out[0].h;
+            const int nstripes = ((h + 1) / 2 + 15) / 16, nblocks = F.grain_nblocks;
+            for (int s = threadIdx.x - 96; s < nstripes; s += blockDim.x - 96) {
+                uint16_t st = fg.grain_seed;
+                st ^= (uint16_t)((((unsigned)s * 37 + 178) & 255) << 8);
+                st ^= (uint16_t)(((unsigned)s * 173 + 105) & 255);
+                for (int k = 0; k < nblocks; k++) {
+                    st = lfsr_step(st);
+                    F.grain_offs[s * nblocks + k] = (uint8_t)(st >> 8);
                 }
             }
         }
@@ -235,19 +325,6 @@ __global__ void __launch_bounds__(128) grain_template_kernel(const FrameDev* __r
             out[LH * LW + i] = T[1][i];
             out[2 * LH * LW + i] = T[2][i];
         }
-        // per-stripe block offsets (add_noise_synthesis, film_grain.rs:604-615)
-        const int w = F.out[0].w, h = F.out[0].h;
-        const int nstripes = ((h + 1) / 2 + 15) / 16, nblocks = F.grain_nblocks;
-        for (int s = threadIdx.x; s < nstripes; s += blockDim.x) {
-            uint16_t st = fg.grain_seed;
-            st ^= (uint16_t)((((unsigned)s * 37 + 178) & 255) << 8);
-            st ^= (uint16_t)(((unsigned)s * 173 + 105) & 255);
-            for (int k = 0; k < nblocks; k++) {
-                st = lfsr_step(st);
-                F.grain_offs[s * nblocks + k] = (uint8_t)(st >> 8);
-            }
-        }
-        (void)w;
     }
 }
 
@@ -499,7 +576,7 @@ int tiles_grain_blend(const FrameDev& f) {
 
 void launch_grain(const FrameDev* frames, const int32_t* starts_tmpl, const int32_t* starts_blend, int n,
                   int total_tmpl, int total_blend, const StageShape& sh, cudaStream_t s) {
-    if (total_tmpl > 0) grain_template_kernel<<<total_tmpl, 128, 0, s>>>(frames, starts_tmpl, n, total_tmpl);
+    if (total_tmpl > 0) grain_template_kernel<<<total_tmpl, kTmplThreads, 0, s>>>(frames, starts_tmpl, n, total_tmpl);
     if (total_blend > 0) grain_blend_kernel<<<shape_grid(sh, total_blend), 256, 0, s>>>(frames, starts_blend, n, total_blend);
 }
 
