@@ -202,7 +202,7 @@ int stage_tiles(const FrameDev& F, int st, int sr_tile) {
 struct Prepared {
     static constexpr int NS = ST_COUNT + 1;
     Batch b;
-    int n = 0, stage_mask = 0, mode = 0, max_cells = 0;
+    int n = 0, stage_mask = 0, mode = 0, max_prep = 0;
     size_t off_starts = 0, off_pf = 0, off_scratch = 0, total_bytes = 0;
     std::vector<size_t> lf_off, grain_off;
     std::vector<uint8_t> host;  // the uploaded prefix [0, off_scratch)
@@ -238,7 +238,8 @@ av1g_status prepare(const av1g_frame_job* jobs, int n, int stage_mask, int mode,
         const FrameDev& F = P.b.frames[i];
         if ((stage_mask & (1 << ST_DEBLOCK)) && F.do_stage[ST_DEBLOCK]) {
             int cells = cells_deblock(F);
-            P.max_cells = cells > P.max_cells ? cells : P.max_cells;
+            const int prep = tiles_lf_prep(F);
+            P.max_prep = prep > P.max_prep ? prep : P.max_prep;
             P.lf_off[i] = P.off_scratch + scratch;
             scratch += ((size_t)cells * 2 + 255) & ~(size_t)255;
         }
@@ -297,12 +298,12 @@ int launch_all(const Prepared& P, const uint8_t* dev, cudaStream_t s) {
     const int32_t* hpf = (const int32_t*)(P.host.data() + P.off_pf);
     int nl = 0;
     auto launch_stage = [&](int st, const FrameDev* fr, const int32_t* starts, const int32_t* starts_tmpl, int nn,
-                            int total, int total_tmpl, int cells) {
+                            int total, int total_tmpl, int prep) {
         static const char* const names[ST_COUNT] = {"av1g deblock", "av1g cdef", "av1g superres",
                                                      "av1g loop restoration", "av1g film grain"};
         NvtxRange range(names[st]);
         switch (st) {
-            case ST_DEBLOCK: if (total) { launch_deblock(fr, starts, nn, total, cells, P.shape[st], s); nl += 2; } break;
+            case ST_DEBLOCK: if (total) { launch_deblock(fr, starts, nn, total, prep, P.shape[st], s); nl += 2; } break;
             case ST_CDEF: if (total) { launch_cdef(fr, starts, nn, total, P.shape[st], s); nl++; } break;
             case ST_SUPERRES: if (total) { launch_superres(fr, starts, nn, total, P.shape[st], s); nl++; } break;
             case ST_LR: if (total) { launch_lr(fr, starts, nn, total, P.shape[st], s); nl++; } break;
@@ -316,11 +317,11 @@ int launch_all(const Prepared& P, const uint8_t* dev, cudaStream_t s) {
         if (!(P.stage_mask & (1 << st))) continue;
         if (P.mode == AV1G_MODE_BATCHED) {
             launch_stage(st, dframes, ds + st * (n + 1), ds + ST_COUNT * (n + 1), n, P.totals[st], P.totals[ST_COUNT],
-                         P.max_cells);
+                         P.max_prep);
         } else {
             for (int i = 0; i < n; i++)
                 launch_stage(st, dframes + i, dpf + (i * NS + st) * 2, dpf + (i * NS + ST_COUNT) * 2, 1,
-                             hpf[(i * NS + st) * 2 + 1], hpf[(i * NS + ST_COUNT) * 2 + 1], cells_deblock(P.b.frames[i]));
+                             hpf[(i * NS + st) * 2 + 1], hpf[(i * NS + ST_COUNT) * 2 + 1], tiles_lf_prep(P.b.frames[i]));
         }
     }
     return nl;
@@ -563,7 +564,7 @@ av1g_status av1g_autotune_postfilter(const av1g_frame_job* jobs, int32_t n, void
     auto starts = [&](int stage) { return ds + stage * (n + 1); };
     auto launch = [&](int stage, const StageShape& sh, int total) {
         switch (stage) {
-            case ST_DEBLOCK: launch_deblock(fr, starts(stage), n, total, P.max_cells, sh, s); break;
+            case ST_DEBLOCK: launch_deblock(fr, starts(stage), n, total, P.max_prep, sh, s); break;
             case ST_CDEF: launch_cdef(fr, starts(stage), n, total, sh, s); break;
             case ST_SUPERRES: launch_superres(fr, starts(stage), n, total, sh, s); break;
             case ST_LR: launch_lr(fr, starts(stage), n, total, sh, s); break;

@@ -125,7 +125,7 @@ av1g_status load_shapes(const char* path, std::string& err);
 // Stage launchers (one per .cu file).  Each takes the batch's device
 // FrameDev array, the stage's tile-start array (n+1 entries, device), the
 // total tile count and the launch shape.
-void launch_deblock(const FrameDev* frames, const int32_t* starts, int n, int total, int max_cells,
+void launch_deblock(const FrameDev* frames, const int32_t* starts, int n, int total, int max_prep,
                     const StageShape& sh, cudaStream_t s);
 void launch_cdef(const FrameDev* frames, const int32_t* starts, int n, int total, const StageShape& sh,
                  cudaStream_t s);
@@ -139,6 +139,7 @@ void launch_grain(const FrameDev* frames, const int32_t* starts_tmpl, const int3
 // Host-side tile counts (must match the kernels' tile decomposition).
 int tiles_deblock(const FrameDev& f);
 int cells_deblock(const FrameDev& f);  // 4x4 cells over all planes (deblock scratch: 2 bytes each)
+int tiles_lf_prep(const FrameDev& f);  // CTAs of the edge-code pass
 int tiles_cdef(const FrameDev& f);
 int tiles_superres(const FrameDev& f, int tile);
 int tiles_lr(const FrameDev& f);
