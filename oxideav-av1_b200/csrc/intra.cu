@@ -550,7 +550,9 @@ __device__ __forceinline__ void residual_task(const G& g, S& s, const IntraFrame
 
 struct Prog {
     int cls, bits;
-    uint16_t* cp;       // the lane's first four samples in the copy
+    // places in the copy are kept as indexes: a pointer carried through a
+    // record would be a 64-bit generic one
+    int cp;             // the lane's first four samples in the copy
     uint8_t* out;       // and in HBM
     int cs, cstep, ostep;  // copy row pitch; from the first four samples to the second
     int ok;             // bit 0 / 1: the first / second four exist; bit 2 / 3: and lie inside the plane
@@ -564,25 +566,24 @@ struct Prog {
     uint32_t tap[2], flt[2];
     // prediction taps of the two groups: places in the edge arrays, weights
     uint32_t px[2], wt[2];
-    uint16_t* tp;       // the TU's first sample in the copy
+    int tp;             // the TU's first sample in the copy
 };
 
 // flt: k0 | k1 << 4 | k2 << 8 | (place << 16) | bits 13 / 14: tap -2 / -1 is
 // the corner | bit 15: upsampled (place holds the interpolated sample, the
 // next one the sample itself) | bit 31: the element exists
 __device__ __forceinline__ void fast_decode(Prog& d, const TuRec* rec, const IntraFrame& F, const SbCtx& c,
-                                            uint16_t* cache, const int32_t* __restrict__ pool, int lane) {
+                                            const int32_t* __restrict__ pool, int lane) {
     constexpr int E = WScr::E;
     const TuHead t = rec->h;
     const PlaneDev& P = F.planes[t.plane];
     const int LW = t.dims & 15, LH = t.dims >> 4, W = 1 << LW, H = 1 << LH, Q = 1 << (LW + LH - 2);
     const int hbd = F.hbd, cs = c.cs[t.plane];
     const int q = lane < Q ? lane : 0, i = q >> (LW - 2), j = (q << 2) & (W - 1), rows = 128 >> LW;
-    uint16_t* tp = cache + t.coff;
     d.cls = t.cls;
     d.bits = t.bits;
-    d.tp = tp;
-    d.cp = tp + i * cs + j;
+    d.tp = t.coff;
+    d.cp = t.coff + i * cs + j;
     d.cs = cs;
     d.cstep = rows * cs;
     d.ostep = rows * P.stride;
@@ -708,19 +709,40 @@ __device__ __forceinline__ void fast_decode(Prog& d, const TuRec* rec, const Int
     }
 }
 
-__device__ __forceinline__ void fast_run(const Prog& d, WScr& s, const IntraFrame& F, const SbCtx& c,
-                                         const uint16_t* cache, const Tables& tb, int lane) {
+// Four predicted samples: curr_frame_step3_merge (cdf.rs:17398-17470),
+// Clip1(pred + residual), to the copy and to HBM (other superblocks read them
+// once this level is published).  ok: bit 0 they exist, bit 2 they lie inside
+// the plane.
+__device__ __forceinline__ void put4(int v0, int v1, int v2, int v3, const int4& r, int maxv, uint16_t* cache, int cp,
+                                     uint8_t* out, int ok, int hbd) {
+    v0 = __viaddmin_s32_relu(v0, r.x, maxv);
+    v1 = __viaddmin_s32_relu(v1, r.y, maxv);
+    v2 = __viaddmin_s32_relu(v2, r.z, maxv);
+    v3 = __viaddmin_s32_relu(v3, r.w, maxv);
+    const uint2 pk = make_uint2(__byte_perm(v0, v1, 0x5410), __byte_perm(v2, v3, 0x5410));
+    if (ok & 1) *reinterpret_cast<uint2*>(cache + cp) = pk;
+    if (ok & 4) {
+        if (hbd) *reinterpret_cast<uint2*>(out) = pk;
+        else *reinterpret_cast<uint32_t*>(out) = __byte_perm(pk.x, pk.y, 0x6420);
+    }
+}
+
+// Each kind is one straight path to its stores: a branch costs a lone warp more
+// than the instructions it skips.
+__device__ __forceinline__ void fast_run(const Prog& d, WScr& s, const IntraFrame& F, const SbCtx& c, uint16_t* cache,
+                                         const Tables& tb, int lane) {
     constexpr int E = WScr::E;
-    const int maxv = (1 << F.bd) - 1, hbd = F.hbd, cs = d.cs;
-    const uint16_t* ed = s.raw;
-    int dc = 0, avg = 0;
+    const int maxv = (1 << F.bd) - 1, hbd = F.hbd, cs = d.cs, tp = d.tp;
+    const bool second = d.ok & 16;
     if (d.cls >= C_D1 && d.cls <= C_D3) {
-        const int v0 = d.tp[(int16_t)(d.src[0] & 0xffff)];
-        const int v1 = d.two ? d.tp[(int16_t)(d.src[1] & 0xffff)] : 0;
+        const int v0 = cache[tp + (int16_t)(d.src[0] & 0xffff)];
+        int v1 = 0;
+        if (d.two) v1 = cache[tp + (int16_t)(d.src[1] & 0xffff)];
         if (d.flt[0] >> 31) s.raw[d.src[0] >> 16] = (uint16_t)v0;
         if (d.two && d.flt[1] >> 31) s.raw[d.src[1] >> 16] = (uint16_t)v1;
         if (lane == 0) s.raw[E + 3] = (uint16_t)v0;
         __syncwarp();
+        int ed = 0;  // raw, or fin 2 E further
         if (d.bits & R_EDGE) {
             // corner filter, intra_edge_filter (cdf.rs:2760) or
             // intra_edge_upsample (cdf.rs:2700) of both edges at once
@@ -733,177 +755,177 @@ __device__ __forceinline__ void fast_run(const Prog& d, WScr& s, const IntraFram
                 int m2 = s.raw[ta & 0xff], m1 = s.raw[(ta >> 8) & 0xff], p1 = s.raw[(ta >> 16) & 0xff], p2 = s.raw[ta >> 24];
                 int v = x ? v1 : v0;
                 if (d.bits & R_CORNER) {
-                    if (fl & (1u << 13)) m2 = fc;
-                    if (fl & (1u << 14)) m1 = fc;
-                    if (x == 0 && lane == 0) v = fc;
+                    m2 = fl & (1u << 13) ? fc : m2;
+                    m1 = fl & (1u << 14) ? fc : m1;
+                    if (x == 0) v = lane == 0 ? fc : v;
                 }
                 const bool up = fl & (1u << 15);
                 const int k0 = up ? -1 : (int)(fl & 15), k1 = up ? 9 : (int)(fl >> 4) & 15, k2 = up ? 9 : (int)(fl >> 8) & 31;
                 const int k3 = up ? -1 : k1, k4 = up ? 0 : k0;
-                const int f = clip3(0, maxv, (k0 * m2 + k1 * m1 + k2 * v + k3 * p1 + k4 * p2 + 8) >> 4);
+                const int f = __vimin_s32_relu((k0 * m2 + k1 * m1 + k2 * v + (k3 * p1 + k4 * p2 + 8)) >> 4, maxv);
                 const int place = (fl >> 16) & 0x7fff;
-                if (fl >> 31) {
-                    s.fin[place] = (uint16_t)f;
-                    if (up) s.fin[place + 1] = (uint16_t)v;
-                }
+                if (fl >> 31) s.fin[place] = (uint16_t)f;
+                if (up) s.fin[place + 1] = (uint16_t)v;
                 if (x == 0 && lane == 0) s.fin[E + (d.bits & R_UPL ? 2 : 3)] = (uint16_t)v;  // the left edge's corner
             }
-            ed = s.fin;
+            ed = (int)(s.fin - s.raw);
             __syncwarp();
+        }
+        const uint16_t* e0 = s.raw + ed;
+#pragma unroll
+        for (int x = 0; x < 2; x++) {
+            if (x && !second) break;
+            const uint32_t px = d.px[x], wt = d.wt[x];
+            int v[4];
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const uint16_t* a = e0 + ((px >> (8 * e)) & 0xff);
+                const int lo = a[0], hi = a[1], w = (wt >> (8 * e)) & 0xff;
+                v[e] = lo + (((hi - lo) * w + 16) >> 5);
+            }
+            put4(v[0], v[1], v[2], v[3], x ? d.r1 : d.r0, maxv, cache, d.cp + x * d.cstep, d.out + (x ? d.ostep : 0),
+                 d.ok >> x, hbd);
         }
     } else if (d.cls == C_DC) {
         // predict_intra_dc_pred (cdf.rs:1348); a missing edge has length 0.
         // The quotient by the reciprocal is exact: sum + n / 2 < 2^20, n <= 128.
         int part = 0;
-        if (d.src[0] != -0x8000) part = d.tp[d.src[0]];
-        if (d.src[1] != -0x8000) part += d.tp[d.src[1]];
+        if (d.src[0] != -0x8000) part = cache[tp + d.src[0]];
+        if (d.src[1] != -0x8000) part += cache[tp + d.src[1]];
         const unsigned n = d.px[1], sum = __reduce_add_sync(0xffffffffu, part);
-        dc = n == 0 ? (maxv + 1) >> 1 : __umulhi(sum + (n >> 1), d.px[0]);
-        if (d.bits & R_CFL) {
+        const int dc = n == 0 ? (maxv + 1) >> 1 : __umulhi(sum + (n >> 1), d.px[0]);
+        if (!(d.bits & R_CFL)) {
+            put4(dc, dc, dc, dc, d.r0, maxv, cache, d.cp, d.out, d.ok, hbd);
+            if (second) put4(dc, dc, dc, dc, d.r1, maxv, cache, d.cp + d.cstep, d.out + d.ostep, d.ok >> 1, hbd);
+        } else {
             // predict_chroma_from_luma_into_curr_frame (cdf.rs:17256-17340)
             const int ssx = F.ssx, ssy = F.ssy, ycs = c.cs[0];
             const int cx = d.flt[0] & 0xffff, cy = d.flt[0] >> 16;
-            const uint16_t* Y = cache + c.off[0] - c.rect[0].y * ycs - c.rect[0].x;
+            const int Y = c.off[0] - c.rect[0].y * ycs - c.rect[0].x;
+            int xs[4], l[2][4] = {};
+#pragma unroll
+            for (int e = 0; e < 4; e++) xs[e] = min((int)(d.tap[0] + e) << ssx, cx);
             part = 0;
-#pragma unroll 1
+#pragma unroll
             for (int x = 0; x < 2; x++) {
-                if (!((d.ok >> x) & 1)) break;
-                const uint16_t* yp = Y + min((int)(d.tap[1] + x * d.wt[1]) << ssy, cy) * ycs;
-                int v[4];
+                if (x && !second) break;
+                const int yp = Y + min((int)(d.tap[1] + x * d.wt[1]) << ssy, cy) * ycs;
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
-                    const uint16_t* p = yp + min((int)(d.tap[0] + e) << ssx, cx);
+                    const uint16_t* p = cache + yp + xs[e];
                     if (ssx) {
                         uint32_t w = *reinterpret_cast<const uint32_t*>(p);  // two samples below 4096: no carry
                         if (ssy) w += *reinterpret_cast<const uint32_t*>(p + ycs);
-                        v[e] = (int)((w & 0xffff) + (w >> 16)) << (2 - ssy);
+                        l[x][e] = (int)((w & 0xffff) + (w >> 16)) << (2 - ssy);
                     } else {
-                        v[e] = ssy ? (p[0] + p[ycs]) << 2 : p[0] << 3;
+                        l[x][e] = ssy ? (p[0] + p[ycs]) << 2 : p[0] << 3;
                     }
-                    part += v[e];
+                    part += l[x][e];
                 }
-                *reinterpret_cast<uint2*>(s.buf + 4 * lane + 128 * x) =
-                    make_uint2((uint32_t)v[0] | (uint32_t)v[1] << 16, (uint32_t)v[2] | (uint32_t)v[3] << 16);
             }
+            if (!(d.ok & 1)) part = 0;  // this lane repeats another's samples
             const unsigned lsum = __reduce_add_sync(0xffffffffu, part);
-            avg = (int)((lsum + (1u << (d.wt[0] - 1))) >> d.wt[0]);
-        }
-    } else if (d.cls == C_FI) {
-        // predict_intra_recursive (cdf.rs:2145): 4x2 cells, wavefront over
-        // i2 + j4; eight lanes per cell, four lanes groups on a diagonal.  The
-        // edges lie in place around the block, so every cell reads the same way.
-        const int W4 = d.px[1], H2 = d.wt[0], o = lane & 7;
-        const uint2 tw = *reinterpret_cast<const uint2*>(tb.fi[d.px[0]][o]);
-        auto tap = [&](int q) { return (int)(int8_t)((q < 4 ? tw.x : tw.y) >> (8 * (q & 3))); };
-        const int w0 = tap(0), w1 = tap(1), w2 = tap(2), w3 = tap(3), w4 = tap(4), w5 = tap(5), w6 = tap(6);
-        const int oo = (o >> 2) * cs + (o & 3);
-#pragma unroll 1
-        for (int dd = 0; dd < W4 + H2 - 1; dd++) {
-#pragma unroll 1
-            for (int i2 = max(0, dd - (W4 - 1)) + (lane >> 3); i2 <= min(dd, H2 - 1); i2 += 4) {
-                uint16_t* cell = d.tp + (i2 << 1) * cs + ((dd - i2) << 2);
-                const uint16_t* up = cell - cs;
-                const int acc = w0 * up[-1] + w1 * up[0] + w2 * up[1] + w3 * up[2] + w4 * up[3] + w5 * cell[-1] +
-                                w6 * cell[cs - 1];
-                cell[oo] = (uint16_t)clip3(0, maxv, acc >= 0 ? (acc + 8) >> 4 : -(((-acc) + 8) >> 4));
-            }
-            __syncwarp();
-        }
-    }
-    int4 rv = d.r0;
-    uint16_t* cp = d.cp;
-    uint8_t* out = d.out;
-    uint32_t px = d.px[0], wt = d.wt[0];
-#pragma unroll 1
-    for (int x = 0;; x++) {
-        int v[4];
-        if (d.cls >= C_D1 && d.cls <= C_D3) {
+            const int avg = (int)((lsum + (1u << (d.wt[0] - 1))) >> d.wt[0]);
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const uint16_t* a = ed + ((px >> (8 * e)) & 0xff);
-                const int lo = a[0], hi = a[1], w = (wt >> (8 * e)) & 0xff;
-                v[e] = lo + (((hi - lo) * w + 16) >> 5);
-            }
-        } else if (d.cls == C_DC) {
-#pragma unroll
-            for (int e = 0; e < 4; e++) v[e] = dc;
-            if ((d.bits & R_CFL) && ((d.ok >> (2 + x)) & 1)) {
+            for (int x = 0; x < 2; x++) {
+                if (x && !second) break;
+                int v[4];
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
-                    const int al = (int)d.flt[1] * ((int)s.buf[4 * lane + 128 * x + e] - avg);
-                    const int sc = al >= 0 ? (al + 32) >> 6 : -(((-al) + 32) >> 6);
-                    v[e] = min(max(dc + sc, 0), maxv);
+                    const int al = (int)d.flt[1] * (l[x][e] - avg);
+                    const int sc = (al + 32 - (al < 0)) >> 6;  // rounds halves away from zero
+                    v[e] = (d.ok >> (2 + x)) & 1 ? min(max(dc + sc, 0), maxv) : dc;
                 }
+                put4(v[0], v[1], v[2], v[3], x ? d.r1 : d.r0, maxv, cache, d.cp + x * d.cstep,
+                     d.out + (x ? d.ostep : 0), d.ok >> x, hbd);
             }
-        } else if (d.cls == C_PAL) {  // predict_palette (cdf.rs:11907); indices checked on the host
-            v[0] = px & 0xffff;
-            v[1] = px >> 16;
-            v[2] = wt & 0xffff;
-            v[3] = wt >> 16;
-        } else if (d.cls == C_FI || d.cls == C_NONE) {  // in the copy already
-            const uint2 w = *reinterpret_cast<const uint2*>(cp);
-            v[0] = w.x & 0xffff;
-            v[1] = w.x >> 16;
-            v[2] = w.y & 0xffff;
-            v[3] = w.y >> 16;
-        } else {
-            const int j = d.wt[0], i = d.wt[1] + (x ? d.two : 0);
-            const uint2 aw = *reinterpret_cast<const uint2*>(d.tp - cs + j);
-            const int l = d.tp[i * cs - 1];
-            v[0] = aw.x & 0xffff;
-            v[1] = aw.x >> 16;
-            v[2] = aw.y & 0xffff;
-            v[3] = aw.y >> 16;
-            if (d.cls == C_H) {
+        }
+    } else if (d.cls >= C_V && d.cls <= C_PAETH) {
+        const int j = d.wt[0], W = d.px[0], H = d.px[1];
+        const uint2 aw = *reinterpret_cast<const uint2*>(cache + tp - cs + j);
+        const int l0 = cache[tp + (int)d.wt[1] * cs - 1];
+        const int l1 = second ? cache[tp + (int)(d.wt[1] + d.two) * cs - 1] : 0;
+        const int a[4] = {(int)(aw.x & 0xffff), (int)(aw.x >> 16), (int)(aw.y & 0xffff), (int)(aw.y >> 16)};
+        const int corner = cache[tp - cs - 1], ar = cache[tp + W - 1 - cs], lb = cache[tp + (H - 1) * cs - 1];
+        const uint32_t wx = *reinterpret_cast<const uint32_t*>(tb.sm + W - 4 + j);
+        const int wy0 = tb.sm[H - 4 + d.wt[1]], wy1 = second ? tb.sm[H - 4 + d.wt[1] + d.two] : 0;
 #pragma unroll
-                for (int e = 0; e < 4; e++) v[e] = l;
-            } else if (d.cls == C_PAETH) {  // cdf.rs:2077
-                const int corner = d.tp[-cs - 1];
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const int base = v[e] + l - corner;
-                    const int dl = abs(base - l), dt = abs(base - v[e]), dtl = abs(base - corner);
-                    v[e] = (dl <= dt && dl <= dtl) ? l : (dt <= dtl ? v[e] : corner);
-                }
-            } else if (d.cls != C_V) {  // SMOOTH (cdf.rs:2267), SMOOTH_V, SMOOTH_H
-                const int W = d.px[0], H = d.px[1];
-                const uint32_t wx = *reinterpret_cast<const uint32_t*>(tb.sm + W - 4 + j);
-                const int wy = tb.sm[H - 4 + i], ar = d.tp[W - 1 - cs], lb = d.tp[(H - 1) * cs - 1];
+        for (int x = 0; x < 2; x++) {
+            if (x && !second) break;
+            const int l = x ? l1 : l0, wy = x ? wy1 : wy0;
+            int v[4];
+            if (d.cls >= C_SMOOTH && d.cls <= C_SMOOTH_H) {  // SMOOTH (cdf.rs:2267), SMOOTH_V, SMOOTH_H
+                // weights of the two directions, 0 for the one a mode leaves out
+                const int kv = d.cls != C_SMOOTH_H, kh = d.cls != C_SMOOTH_V, sh = 7 + kv + kh;
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
                     const int w = (wx >> (8 * e)) & 0xff;
-                    const int vv = wy * v[e] + (256 - wy) * lb, vh = w * l + (256 - w) * ar;
-                    v[e] = d.cls == C_SMOOTH ? (vv + vh + 256) >> 9 : ((d.cls == C_SMOOTH_V ? vv : vh) + 128) >> 8;
+                    const int vv = wy * (a[e] - lb) + 256 * lb, vh = w * (l - ar) + 256 * ar;
+                    v[e] = ((kv ? vv : 0) + (kh ? vh : 0) + (1 << (sh - 1))) >> sh;
                 }
+            } else if (d.cls == C_PAETH) {  // cdf.rs:2077
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int base = a[e] + l - corner;
+                    const int dl = abs(base - l), dt = abs(base - a[e]), dtl = abs(base - corner);
+                    v[e] = (dl <= dt && dl <= dtl) ? l : (dt <= dtl ? a[e] : corner);
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; e++) v[e] = d.cls == C_V ? a[e] : l;
+            }
+            put4(v[0], v[1], v[2], v[3], x ? d.r1 : d.r0, maxv, cache, d.cp + x * d.cstep, d.out + (x ? d.ostep : 0),
+                 d.ok >> x, hbd);
+        }
+    } else if (d.cls == C_PAL) {  // predict_palette (cdf.rs:11907); indices checked on the host
+        put4(d.px[0] & 0xffff, d.px[0] >> 16, d.wt[0] & 0xffff, d.wt[0] >> 16, d.r0, maxv, cache, d.cp, d.out, d.ok, hbd);
+        if (second)
+            put4(d.px[1] & 0xffff, d.px[1] >> 16, d.wt[1] & 0xffff, d.wt[1] >> 16, d.r1, maxv, cache, d.cp + d.cstep,
+                 d.out + d.ostep, d.ok >> 1, hbd);
+    } else {
+        if (d.cls == C_FI) {
+            // predict_intra_recursive (cdf.rs:2145): 4x2 cells, wavefront over
+            // i2 + j4; eight lanes per cell and a column of cells per eight
+            // lanes (two for 32 wide).  The edges lie in place around the
+            // block, so every cell reads the same way.
+            const int W4 = d.px[1], H2 = d.wt[0], o = lane & 7;
+            const uint2 tw = *reinterpret_cast<const uint2*>(tb.fi[d.px[0]][o]);
+            auto tap = [&](int q) { return (int)(int8_t)((q < 4 ? tw.x : tw.y) >> (8 * (q & 3))); };
+            const int w0 = tap(0), w1 = tap(1), w2 = tap(2), w3 = tap(3), w4 = tap(4), w5 = tap(5), w6 = tap(6);
+            const int oo = (o >> 2) * cs + (o & 3), j4 = lane >> 3;
+            int up = tp + (4 - 2 * cs) * j4 - cs;  // the row above the lane's cell, whose row is dd - j4
+#pragma unroll 1
+            for (int dd = 0; dd < W4 + H2 - 1; dd++) {
+                auto cell = [&](int at) {  // at: the row above it
+                    const uint16_t* q = cache + at;
+                    const int lo = w0 * q[-1] + w1 * q[0] + w2 * q[1] + 8;
+                    const int hi = w3 * q[2] + w4 * q[3] + w5 * q[cs - 1] + w6 * q[2 * cs - 1];
+                    cache[at + cs + oo] = (uint16_t)__vimin_s32_relu((lo + hi) >> 4, maxv);
+                };
+                if (j4 < W4 && (unsigned)(dd - j4) < (unsigned)H2) cell(up);
+                if (W4 > 4 && (unsigned)(dd - j4 - 4) < (unsigned)H2) cell(up + 16 - 8 * cs);
+                up += 2 * cs;
+                __syncwarp();
             }
         }
-        // curr_frame_step3_merge (cdf.rs:17398-17470): Clip1(pred + residual)
-        v[0] = __viaddmin_s32_relu(v[0], rv.x, maxv);
-        v[1] = __viaddmin_s32_relu(v[1], rv.y, maxv);
-        v[2] = __viaddmin_s32_relu(v[2], rv.z, maxv);
-        v[3] = __viaddmin_s32_relu(v[3], rv.w, maxv);
-        // the final samples to the copy and to HBM: other superblocks read
-        // them once this level is published
-        const uint2 pk = make_uint2(__byte_perm(v[0], v[1], 0x5410), __byte_perm(v[2], v[3], 0x5410));
-        if ((d.ok >> x) & 1) *reinterpret_cast<uint2*>(cp) = pk;
-        if ((d.ok >> (2 + x)) & 1) {
-            if (hbd) *reinterpret_cast<uint2*>(out) = pk;
-            else *reinterpret_cast<uint32_t*>(out) = __byte_perm(pk.x, pk.y, 0x6420);
+        // in the copy already
+        const uint2 p0 = *reinterpret_cast<const uint2*>(cache + d.cp);
+        put4(p0.x & 0xffff, p0.x >> 16, p0.y & 0xffff, p0.y >> 16, d.r0, maxv, cache, d.cp, d.out, d.ok, hbd);
+        if (second) {
+            const uint2 p1 = *reinterpret_cast<const uint2*>(cache + d.cp + d.cstep);
+            put4(p1.x & 0xffff, p1.x >> 16, p1.y & 0xffff, p1.y >> 16, d.r1, maxv, cache, d.cp + d.cstep,
+                 d.out + d.ostep, d.ok >> 1, hbd);
         }
-        if (x || !(d.ok & 16)) break;
-        rv = d.r1;
-        cp += d.cstep;
-        out += d.ostep;
-        px = d.px[1];
-        wt = d.wt[1];
     }
 }
 
-// One TU: the edges, the prediction (+ inter-intra blend, + CfL), the residual,
-// all on the shared-memory copy of the superblock, and its final samples to
-// HBM.  A thread computes four horizontally adjacent samples at a time (every
-// TU is at least four wide).
-//
+// The first four residual samples of the thread of rank r in a TU.
+__device__ __forceinline__ int4 first_res(const TuRec* rec, const int32_t* __restrict__ pool, int r) {
+    const int Q = 1 << ((rec->h.dims & 15) + (rec->h.dims >> 4) - 2);
+    if (!(rec->h.bits & R_RES) || r >= Q) return make_int4(0, 0, 0, 0);
+    return __ldg(reinterpret_cast<const int4*>(pool + rec->h.res) + r);
+}
+
 // The general form, for any TU: the large ones (a group of warps each) and what
 // fast_decode does not take (edges past the copy or cut off by the frame's edge,
 // inter-intra blocks, intra block copies, unaligned positions).  One body
@@ -911,7 +933,8 @@ __device__ __forceinline__ void fast_run(const Prog& d, WScr& s, const IntraFram
 // which a body per transform size missed on almost every TU.
 template <class G, class S>
 __device__ __forceinline__ void run_tu(const G& g, S& s, const TuRec* rec, const IntraFrame& F, const SbCtx& c,
-                                       uint16_t* cache, const Tables& tb, const int32_t* __restrict__ pool) {
+                                       uint16_t* cache, const Tables& tb, const int32_t* __restrict__ pool,
+                                       int4 rv) {
     const TuHead t = rec->h;
     const int tid = g.r, pl = t.plane, bd = F.bd, hbd = F.hbd, maxv = (1 << bd) - 1;
     const int LW = t.dims & 15, LH = t.dims >> 4, W = 1 << LW, H = 1 << LH, Q = 1 << (LW + LH - 2);
@@ -1110,8 +1133,8 @@ __device__ __forceinline__ void run_tu(const G& g, S& s, const TuRec* rec, const
 #pragma unroll 1
     for (int q = tid; q < Q; q += G::N) {
         const int i = q >> (LW - 2), j = (q << 2) & (W - 1);
-        int4 rv = make_int4(0, 0, 0, 0);
-        if (t.bits & R_RES) rv = __ldg(rp + q);
+        int4 rn = rv;  // the next round's residual
+        if ((t.bits & R_RES) && q + G::N < Q) rn = __ldg(rp + q + G::N);
         uint16_t* cp = tp + i * cs + j;
         int v[4];
         switch (t.cls) {
@@ -1250,6 +1273,7 @@ __device__ __forceinline__ void run_tu(const G& g, S& s, const TuRec* rec, const
                 }
             }
         }
+        rv = rn;
     }
 }
 
@@ -1546,15 +1570,17 @@ __global__ void __launch_bounds__(kIT, 1) intra_kernel(const IntraFrame* __restr
             int b = 0, m = 0, e = 0;
             Prog d;
             bool fast = false;
+            int4 big = make_int4(0, 0, 0, 0);  // the first large TU's residual
             if (lg < it.nlv) {
                 const int2 cur = level(lg);
                 b = cur.x;
                 m = cur.y & ~kLevelPublished;
                 e = level(lg + 1).x;
+                if (m < e) big = first_res(record(m), res, tid - grp * kGT);
                 if (b + wi < m) {
                     const TuRec* rec = record(b + wi);
                     fast = rec->h.where & W_FAST;
-                    if (fast) fast_decode(d, rec, F, S.sb, cache, res, lane);
+                    if (fast) fast_decode(d, rec, F, S.sb, res, lane);
                 }
             }
             if (lg > 0) {
@@ -1576,17 +1602,18 @@ __global__ void __launch_bounds__(kIT, 1) intra_kernel(const IntraFrame* __restr
                 if (k > b + wi) {
                     const TuRec* rec = record(k);
                     fast = rec->h.where & W_FAST;
-                    if (fast) fast_decode(d, rec, F, S.sb, cache, res, lane);
+                    if (fast) fast_decode(d, rec, F, S.sb, res, lane);
                 }
                 if (fast) fast_run(d, ws, F, S.sb, cache, S.tb, lane);
-                else run_tu(WarpG{lane}, ws, record(k), F, S.sb, cache, S.tb, res);
+                else run_tu(WarpG{lane}, ws, record(k), F, S.sb, cache, S.tb, res, first_res(record(k), res, lane));
                 __syncwarp();
             }
             if (m < e) {
                 const WorkG g{tid - grp * kGT, 4 + grp};
                 for (int k = m; k < e; k++) {
                     if (k > b) g.sync();
-                    run_tu(g, S.s[grp].c, record(k), F, S.sb, cache, S.tb, res);
+                    if (k > m) big = first_res(record(k), res, g.r);
+                    run_tu(g, S.s[grp].c, record(k), F, S.sb, cache, S.tb, res, big);
                 }
             }
             bar_arrive(1 + lg % kGroups, 2 * kGT);
