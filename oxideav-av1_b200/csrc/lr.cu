@@ -25,6 +25,12 @@
 //    reference's weights are zero on even rows of the A/B grid, so those rows
 //    are not computed.
 // Units of type RESTORE_NONE copy the CDEF samples through.
+//
+// Bound by instruction issue (198 thread instructions per sample when every
+// thread worked its tile out for itself, with 64-bit divisions for the box
+// filter's scale): 64 x 1080p 8-bit 1.67 -> 1.38 ms with one thread working out
+// the next tile and the scales in a table.  Four CTAs per SM: five, at 48
+// registers, take 1.50 ms.
 #include <cstddef>
 
 #include "common.cuh"
@@ -40,10 +46,43 @@ constexpr int SH = TH + 2 * H3;
 constexpr int VW = TW + 2 * H3 + 1;           // column-sum row pitch (odd: rows fall on distinct banks)
 constexpr int AR = TH + 2, AP = TW + 2 + 1;   // A/B grid rows / pitch
 
-__constant__ int8_t c_sgr_params[16][4] = {
+constexpr int8_t kSgrParams[16][4] = {
     {2, 12, 1, 4}, {2, 15, 1, 6}, {2, 18, 1, 8}, {2, 21, 1, 9}, {2, 24, 1, 10}, {2, 29, 1, 11},
     {2, 36, 1, 12}, {2, 45, 1, 13}, {2, 56, 1, 14}, {2, 68, 1, 15}, {0, 0, 1, 5}, {0, 0, 1, 8},
     {0, 0, 1, 11}, {0, 0, 1, 14}, {2, 30, 0, 0}, {2, 75, 0, 0}};
+
+// box_filter's scale of one pass of a self-guided set: the radius, the rounded
+// 2^20 / (n^2 eps), n the box's samples, and the p from which
+// z = (p * scale + 2^19) >> 20 reaches 255 (a2 = 256): clamping p to it keeps every
+// product below 2^32 (zsat + scale) and leaves a2 unchanged, so z is computed in
+// 32 bits.
+struct SgrPass {
+    uint32_t r, scale, pcap;
+};
+struct SgrSets {
+    SgrPass pass[16][2];
+};
+constexpr SgrSets make_sgr() {
+    SgrSets t{};
+    for (int s = 0; s < 16; s++)
+        for (int k = 0; k < 2; k++) {
+            const int r = kSgrParams[s][2 * k], eps = kSgrParams[s][2 * k + 1];
+            if (r == 0) continue;
+            const long long n = (2 * r + 1) * (2 * r + 1), n2e = n * n * eps;
+            const uint32_t scale = (uint32_t)(((1LL << 20) + n2e / 2) / n2e), zsat = (255u << 20) - (1u << 19);
+            t.pass[s][k] = SgrPass{(uint32_t)r, scale, (zsat + scale - 1) / scale};
+        }
+    return t;
+}
+__constant__ SgrSets c_sgr = make_sgr();
+
+// A tile: what every thread of its CTA needs, worked out once.  Deriving it
+// takes a few dozen divisions, as many instructions as 40 of the thread's
+// outputs when each of the 256 threads did it for its own 8.
+struct Tile {
+    int frame, plane, x0, y0, tw, th, sstart, send, pw, ph;
+    av1g_lr_unit u;
+};
 
 struct Smem {
     uint16_t src[SH * SP];
@@ -52,7 +91,7 @@ struct Smem {
     int B[AR * AP];
     uint16_t A[AR * AP];
     uint16_t a2lut[256];
-    int F0[TH * TW];
+    Tile tile[2];  // the current one, and the next one while it is worked out
 };
 // The Wiener intermediate ((TH + 6) x TW ints) spans the adjacent v1 and v2 arrays.
 static_assert((TH + 6) * TW <= 2 * AR * VW, "Wiener intermediate does not fit");
@@ -85,17 +124,11 @@ __device__ __forceinline__ int count_units(int us, int sz) {
 // instead of 2R + 1; the runs have fixed lengths so the loops unroll and the
 // coefficient arithmetic of neighbouring positions overlaps.
 template <int R, bool HBD>
-__device__ void box_coeffs(Smem& s, int th, int tw, int bd, int eps, int y0) {
+__device__ void box_coeffs(Smem& s, int th, int tw, int bd, const SgrPass& ps, int y0) {
     constexpr bool ODD = R == 2;
     constexpr int n = (2 * R + 1) * (2 * R + 1);
-    const long long n2e = (long long)n * n * eps;
-    const unsigned sm = (unsigned)(((1LL << 20) + n2e / 2) / n2e);
+    const unsigned sm = ps.scale, pcap = ps.pcap;
     constexpr int one_over_n = ((1 << 12) + n / 2) / n;
-    // z = (p * sm + 2^19) >> 20 reaches 255 (a2 = 256) once p * sm >= zsat;
-    // clamping p to the first such value keeps every product below 2^32
-    // (zsat + sm) and leaves a2 unchanged, so z is computed in 32 bits
-    constexpr unsigned zsat = (255u << 20) - (1u << 19);
-    const unsigned pcap = (zsat + sm - 1) / sm;
     const int sa = 2 * (bd - 8), sb = bd - 8;
     const int vw = tw + 2 * H3;
     const int rows = th + 2;
@@ -238,54 +271,68 @@ __device__ __forceinline__ void box_weight4(const Smem& s, int i, int j0, const 
     }
 }
 
-__global__ void __launch_bounds__(kLrThreads) lr_kernel(const FrameDev* __restrict__ frames,
+// Tile t of the batch: its frame, plane, stripe half, column tile and
+// restoration unit (derive_block_geometry, loop_restoration.rs:370-428).
+__device__ void plan_tile(Tile& T, const FrameDev* __restrict__ frames, const int32_t* __restrict__ starts, int n,
+                          int t) {
+    const int f = find_frame(starts, n, t);
+    const FrameDev& F = frames[f];
+    const av1g_frame_header& h = F.h;
+    int local = t - starts[f];
+    int plane = 0, stripe = 0, half = 0, ct = 0;
+    for (int p = 0; p < h.num_planes; p++) {
+        if (h.lr_type[p] == 0) continue;
+        const int pw = r2u(h.upscaled_width, p ? h.subsampling_x : 0);
+        const int nct = (pw + tile_w(h, p) - 1) / tile_w(h, p);
+        const int halves = 2 >> (p ? h.subsampling_y : 0);
+        const int cnt = nct * halves * n_stripes(h, p);
+        if (local < cnt) {
+            plane = p;
+            ct = local % nct;
+            half = (local / nct) % halves;
+            stripe = local / (nct * halves);
+            break;
+        }
+        local -= cnt;
+    }
+    const int ssx = plane ? h.subsampling_x : 0, ssy = plane ? h.subsampling_y : 0;
+    const int pw = r2u(h.upscaled_width, ssx), ph = r2u(h.frame_height, ssy);
+    const int tw = tile_w(h, plane), x0 = ct * tw;
+    const int sstart = (-8 + stripe * 64) >> ssy, send = sstart + (64 >> ssy) - 1;
+    const int y0 = max(0, sstart + half * TH), y1 = min(min(ph, send + 1), sstart + half * TH + TH);
+    const int us = h.lr_unit_size[plane] > 0 ? h.lr_unit_size[plane] : 1;
+    const int ur = min(count_units(us, ph) - 1, (((max(0, sstart) << ssy) + 8) >> ssy) / us);
+    const int uc = min(count_units(us, pw) - 1, x0 / us);
+    av1g_lr_unit u{};
+    if (F.lr_units[plane] && ur < F.lr_unit_rows[plane] && uc < F.lr_unit_cols[plane])
+        u = F.lr_units[plane][ur * F.lr_unit_cols[plane] + uc];
+    T = Tile{f, plane, x0, y0, min(x0 + tw, pw) - x0, y1 - y0, sstart, send, pw, ph, u};
+}
+
+__global__ void __launch_bounds__(kLrThreads, 4) lr_kernel(const FrameDev* __restrict__ frames,
                                                  const int32_t* __restrict__ starts, int n, int total) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem& s = *reinterpret_cast<Smem*>(smem_raw);
     for (int z = threadIdx.x; z < 256; z += blockDim.x)
         s.a2lut[z] = (uint16_t)(z == 0 ? 1 : ((z << 8) + z / 2) / (z + 1));
-    for (int t = blockIdx.x; t < total; t += gridDim.x) {
-        int f = find_frame(starts, n, t);
-        const FrameDev& F = frames[f];
-        const av1g_frame_header& h = F.h;
-        int local = t - starts[f];
-        int plane = 0, stripe = 0, half = 0, ct = 0;
-        for (int p = 0; p < h.num_planes; p++) {
-            if (h.lr_type[p] == 0) continue;
-            int pw = r2u(h.upscaled_width, p ? h.subsampling_x : 0);
-            int nct = (pw + tile_w(h, p) - 1) / tile_w(h, p);
-            int halves = 2 >> (p ? h.subsampling_y : 0);
-            int cnt = nct * halves * n_stripes(h, p);
-            if (local < cnt) {
-                plane = p;
-                ct = local % nct;
-                half = (local / nct) % halves;
-                stripe = local / (nct * halves);
-                break;
-            }
-            local -= cnt;
-        }
-        const int ssx = plane ? h.subsampling_x : 0, ssy = plane ? h.subsampling_y : 0;
-        const int pw = r2u(h.upscaled_width, ssx), ph = r2u(h.frame_height, ssy);
-        const int tw_ = tile_w(h, plane);
-        const int x0 = ct * tw_, x1 = min(x0 + tw_, pw);
-        const int sstart = (-8 + stripe * 64) >> ssy, send = sstart + (64 >> ssy) - 1;
-        const int y0 = max(0, sstart + half * TH), y1 = min(min(ph, send + 1), sstart + half * TH + TH);
-        const int tw = x1 - x0, th = y1 - y0;
+    // the next tile is worked out by one thread while the CTA filters the
+    // current one (the first by the same thread ahead of the loop)
+    const bool planner = threadIdx.x == kLrThreads - 32;
+    if (planner && (int)blockIdx.x < total) plan_tile(s.tile[0], frames, starts, n, blockIdx.x);
+    int cur = 0;
+    for (int t = blockIdx.x; t < total; t += gridDim.x, cur ^= 1) {
+        __syncthreads();  // the tile is worked out; the previous one is done with shared memory
+        if (planner && t + (int)gridDim.x < total) plan_tile(s.tile[cur ^ 1], frames, starts, n, t + gridDim.x);
+        const Tile& T = s.tile[cur];
+        const FrameDev& F = frames[T.frame];
+        const int plane = T.plane, pw = T.pw, ph = T.ph, x0 = T.x0, y0 = T.y0, tw = T.tw, th = T.th;
+        const int sstart = T.sstart, send = T.send;
         if (th <= 0) continue;  // uniform across the CTA
-        const int hbd = F.hbd, bd = h.bit_depth;
+        const int hbd = F.hbd, bd = F.h.bit_depth;
         const PlaneDev& C = F.upcdef[plane];
         const PlaneDev& Dq = F.updeb[plane];
         const PlaneDev& O = F.lr[plane];
-        // restoration unit of this tile (derive_block_geometry, loop_restoration.rs:370-428)
-        int us = h.lr_unit_size[plane] > 0 ? h.lr_unit_size[plane] : 1;
-        int urows = count_units(us, ph), ucols = count_units(us, pw);
-        int ur = min(urows - 1, (((max(0, sstart) << ssy) + 8) >> ssy) / us);
-        int uc = min(ucols - 1, x0 / us);
-        av1g_lr_unit u{};
-        if (F.lr_units[plane] && ur < F.lr_unit_rows[plane] && uc < F.lr_unit_cols[plane])
-            u = F.lr_units[plane][ur * F.lr_unit_cols[plane] + uc];
-        __syncthreads();
+        const av1g_lr_unit& u = T.u;
         if (u.type != 1 && u.type != 2) {
             // RESTORE_NONE: copied through, four samples per thread (x0 is a
             // multiple of 32 and plane rows start on 16-byte boundaries, so
@@ -314,7 +361,8 @@ __global__ void __launch_bounds__(kLrThreads) lr_kernel(const FrameDev* __restri
             // every thread issues its (at most 3) loads before it unpacks
             // any, so their latencies overlap
             const int ng = (tw + 8) >> 2, items = (th + 2 * H3) * ng;
-            const unsigned mag = (1u << 16) / ng + 1;  // k / ng for k < 38 * ng
+            // k / ng for k < 38 * ng
+            const unsigned mag = ng == (TW + 8) / 4 ? (1u << 16) / ((TW + 8) / 4) + 1 : (1u << 16) / ng + 1;
             constexpr int PER = (SH * ((TW + 8) >> 2) + kLrThreads - 1) / kLrThreads;
             uint2 q[PER];
 #pragma unroll
@@ -447,49 +495,52 @@ __global__ void __launch_bounds__(kLrThreads) lr_kernel(const FrameDev* __restri
         }
         // self-guided (loop_restoration.rs:485-588)
         const int set = u.sgr_set < 16 ? u.sgr_set : 15;
-        const int r0 = c_sgr_params[set][0], e0 = c_sgr_params[set][1];
-        const int r1 = c_sgr_params[set][2], e1 = c_sgr_params[set][3];
+        const SgrPass &p0 = c_sgr.pass[set][0], &p1 = c_sgr.pass[set][1];
+        const int r0 = p0.r, r1 = p1.r;
         const int w0 = u.sgr_xqd[0], w1 = u.sgr_xqd[1], w2 = 128 - w0 - w1;
-        // outputs in runs of four along a row
-        constexpr int Q = TW / 4;
+        // outputs in runs of four along a row, two runs per thread, the same
+        // in both passes, so that the first pass's outputs stay in registers.
+        // Rows of one parity run together (the first pass weights odd and even
+        // rows differently), so a warp's two rows share a code path.
+        constexpr int Q = TW / 4, RUNS = TH * Q / kLrThreads;
+        const int n_odd = (th + ((y0 & 1) ? 1 : 0)) >> 1;      // rows i with (y0 + i) odd
+        const int odd0 = (y0 & 1) ? 0 : 1;
+        auto run_row = [&](int rk) { return rk < n_odd ? odd0 + 2 * rk : (1 - odd0) + 2 * (rk - n_odd); };
+        int f0[RUNS][4] = {};
         if (r0) {
-            if (bd > 8) box_coeffs<2, true>(s, th, tw, bd, e0, y0);  // r0 is 2 in every set that has it
-            else box_coeffs<2, false>(s, th, tw, bd, e0, y0);
-            // rows of one parity run together (the odd-row and even-row
-            // weightings differ), so a warp's two rows share a code path
-            const int n_odd = (th + ((y0 & 1) ? 1 : 0)) >> 1;      // rows i with (y0 + i) odd
-            const int odd0 = (y0 & 1) ? 0 : 1;
-            for (int k = threadIdx.x; k < th * Q; k += blockDim.x) {
-                const int rk = k / Q, j0 = (k - rk * Q) * 4;
-                const int i = rk < n_odd ? odd0 + 2 * rk : (1 - odd0) + 2 * (rk - n_odd);
-                if (j0 >= tw) continue;
-                int u[4], f[4];
+            if (bd > 8) box_coeffs<2, true>(s, th, tw, bd, p0, y0);  // r0 is 2 in every set that has it
+            else box_coeffs<2, false>(s, th, tw, bd, p0, y0);
 #pragma unroll
-                for (int e = 0; e < 4; e++) u[e] = s.src[(i + H3) * SP + j0 + e + H3];
-                box_weight4(s, i, j0, u, 0, y0, f);
+            for (int e = 0; e < RUNS; e++) {
+                const int k = threadIdx.x + e * kLrThreads, rk = k / Q, j0 = (k - rk * Q) * 4;
+                if (rk >= th || j0 >= tw) continue;
+                const int i = run_row(rk);
+                int uq[4];
 #pragma unroll
-                for (int e = 0; e < 4; e++) s.F0[i * TW + j0 + e] = f[e];
+                for (int q = 0; q < 4; q++) uq[q] = s.src[(i + H3) * SP + j0 + q + H3];
+                box_weight4(s, i, j0, uq, 0, y0, f0[e]);
             }
             __syncthreads();
         }
         if (r1) {  // r1 is 1 in every set that has it
-            if (bd > 8) box_coeffs<1, true>(s, th, tw, bd, e1, y0);
-            else box_coeffs<1, false>(s, th, tw, bd, e1, y0);
+            if (bd > 8) box_coeffs<1, true>(s, th, tw, bd, p1, y0);
+            else box_coeffs<1, false>(s, th, tw, bd, p1, y0);
         }
-        for (int k = threadIdx.x; k < th * Q; k += blockDim.x) {
-            int i = k / Q, j0 = (k - i * Q) * 4;
-            if (j0 >= tw) continue;
-            int u[4], f1[4];
 #pragma unroll
-            for (int e = 0; e < 4; e++) u[e] = s.src[(i + H3) * SP + j0 + e + H3];
-            if (r1) box_weight4(s, i, j0, u, 1, y0, f1);
+        for (int e = 0; e < RUNS; e++) {
+            const int k = threadIdx.x + e * kLrThreads, rk = k / Q, j0 = (k - rk * Q) * 4;
+            if (rk >= th || j0 >= tw) continue;
+            const int i = run_row(rk);
+            int uq[4], f1[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) uq[q] = s.src[(i + H3) * SP + j0 + q + H3];
+            if (r1) box_weight4(s, i, j0, uq, 1, y0, f1);
             int o[4];
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-                int uu = u[e] << 4;
-                int f0 = r0 ? s.F0[i * TW + j0 + e] : uu;
-                int v = w1 * uu + w0 * f0 + w2 * (r1 ? f1[e] : uu);
-                o[e] = clip3(0, maxv, (v + (1 << 10)) >> 11);
+            for (int q = 0; q < 4; q++) {
+                const int uu = uq[q] << 4;
+                const int v = w1 * uu + w0 * (r0 ? f0[e][q] : uu) + w2 * (r1 ? f1[q] : uu);
+                o[q] = clip3(0, maxv, (v + (1 << 10)) >> 11);
             }
             if (j0 + 4 <= tw && !((x0 + j0) & 3)) {  // one aligned vector store
                 uint8_t* row = O.p + (size_t)(y0 + i) * O.stride;
