@@ -203,6 +203,7 @@ struct Prepared {
     static constexpr int NS = ST_COUNT + 1;
     Batch b;
     int n = 0, stage_mask = 0, mode = 0, max_prep = 0;
+    bool full_chroma = false;
     size_t off_starts = 0, off_pf = 0, off_scratch = 0, total_bytes = 0;
     std::vector<size_t> lf_off, grain_off;
     std::vector<uint8_t> host;  // the uploaded prefix [0, off_scratch)
@@ -236,6 +237,7 @@ av1g_status prepare(const av1g_frame_job* jobs, int n, int stage_mask, int mode,
     P.grain_off.assign(n, 0);
     for (int i = 0; i < n; i++) {
         const FrameDev& F = P.b.frames[i];
+        P.full_chroma = P.full_chroma || (F.h.num_planes > 1 && !F.h.subsampling_y);
         if ((stage_mask & (1 << ST_DEBLOCK)) && F.do_stage[ST_DEBLOCK]) {
             int cells = cells_deblock(F);
             const int prep = tiles_lf_prep(F);
@@ -304,7 +306,7 @@ int launch_all(const Prepared& P, const uint8_t* dev, cudaStream_t s) {
         NvtxRange range(names[st]);
         switch (st) {
             case ST_DEBLOCK: if (total) { launch_deblock(fr, starts, nn, total, prep, P.shape[st], s); nl += 2; } break;
-            case ST_CDEF: if (total) { launch_cdef(fr, starts, nn, total, P.shape[st], s); nl++; } break;
+            case ST_CDEF: if (total) { launch_cdef(fr, starts, nn, total, P.full_chroma, P.shape[st], s); nl++; } break;
             case ST_SUPERRES: if (total) { launch_superres(fr, starts, nn, total, P.shape[st], s); nl++; } break;
             case ST_LR: if (total) { launch_lr(fr, starts, nn, total, P.shape[st], s); nl++; } break;
             case ST_GRAIN:
@@ -565,7 +567,7 @@ av1g_status av1g_autotune_postfilter(const av1g_frame_job* jobs, int32_t n, void
     auto launch = [&](int stage, const StageShape& sh, int total) {
         switch (stage) {
             case ST_DEBLOCK: launch_deblock(fr, starts(stage), n, total, P.max_prep, sh, s); break;
-            case ST_CDEF: launch_cdef(fr, starts(stage), n, total, sh, s); break;
+            case ST_CDEF: launch_cdef(fr, starts(stage), n, total, P.full_chroma, sh, s); break;
             case ST_SUPERRES: launch_superres(fr, starts(stage), n, total, sh, s); break;
             case ST_LR: launch_lr(fr, starts(stage), n, total, sh, s); break;
             default:

@@ -127,8 +127,9 @@ av1g_status load_shapes(const char* path, std::string& err);
 // total tile count and the launch shape.
 void launch_deblock(const FrameDev* frames, const int32_t* starts, int n, int total, int max_prep,
                     const StageShape& sh, cudaStream_t s);
-void launch_cdef(const FrameDev* frames, const int32_t* starts, int n, int total, const StageShape& sh,
-                 cudaStream_t s);
+// full_chroma: some frame of the batch has chroma planes of the luma height
+void launch_cdef(const FrameDev* frames, const int32_t* starts, int n, int total, bool full_chroma,
+                 const StageShape& sh, cudaStream_t s);
 void launch_superres(const FrameDev* frames, const int32_t* starts, int n, int total, const StageShape& sh,
                      cudaStream_t s);
 void launch_lr(const FrameDev* frames, const int32_t* starts, int n, int total, const StageShape& sh,
