@@ -29,7 +29,7 @@ StageShape g_shape[ST_COUNT][2] = {
     {{16, 0}, {16, 0}},    // CDEF
     {{16, 512}, {16, 512}},  // superres
     {{8, 0}, {8, 0}},      // loop restoration
-    {{8, 0}, {8, 0}},      // film grain blend
+    {{16, 0}, {16, 0}},    // film grain blend
 };
 
 }  // namespace

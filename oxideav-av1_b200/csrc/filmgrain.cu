@@ -18,14 +18,23 @@
 //    behind the luma one's.  The chain of those steps bounds the kernel: 56 us
 //    for any batch of frames (190 us for twelve 4:4:4 frames, 171 us for four
 //    4:2:0 ones with all taps read from shared memory and chroma after luma).
-//  * grain_blend_kernel — every thread owns one chroma-resolution position
-//    and the (1 << ssx) x (1 << ssy) luma samples it covers.  The noise value
-//    of a sample is evaluated in closed form from the template, the random
-//    offsets of the (at most two) 32-sample blocks that wrote it in each
-//    direction and the 27/17, 17/27 and 23/22 overlap blends, which is exactly
-//    what the reference's materialised noise stripes and noise image hold
+//  * grain_blend_kernel — a tile is a noise stripe (32 luma rows) by 256 luma
+//    columns; a warp takes a chroma-resolution row of it at a time, a lane eight
+//    luma columns.  Those lie in one noise block, so a lane reads its random
+//    offsets once per tile.  The noise value of a sample is evaluated in closed
+//    form from the template, the offsets of the (at most two) blocks that wrote
+//    it in each direction and the 27/17, 17/27 and 23/22 overlap blends, which is
+//    exactly what the reference's materialised noise stripes and noise image hold
 //    (film_grain.rs:599-760).  Chroma is blended first from the un-noised
 //    luma, then luma, as the reference orders it (film_grain.rs:758-828).
+//    A CTA lays the frame's templates out in shared memory, with a scaling table
+//    of one entry per sample value.  Bound by issue and the latency of the
+//    samples' loads: 193 us for four 3840x2160 10-bit 4:2:0 frames and 170 us for
+//    twelve 718p 4:4:4 ones when a thread took four columns, interpolated each
+//    scaling value and reread the frame's parameters after every store; 112 and
+//    87 us with tiles, tables and templates in shared memory; 89 and 67 us with
+//    all of a row's samples asked for at once (2.2 TB/s and 2.3 TB/s of planes
+//    read and written).
 #include "common.cuh"
 #include "av1_spec_tables.h"
 
@@ -328,240 +337,293 @@ __global__ void __launch_bounds__(kTmplThreads) grain_template_kernel(const Fram
     }
 }
 
-// Noise of N adjacent samples of one plane, (y, x0 .. x0 + N - 1): the
-// materialised noiseImage of the reference (film_grain.rs:599-760) in closed
-// form.  x0 is a multiple of N and N divides the 16- or 32-sample noise block,
-// so the group lies in one block: one offset lookup serves all N samples.
-template <int N>
-struct Noise {
-    const int16_t* tmpl;
-    const uint8_t* offs;
-    int nblocks, tw;  // blocks per stripe, template row width
-    int psx, psy, overlap, gmin, gmax;
+// ---- blend ------------------------------------------------------------------
+constexpr int kBlendThreads = 256;
+constexpr int kLumaCols = 8;    // luma columns of a thread: 16 bytes of a high-bit-depth row
+constexpr int kTileGroups = 32;  // threads across a tile: 256 luma columns
+constexpr int kStripe = 32;      // luma rows of a tile, the height of a noise stripe
+constexpr int kWarps = kBlendThreads / 32;
+static_assert(kTileGroups == 32, "a warp is one row of groups");
 
-    __device__ __forceinline__ const int16_t* block_row(int s, int k, int i) const {
-        const int o = offs[s * nblocks + k];
-        const int ox = o >> 4, oy = o & 15;
-        const int pox = psx ? 6 + ox : 9 + ox * 2, poy = psy ? 6 + oy : 9 + oy * 2;
-        return tmpl + (poy + i) * tw + pox;
-    }
-    // noise stripe s, row i, after the horizontal overlap blend
-    __device__ __forceinline__ void stripe(int s, int i, int x0, int (&v)[N]) const {
-        const int bs = psx ? 4 : 5;
-        const int k = x0 >> bs, j0 = x0 & ((1 << bs) - 1);
-        const int16_t* row = block_row(s, k, i) + j0;
-#pragma unroll
-        for (int e = 0; e < N; e++) v[e] = __ldg(row + e);
-        if (overlap && k > 0 && j0 == 0) {
-            const int16_t* old = block_row(s, k - 1, i);
-            if (psx == 0) {  // columns 0 and 1 blend with columns 32 and 33 of the left block
-                v[0] = clip3(gmin, gmax, r2(__ldg(old + 32) * 27 + v[0] * 17, 5));
-                if (N > 1) v[1] = clip3(gmin, gmax, r2(__ldg(old + 33) * 17 + v[1] * 27, 5));
-            } else {  // column 0 blends with column 16 of the left block
-                v[0] = clip3(gmin, gmax, r2(__ldg(old + 16) * 23 + v[0] * 22, 5));
-            }
-        }
-    }
-    __device__ __forceinline__ void noise(int y, int x0, int (&v)[N]) const {
-        const int bs = psy ? 4 : 5;
-        const int s = y >> bs, i = y & ((1 << bs) - 1);
-        stripe(s, i, x0, v);
-        if (overlap && s > 0 && (psy ? i == 0 : i < 2)) {
-            int old[N];
-            stripe(s - 1, psy ? 16 : i + 32, x0, old);
-#pragma unroll
-            for (int e = 0; e < N; e++) {
-                const int m = psy ? old[e] * 23 + v[e] * 22 : (i == 0 ? old[e] * 27 + v[e] * 17 : old[e] * 17 + v[e] * 27);
-                v[e] = clip3(gmin, gmax, r2(m, 5));
-            }
-        }
-    }
+// What the CTA needs of the frame whose tiles it works on.
+struct BlendPlan {
+    PlaneDev in[3], out[3];
+    const uint8_t* offs;
+    int nblocks, hbd, bd, np, ssx, ssy, tcols;
+    int gmin, gmax, overlap, scaling, rnd;
+    int noise[3];             // the plane gets grain
+    int minv, maxv[3];        // clip of the result
+    int luma[3], self[3], add[3];  // the scaling index of a chroma sample
 };
 
-__device__ __forceinline__ int scale_lut(const uint8_t* lut, int index, int bd) {
-    int shift = bd - 8, x = index >> shift;
-    if (bd == 8 || x >= 255) return lut[x < 255 ? x : 255];
-    int rem = index - (x << shift);
-    int a = lut[x], b = lut[x + 1];
-    return a + r2((b - a) * rem, shift);
+struct BlendShared {
+    BlendPlan P;
+    uint32_t tmpl[3][LH * LW / 2];
+    uint8_t lut[3 << 12];  // scaling by sample value, 1 << bit depth entries per plane
+};
+
+// N template samples from sample `at` on, which may be odd.
+template <int N>
+__device__ __forceinline__ void template_row(const uint32_t* __restrict__ t, int at, int (&v)[N]) {
+    const uint32_t* w = t + (at >> 1);
+    const unsigned sel = (at & 1) ? 0x5432u : 0x3210u;
+    uint32_t a = w[0];
+#pragma unroll
+    for (int e = 0; e < N; e += 2) {
+        const uint32_t b = w[e / 2 + 1];
+        const uint32_t u = __byte_perm(a, b, sel);
+        v[e] = (int16_t)u;
+        v[e + 1] = (int)u >> 16;
+        a = b;
+    }
 }
 
-// N samples of a row at x0: one vector access when the group is whole and the
-// row keeps it aligned, else sample by sample (x < w only).
+// Noise of N adjacent samples of a plane subsampled by SX and SY: the
+// materialised noiseImage of the reference (film_grain.rs:599-760) in closed
+// form.  The samples lie in one block of one stripe, from column j on, in the
+// stripe's row i.  `o` holds the random offsets of the block (byte 0), the block
+// to its left (1) and the same two of the stripe above (2, 3).
+template <int N, int SX>
+__device__ __forceinline__ void stripe_row(const BlendPlan& P, const uint32_t* t, int o, bool left, int sy, int i, int j,
+                                           int (&v)[N]) {
+    const int tw = SX ? 44 : LW;
+    const int ox = (o >> 4) & 15, oy = o & 15;
+    template_row<N>(t, ((sy ? 6 + oy : 9 + oy * 2) + i) * tw + (SX ? 6 + ox : 9 + ox * 2) + j, v);
+    if (left && j == 0) {  // the left block's last columns blend into the first ones
+        const int px = (o >> 12) & 15, py = (o >> 8) & 15;
+        const int16_t* old = reinterpret_cast<const int16_t*>(t) + ((sy ? 6 + py : 9 + py * 2) + i) * tw +
+                             (SX ? 6 + px + 16 : 9 + px * 2 + 32);
+        if (SX) {
+            v[0] = clip3(P.gmin, P.gmax, r2(old[0] * 23 + v[0] * 22, 5));
+        } else {
+            v[0] = clip3(P.gmin, P.gmax, r2(old[0] * 27 + v[0] * 17, 5));
+            v[1] = clip3(P.gmin, P.gmax, r2(old[1] * 17 + v[1] * 27, 5));
+        }
+    }
+}
+template <int N, int SX>
+__device__ __forceinline__ void noise_row(const BlendPlan& P, const uint32_t* t, uint32_t o, bool left, bool above, int sy,
+                                          int i, int j, int (&v)[N]) {
+    stripe_row<N, SX>(P, t, o & 0xffff, left, sy, i, j, v);
+    if (above && (sy ? i == 0 : i < 2)) {  // the stripe above's last rows blend into the first ones
+        int old[N];
+        stripe_row<N, SX>(P, t, o >> 16, left, sy, sy ? 16 : i + 32, j, old);
+        const int a = sy ? 23 : (i == 0 ? 27 : 17), b = sy ? 22 : (i == 0 ? 17 : 27);
+#pragma unroll
+        for (int e = 0; e < N; e++) v[e] = clip3(P.gmin, P.gmax, r2(old[e] * a + v[e] * b, 5));
+    }
+}
+
+// N samples of a row at x0, two to a word: one vector access when the group is
+// whole (rows start on 16-byte boundaries), else sample by sample (x < w only).
 template <int N>
-__device__ __forceinline__ void ld_n(const PlaneDev& P, int hbd, int y, int x0, int w, int (&v)[N]) {
+__device__ __forceinline__ void ld_n(const PlaneDev& P, int hbd, int y, int x0, int w, uint32_t (&u)[N / 2]) {
     const uint8_t* row = P.p + (size_t)y * P.stride;
     if (x0 + N <= w) {
         if (hbd) {
-            if constexpr (N == 4) {
-                const uint2 u = *reinterpret_cast<const uint2*>(reinterpret_cast<const uint16_t*>(row) + x0);
-                v[0] = u.x & 0xffff; v[1] = u.x >> 16; v[2] = u.y & 0xffff; v[3] = u.y >> 16;
-                return;
-            } else if constexpr (N == 2) {
-                const uint32_t u = *reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint16_t*>(row) + x0);
-                v[0] = u & 0xffff; v[1] = u >> 16;
-                return;
+            if constexpr (N == 8) {
+                const uint4 q = *reinterpret_cast<const uint4*>(row + 2 * x0);
+                u[0] = q.x, u[1] = q.y, u[2] = q.z, u[3] = q.w;
+            } else {
+                const uint2 q = *reinterpret_cast<const uint2*>(row + 2 * x0);
+                u[0] = q.x, u[1] = q.y;
             }
         } else {
-            if constexpr (N == 4) {
-                const uint32_t u = *reinterpret_cast<const uint32_t*>(row + x0);
-                v[0] = u & 0xff; v[1] = (u >> 8) & 0xff; v[2] = (u >> 16) & 0xff; v[3] = u >> 24;
-                return;
-            } else if constexpr (N == 2) {
-                const uint16_t u = *reinterpret_cast<const uint16_t*>(row + x0);
-                v[0] = u & 0xff; v[1] = u >> 8;
-                return;
+            uint32_t b[N / 4];
+            if constexpr (N == 8) {
+                const uint2 q = *reinterpret_cast<const uint2*>(row + x0);
+                b[0] = q.x, b[1] = q.y;
+            } else {
+                b[0] = *reinterpret_cast<const uint32_t*>(row + x0);
+            }
+#pragma unroll
+            for (int e = 0; e < N / 4; e++) {
+                u[2 * e] = __byte_perm(b[e], 0u, 0x4140);
+                u[2 * e + 1] = __byte_perm(b[e], 0u, 0x4342);
             }
         }
+        return;
     }
 #pragma unroll
-    for (int e = 0; e < N; e++) v[e] = x0 + e < w ? ld_px(P, hbd, y, x0 + e) : 0;
+    for (int e = 0; e < N; e += 2)
+        u[e / 2] = (x0 + e < w ? (uint32_t)ld_px(P, hbd, y, x0 + e) : 0u) |
+                   (x0 + e + 1 < w ? (uint32_t)ld_px(P, hbd, y, x0 + e + 1) << 16 : 0u);
+}
+template <int N>
+__device__ __forceinline__ void unpack(const uint32_t (&u)[N / 2], int (&v)[N]) {
+#pragma unroll
+    for (int e = 0; e < N; e += 2) {
+        v[e] = (int)(u[e / 2] & 0xffff);
+        v[e + 1] = (int)(u[e / 2] >> 16);
+    }
 }
 template <int N>
 __device__ __forceinline__ void st_n(const PlaneDev& P, int hbd, int y, int x0, int w, const int (&v)[N]) {
     uint8_t* row = P.p + (size_t)y * P.stride;
     if (x0 + N <= w) {
+        uint32_t u[N / 2];
+#pragma unroll
+        for (int e = 0; e < N / 2; e++) u[e] = (uint32_t)v[2 * e] | (uint32_t)v[2 * e + 1] << 16;
         if (hbd) {
-            if constexpr (N == 4) {
-                *reinterpret_cast<uint2*>(reinterpret_cast<uint16_t*>(row) + x0) =
-                    make_uint2((uint32_t)v[0] | ((uint32_t)v[1] << 16), (uint32_t)v[2] | ((uint32_t)v[3] << 16));
-                return;
-            } else if constexpr (N == 2) {
-                *reinterpret_cast<uint32_t*>(reinterpret_cast<uint16_t*>(row) + x0) =
-                    (uint32_t)v[0] | ((uint32_t)v[1] << 16);
-                return;
-            }
+            if constexpr (N == 8) *reinterpret_cast<uint4*>(row + 2 * x0) = make_uint4(u[0], u[1], u[2], u[3]);
+            else *reinterpret_cast<uint2*>(row + 2 * x0) = make_uint2(u[0], u[1]);
         } else {
-            if constexpr (N == 4) {
-                *reinterpret_cast<uint32_t*>(row + x0) =
-                    (uint32_t)v[0] | ((uint32_t)v[1] << 8) | ((uint32_t)v[2] << 16) | ((uint32_t)v[3] << 24);
-                return;
-            } else if constexpr (N == 2) {
-                *reinterpret_cast<uint16_t*>(row + x0) = (uint16_t)(v[0] | (v[1] << 8));
-                return;
-            }
+            const uint32_t a = __byte_perm(u[0], u[1], 0x6420);
+            if constexpr (N == 8) *reinterpret_cast<uint2*>(row + x0) = make_uint2(a, __byte_perm(u[2], u[3], 0x6420));
+            else *reinterpret_cast<uint32_t*>(row + x0) = a;
         }
+        return;
     }
 #pragma unroll
     for (int e = 0; e < N; e++)
         if (x0 + e < w) st_px(P, hbd, y, x0 + e, v[e]);
 }
 
-constexpr int BR = 8;      // chroma-resolution rows per tile
-constexpr int QPT = 256;   // groups of 4 luma columns per tile (one per thread)
-
-// One chroma-resolution row yc of a group: CQ = 4 >> ssx chroma samples of
-// each chroma plane (blended from the un-noised luma first), then the
-// 4 x (1 << ssy) luma samples they cover, as the reference orders it
-// (film_grain.rs:758-828).
+// One chroma-resolution row yc of a thread's columns: CQ chroma samples of each
+// chroma plane (blended from the un-noised luma first), then the luma samples
+// they cover, as the reference orders it (film_grain.rs:758-828).
 template <int CQ>
-__device__ __forceinline__ void blend_group(const FrameDev& F, const av1g_film_grain& fg, const uint8_t (*lut)[256],
-                                            int q, int yc, int gmin, int gmax, int minv, int maxl, int maxc) {
-    const int bd = F.h.bit_depth, hbd = F.hbd;
-    const int np = F.h.num_planes;
-    const int ssx = np > 1 ? F.h.subsampling_x : 0, ssy = np > 1 ? F.h.subsampling_y : 0;
-    const int w = F.out[0].w, h = F.out[0].h;
-    const int gw = (w + ssx) >> ssx;
-    const int x0 = q * 4, xc0 = q * CQ, ly = yc << ssy;
-    if (np >= 3 && xc0 < gw) {
-        const bool chroma = fg.num_cb_points > 0 || fg.num_cr_points > 0 || fg.chroma_scaling_from_luma;
-        int avg[CQ];
-        if (chroma) {
-            int l[4];
-            ld_n<4>(F.lr[0], hbd, ly, x0, w, l);
-            if (ssx) {
-                // average of the two luma columns, the right one clamped to the plane
+__device__ __forceinline__ void blend_row(const BlendShared& S, uint32_t offs, bool left, bool above, int x0, int yc,
+                                          int ly0) {
+    constexpr int SX = CQ < kLumaCols;
+    const BlendPlan& P = S.P;
+    const int hbd = P.hbd, bd = P.bd, ssy = P.ssy, scaling = P.scaling, rnd = P.rnd, minv = P.minv;
+    const int w = P.out[0].w, h = P.out[0].h, top = (1 << bd) - 1;
+    const int ly = yc << ssy;
+    // all the row's samples are asked for before the first is needed
+    uint32_t lu[2][kLumaCols / 2], cu[2][CQ / 2];
+    ld_n<kLumaCols>(P.in[0], hbd, ly, x0, w, lu[0]);
+    const bool two = ssy && ly + 1 < h;
+    if (two) ld_n<kLumaCols>(P.in[0], hbd, ly + 1, x0, w, lu[1]);
+    if (P.np >= 3) {
+        const int xc0 = x0 >> SX, gw = (w + SX) >> SX;
+        ld_n<CQ>(P.in[1], hbd, yc, xc0, gw, cu[0]);
+        ld_n<CQ>(P.in[2], hbd, yc, xc0, gw, cu[1]);
+#pragma unroll
+        for (int p = 1; p <= 2; p++) {
+            int v[CQ];
+            unpack<CQ>(cu[p - 1], v);
+            if (P.noise[p]) {
+                int l[kLumaCols], nz[CQ];
+                unpack<kLumaCols>(lu[0], l);
+                noise_row<CQ, SX>(P, S.tmpl[p], offs, left, above, ssy, yc - (ly0 >> ssy), xc0 & (SX ? 15 : 31), nz);
+                const int a = P.luma[p], b = P.self[p], add = P.add[p], maxc = P.maxv[p];
+                const uint8_t* lut = S.lut + (p << bd);
 #pragma unroll
                 for (int c = 0; c < CQ; c++) {
-                    const int bx = 2 * c + 1;
-                    avg[c] = r2(l[2 * c] + (x0 + bx < w ? l[bx] : l[min(w - 1 - x0, 3)]), 1);
+                    // average of the two luma columns, the right one clamped to the plane
+                    const int avg = SX ? (l[2 * c] + (x0 + 2 * c + 1 < w ? l[2 * c + 1] : l[2 * c]) + 1) >> 1 : l[c];
+                    // with scaling from luma the index is the average alone
+                    const int at = clip3(0, top, ((avg * a + v[c] * b) >> 6) + add);
+                    v[c] = clip3(minv, maxc, v[c] + ((lut[at] * nz[c] + rnd) >> scaling));
                 }
-            } else {
-#pragma unroll
-                for (int c = 0; c < CQ; c++) avg[c] = l[c];
             }
-        }
-        for (int p = 1; p <= 2; p++) {
-            int orig[CQ];
-            ld_n<CQ>(F.lr[p], hbd, yc, xc0, gw, orig);
-            const int npts = p == 1 ? fg.num_cb_points : fg.num_cr_points;
-            if (!(npts > 0 || fg.chroma_scaling_from_luma)) {
-                st_n<CQ>(F.out[p], hbd, yc, xc0, gw, orig);
-                continue;
-            }
-            const Noise<CQ> nc{F.grain_tmpl + p * LH * LW, F.grain_offs, F.grain_nblocks, F.h.subsampling_x ? 44 : 82,
-                               F.h.subsampling_x, F.h.subsampling_y, fg.overlap_flag, gmin, gmax};
-            int nz[CQ];
-            nc.noise(yc, xc0, nz);
-            const int lm = p == 1 ? fg.cb_luma_mult : fg.cr_luma_mult;
-            const int m = p == 1 ? fg.cb_mult : fg.cr_mult;
-            const int off = p == 1 ? fg.cb_offset : fg.cr_offset;
-            int o[CQ];
-#pragma unroll
-            for (int c = 0; c < CQ; c++) {
-                int merged;
-                if (fg.chroma_scaling_from_luma) {
-                    merged = avg[c];
-                } else {
-                    const int comb = avg[c] * (lm - 128) + orig[c] * (m - 128);
-                    merged = clip3(0, (1 << bd) - 1, (comb >> 6) + (off - 256) * (1 << (bd - 8)));
-                }
-                o[c] = clip3(minv, maxc, orig[c] + r2(scale_lut(lut[p], merged, bd) * nz[c], fg.grain_scaling));
-            }
-            st_n<CQ>(F.out[p], hbd, yc, xc0, gw, o);
+            st_n<CQ>(P.out[p], hbd, yc, xc0, gw, v);
         }
     }
-    if (x0 >= w) return;
-    const Noise<4> nl{F.grain_tmpl, F.grain_offs, F.grain_nblocks, LW, 0, 0, fg.overlap_flag, gmin, gmax};
-    for (int dy = 0; dy <= ssy; dy++) {
-        const int y = ly + dy;
-        if (y >= h) break;
-        int orig[4];
-        ld_n<4>(F.lr[0], hbd, y, x0, w, orig);
-        if (fg.num_y_points > 0) {
-            int nz[4];
-            nl.noise(y, x0, nz);
 #pragma unroll
-            for (int e = 0; e < 4; e++)
-                orig[e] = clip3(minv, maxl, orig[e] + r2(scale_lut(lut[0], orig[e], bd) * nz[e], fg.grain_scaling));
+    for (int dy = 0; dy < (SX ? 2 : 1); dy++) {
+        if (dy && !two) break;
+        int v[kLumaCols];
+        unpack<kLumaCols>(lu[dy], v);
+        if (P.noise[0]) {
+            int nz[kLumaCols];
+            noise_row<kLumaCols, 0>(P, S.tmpl[0], offs, left, above, 0, ly + dy - ly0, x0 & 31, nz);
+            const int maxl = P.maxv[0];
+#pragma unroll
+            for (int e = 0; e < kLumaCols; e++)
+                v[e] = clip3(minv, maxl, v[e] + ((S.lut[min(v[e], top)] * nz[e] + rnd) >> scaling));
         }
-        st_n<4>(F.out[0], hbd, y, x0, w, orig);
+        st_n<kLumaCols>(P.out[0], hbd, ly + dy, x0, w, v);
     }
 }
 
-__global__ void __launch_bounds__(256) grain_blend_kernel(const FrameDev* __restrict__ frames,
-                                                          const int32_t* __restrict__ starts, int n, int total) {
-    __shared__ uint8_t lut[3][256];
-    for (int t = blockIdx.x; t < total; t += gridDim.x) {
-        const int f = find_frame(starts, n, t);
-        const FrameDev& F = frames[f];
-        const av1g_film_grain& fg = F.h.film_grain;
-        const int bd = F.h.bit_depth;
-        const int np = F.h.num_planes;
-        const int ssx = np > 1 ? F.h.subsampling_x : 0, ssy = np > 1 ? F.h.subsampling_y : 0;
-        const int w = F.out[0].w, h = F.out[0].h;
-        const int gh = (h + ssy) >> ssy, nq = (w + 3) >> 2;
-        const int ntc = (nq + QPT - 1) / QPT;
-        const int local = t - starts[f];
-        const int tr = local / ntc, tc = local % ntc;
-        __syncthreads();  // the previous tile's LUTs are no longer read
-        for (int i = threadIdx.x; i < 3 * 256; i += blockDim.x) lut[i >> 8][i & 255] = F.grain_lut[i];
-        __syncthreads();
-        const int q = tc * QPT + threadIdx.x;
-        if (q >= nq) continue;
-        const int center = 128 << (bd - 8), gmin = -center, gmax = (256 << (bd - 8)) - 1 - center;
-        int minv, maxl, maxc;
-        if (fg.clip_to_restricted_range) {
-            minv = 16 << (bd - 8);
-            maxl = 235 << (bd - 8);
-            maxc = F.h.matrix_coefficients == 0 ? maxl : 240 << (bd - 8);
-        } else {
-            minv = 0;
-            maxl = maxc = (256 << (bd - 8)) - 1;
+__device__ __noinline__ void plan_blend(const FrameDev& F, BlendPlan& P) {
+    const av1g_frame_header& h = F.h;
+    const av1g_film_grain& fg = h.film_grain;
+    const int bd = h.bit_depth, np = h.num_planes, center = 128 << (bd - 8);
+    for (int p = 0; p < 3; p++) {
+        P.in[p] = F.lr[p];
+        P.out[p] = F.out[p];
+    }
+    P.offs = F.grain_offs;
+    P.nblocks = F.grain_nblocks;
+    P.hbd = F.hbd;
+    P.bd = bd;
+    P.np = np;
+    P.ssx = np > 1 ? h.subsampling_x : 0;
+    P.ssy = np > 1 ? h.subsampling_y : 0;
+    P.tcols = (F.out[0].w + kTileGroups * kLumaCols - 1) / (kTileGroups * kLumaCols);
+    P.gmin = -center;
+    P.gmax = (256 << (bd - 8)) - 1 - center;
+    P.overlap = fg.overlap_flag;
+    P.scaling = fg.grain_scaling;
+    P.rnd = fg.grain_scaling ? 1 << (fg.grain_scaling - 1) : 0;
+    const bool cfl = fg.chroma_scaling_from_luma;
+    P.noise[0] = fg.num_y_points > 0;
+    P.noise[1] = np > 1 && (cfl || fg.num_cb_points > 0);
+    P.noise[2] = np > 1 && (cfl || fg.num_cr_points > 0);
+    const bool clip = fg.clip_to_restricted_range;
+    P.minv = clip ? 16 << (bd - 8) : 0;
+    P.maxv[0] = clip ? 235 << (bd - 8) : (256 << (bd - 8)) - 1;
+    P.maxv[1] = P.maxv[2] = clip && h.matrix_coefficients != 0 ? 240 << (bd - 8) : P.maxv[0];
+    // (avg * luma + sample * self) >> 6, plus add; from luma: the average itself
+    P.luma[1] = cfl ? 64 : fg.cb_luma_mult - 128;
+    P.luma[2] = cfl ? 64 : fg.cr_luma_mult - 128;
+    P.self[1] = cfl ? 0 : fg.cb_mult - 128;
+    P.self[2] = cfl ? 0 : fg.cr_mult - 128;
+    P.add[1] = cfl ? 0 : (fg.cb_offset - 256) * (1 << (bd - 8));
+    P.add[2] = cfl ? 0 : (fg.cr_offset - 256) * (1 << (bd - 8));
+}
+
+__global__ void __launch_bounds__(kBlendThreads, 4) grain_blend_kernel(const FrameDev* __restrict__ frames,
+                                                                   const int32_t* __restrict__ starts, int n, int total) {
+    __shared__ BlendShared S;
+    const BlendPlan& P = S.P;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // each CTA walks a contiguous run of tiles, so it lays out a frame's
+    // templates and tables once
+    const int per = (total + gridDim.x - 1) / gridDim.x;
+    const int t_end = min(total, ((int)blockIdx.x + 1) * per);
+    int end = -1, first = 0;
+    for (int t = blockIdx.x * per; t < t_end; t++) {
+        if (t >= end) {
+            const int f = find_frame(starts, n, t);
+            const FrameDev& F = frames[f];
+            first = starts[f];
+            end = starts[f + 1];
+            __syncthreads();  // the previous frame's are no longer read
+            if (threadIdx.x == 0) plan_blend(F, S.P);
+            const int np = F.h.num_planes, bd = F.h.bit_depth, sub = bd - 8;
+            const int cw = F.h.subsampling_x ? 44 : LW, ch = F.h.subsampling_y ? 38 : LH;
+            for (int p = 0; p < np; p++) {
+                const uint32_t* src = reinterpret_cast<const uint32_t*>(F.grain_tmpl) + p * (LH * LW / 2);
+                const int words = p ? cw * ch / 2 : LH * LW / 2;
+                for (int i = threadIdx.x; i < words; i += kBlendThreads) S.tmpl[p][i] = __ldg(src + i);
+                // between two of the 256 entries the table is linear; above the last, flat
+                for (int x = threadIdx.x; x < 256; x += kBlendThreads) {
+                    const int a = F.grain_lut[p * 256 + x], d = x < 255 ? F.grain_lut[p * 256 + x + 1] - a : 0;
+                    for (int k = 0; k < 1 << sub; k++) S.lut[(p << bd) + (x << sub) + k] = (uint8_t)(a + r2(d * k, sub));
+                }
+            }
+            __syncthreads();
         }
-        for (int yc = tr * BR; yc < min(gh, tr * BR + BR); yc++) {
-            if (ssx) blend_group<2>(F, fg, lut, q, yc, gmin, gmax, minv, maxl, maxc);
-            else blend_group<4>(F, fg, lut, q, yc, gmin, gmax, minv, maxl, maxc);
+        const int stripe = (t - first) / P.tcols, col = (t - first) - stripe * P.tcols;
+        const int x0 = (col * kTileGroups + lane) * kLumaCols, ly0 = stripe * kStripe;
+        if (x0 >= P.out[0].w) continue;
+        const int k = x0 >> 5;
+        const bool left = P.overlap && k > 0, above = P.overlap && stripe > 0;
+        const uint8_t* o = P.offs + stripe * P.nblocks + k;
+        uint32_t offs = o[0];
+        if (left) offs |= (uint32_t)o[-1] << 8;
+        if (above) {
+            offs |= (uint32_t)o[-P.nblocks] << 16;
+            if (left) offs |= (uint32_t)o[-P.nblocks - 1] << 24;
+        }
+        const int gh = (P.out[0].h + P.ssy) >> P.ssy, yc1 = min(gh, (ly0 + kStripe) >> P.ssy);
+        for (int yc = (ly0 >> P.ssy) + warp; yc < yc1; yc += kWarps) {
+            if (P.ssx) blend_row<kLumaCols / 2>(S, offs, left, above, x0, yc, ly0);
+            else blend_row<kLumaCols>(S, offs, left, above, x0, yc, ly0);
         }
     }
 }
@@ -569,15 +631,15 @@ __global__ void __launch_bounds__(256) grain_blend_kernel(const FrameDev* __rest
 }  // namespace
 
 int tiles_grain_blend(const FrameDev& f) {
-    int ssy = f.h.num_planes > 1 ? f.h.subsampling_y : 0;
-    int gh = (f.out[0].h + ssy) >> ssy, nq = (f.out[0].w + 3) >> 2;
-    return ((gh + BR - 1) / BR) * ((nq + QPT - 1) / QPT);
+    const int cols = kTileGroups * kLumaCols;
+    return ((f.out[0].h + kStripe - 1) / kStripe) * ((f.out[0].w + cols - 1) / cols);
 }
 
 void launch_grain(const FrameDev* frames, const int32_t* starts_tmpl, const int32_t* starts_blend, int n,
                   int total_tmpl, int total_blend, const StageShape& sh, cudaStream_t s) {
     if (total_tmpl > 0) grain_template_kernel<<<total_tmpl, kTmplThreads, 0, s>>>(frames, starts_tmpl, n, total_tmpl);
-    if (total_blend > 0) grain_blend_kernel<<<shape_grid(sh, total_blend), 256, 0, s>>>(frames, starts_blend, n, total_blend);
+    if (total_blend <= 0) return;
+    grain_blend_kernel<<<shape_grid(sh, total_blend), kBlendThreads, 0, s>>>(frames, starts_blend, n, total_blend);
 }
 
 }  // namespace av1g
