@@ -10,13 +10,23 @@
 // of a pass is independent and the sequential order is immaterial.
 //
 // B200 mapping: one CTA owns a 64x64 output tile of one plane and stages a
-// 96x96 window (16-sample halo: an output sample can be moved by an edge up to
-// 6 samples away whose taps reach 7 further) in shared memory.  It computes
-// the per-4x4 edge parameters (filter length, limit, blimit, thresh) for the
-// window from the mi grid, runs the vertical pass over all window rows, then
+// 96x88 window (16- and 12-sample halos: an output sample can be moved by an edge up
+// to 6 samples away whose taps reach 7 further) in shared memory with the edge
+// codes of its cells.  It runs the vertical pass over all window rows, then
 // the horizontal pass over the tile's columns, and writes the tile.  The
 // frame is filtered out of place (recon -> deblocked) so halo reads never
 // observe another tile's output.
+//
+// A thread filters two lines at a time, the halves of a word, in
+// half-precision differences and 16-bit sums that are exact for 8 and 10 bits
+// (12-bit lines go one by one); both passes read two lines' samples as pairs of
+// words without bank conflicts.  Bound by issue, and by warps whose edges take
+// different filters: 713 us for 64 1080p 8-bit frames and 119 us for four 3840x2160
+// 10-bit ones with a line per thread, every thread deriving its tile and a pass that
+// unpacked each cell's strengths; 608 and 101 us with pairs and a planning thread;
+// 540 and 95 us with the filters that few edges take in calls of their own, and 497 and
+// 88 us (1.4 TB/s of planes read and written) at six CTAs per SM.
+#include <cuda_fp16.h>
 #include "common.cuh"
 #include "av1_spec_tables.h"
 
@@ -31,13 +41,16 @@ __constant__ AV1T_TX_HEIGHT_TYPE c_txh AV1T_TX_HEIGHT_DIMS = AV1T_TX_HEIGHT_INIT
 
 namespace {
 
-// window rows hold u16 samples at an odd number of 32-bit words per row
-// (49), so a warp walking down a column touches 32 distinct banks; a row
-// starts on a 4-byte (not always 8-byte) boundary, so the window is moved in
-// 32-bit words
-constexpr int TILE = 64, HALO = 16, WIN = TILE + 2 * HALO, PITCH = WIN + 2, CELLS = WIN / 4;
+// Window rows hold u16 samples two to a word, a pair of rows kPair words apart and
+// its second row kRow words after the first: two rows of a line pair are one offset
+// apart, and 8-byte accesses of 16 consecutive pairs touch 32 distinct banks.
+constexpr int TILE = 64, HALO = 16, WIN = TILE + 2 * HALO, CELLS = WIN / 4;
+constexpr int kRow = WIN / 2, kPair = 2 * kRow + 2;
+static_assert(kPair % 32 == 2, "pairs of rows two banks apart");
+// The horizontal pass reads at most 7 samples above and 6 below its edges, which
+// lie in rows 12 to 84: no other row of the window is loaded or filtered.
+constexpr int kRow0 = 4, kRow1 = 92;
 constexpr int kDbThreads = 256;  // deblock_kernel's CTA size
-static_assert(WIN * (WIN / 4) % kDbThreads == 0, "window groups split evenly over the CTA");
 constexpr int BLOCK_SIZES = 22, BLOCK_INVALID = 22;
 
 // ---- edge codes ---------------------------------------------------------------
@@ -247,57 +260,206 @@ __global__ void __launch_bounds__(256) lf_prep_kernel(const FrameDev* __restrict
     }
 }
 
-// Unpacks a cell code into filter length | limit << 8 | blimit << 16 |
-// thresh << 24 (adaptive_filter_strength, loop_filter.rs:500-525).
-__device__ __forceinline__ uint32_t decode_code(uint32_t code, int sharp) {
-    if (code == 0) return 0;
-    int lvl = code & 63, fsc = code >> 6;
-    int fsize = fsc == 1 ? 4 : (fsc == 2 ? 8 : 16);
-    int sh = sharp > 4 ? 2 : (sharp > 0 ? 1 : 0);
-    int limit = sharp > 0 ? clip3(1, 9 - sharp, lvl >> sh) : max(lvl >> sh, 1);
-    int blimit = (2 * (lvl + 2) + limit) & 0xff;
-    return (uint32_t)fsize | ((uint32_t)limit << 8) | ((uint32_t)blimit << 16) | ((uint32_t)(lvl >> 4) << 24);
+// limit, blimit and thresh of a level (adaptive_filter_strength,
+// loop_filter.rs:500-525), before the scaling by bit depth.
+struct Strength {
+    int limit, blimit, thresh;
+};
+__device__ __forceinline__ Strength strength(int lvl, int sharp) {
+    const int sh = sharp > 4 ? 2 : (sharp > 0 ? 1 : 0);
+    const int limit = sharp > 0 ? clip3(1, 9 - sharp, lvl >> sh) : max(lvl >> sh, 1);
+    return Strength{limit, (2 * (lvl + 2) + limit) & 0xff, lvl >> 4};
 }
 
 __device__ __forceinline__ int f4clamp(int v, int bd) { return clip3(-(1 << (bd - 1)), (1 << (bd - 1)) - 1, v); }
 
 // wide_filter (loop_filter.rs:789-822) for one (n, log2Size) case: outputs
 // i in [-n, n) from taps j in [-n, n] weighted 2 for |j| <= n2 else 1, source
-// positions clamped to [-(n + 1), n].  All indices are compile-time.
+// positions clamped to [-(n + 1), n].  Two lines at a time, one per half of a word:
+// no sum passes 16 bits (16 times 4095, plus the rounding).
 template <int N, int LOG2, int N2>
-__device__ __forceinline__ void wide(uint16_t* b, int st) {
-    int v[2 * N + 2];
+__device__ __forceinline__ void wide(const uint32_t (&v)[2 * N + 2], uint32_t (&o)[2 * N]) {
+    auto at = [&](int k) { return v[(k < -(N + 1) ? -(N + 1) : (k > N ? N : k)) + N + 1]; };
+    uint32_t box = (1u << (LOG2 - 1)) * 0x10001u;
 #pragma unroll
-    for (int k = 0; k < 2 * N + 2; k++) v[k] = b[(k - N - 1) * st];
-    int o[2 * N];
+    for (int j = -N; j <= N; j++) box += at(j - N);
 #pragma unroll
     for (int i = -N; i < N; i++) {
-        int t = 0;
-#pragma unroll
-        for (int j = -N; j <= N; j++) {
-            int pp = i + j < -(N + 1) ? -(N + 1) : (i + j > N ? N : i + j);
-            t += v[pp + N + 1] * ((j <= N2 && j >= -N2) ? 2 : 1);
-        }
-        o[i + N] = (t + (1 << (LOG2 - 1))) >> LOG2;
+        uint32_t t = box + at(i);
+        if (N2) t += at(i - 1) + at(i + 1);
+        o[i + N] = (t >> LOG2) & 0x0fff0fffu;
+        box += at(i + N + 1) - at(i - N);
     }
-#pragma unroll
-    for (int i = -N; i < N; i++) b[i * st] = (uint16_t)o[i + N];
 }
 
-// sample_filtering + filter_mask + narrow/wide filters (loop_filter.rs:582-822)
-// on a line of shared-memory samples; b points at q0, st is the step.
-__device__ void filter_line(uint16_t* b, int st, uint32_t prm, int plane, int bd) {
-    int fs = prm & 0xff;
-    int limit = (prm >> 8) & 0xff, blimit = (prm >> 16) & 0xff, thresh = prm >> 24;
+// ---- two lines at a time, 8 and 10 bits -------------------------------------
+// A sample v is the half 1024 + v (0x6400 | v): the differences of two are exact,
+// and so is all that decides or makes a result below; what is larger than
+// that is rounded only where it is beyond a bound or a clamp already.
+constexpr uint32_t kBias = 0x64006400u, kSample = 0x03ff03ffu;
+
+__device__ __forceinline__ __half2 h2(uint32_t u) { return *reinterpret_cast<const __half2*>(&u); }
+__device__ __forceinline__ uint32_t u32(__half2 h) { return *reinterpret_cast<const uint32_t*>(&h); }
+__device__ __forceinline__ __half2 dup(float x) { return __float2half2_rn(x); }
+// max(m, |a - b|)
+__device__ __forceinline__ __half2 far(__half2 m, uint32_t a, uint32_t b) {
+    return __hmax2(m, __habs2(__hsub2(h2(a), h2(b))));
+}
+__device__ __forceinline__ uint32_t pick(uint32_t mask, uint32_t a, uint32_t b) { return (a & mask) | (b & ~mask); }
+
+struct HalfConsts {
+    __half2 one, lo, hi, top;  // 1 << (bd - 8), the clamp's ends, 1024 + the largest sample
+};
+
+// Samples 2j and 2j + 1 of both lines of a pair, counted from q0: the vertical
+// pass's lines are the two rows of a pair, the horizontal pass's two adjacent columns.
+template <bool VERT>
+__device__ __forceinline__ void ld_pair(const uint32_t* m, int j, uint32_t& a, uint32_t& b) {
+    if (VERT) {
+        const uint32_t u = m[j], v = m[j + kRow];
+        a = __byte_perm(u, v, 0x5410);
+        b = __byte_perm(u, v, 0x7632);
+    } else {
+        a = m[j * kPair];
+        b = m[j * kPair + kRow];
+    }
+}
+template <bool VERT>
+__device__ __forceinline__ void st_pair(uint32_t* m, int j, uint32_t a, uint32_t b) {
+    if (VERT) {
+        m[j] = __byte_perm(a, b, 0x5410);
+        m[j + kRow] = __byte_perm(a, b, 0x7632);
+    } else {
+        m[j * kPair] = a;
+        m[j * kPair + kRow] = b;
+    }
+}
+
+// The 13-tap filter on the lines of `on`, which are unchanged so far: a call of its
+// own that reads its samples again, so that the path most edges take fits the
+// 40 registers that six CTAs per SM leave.
+template <bool VERT>
+__device__ __noinline__ void filter_wide(uint32_t* m, uint32_t on) {
+    uint32_t v[16];
+#pragma unroll
+    for (int j = 0; j < 8; j++) ld_pair<VERT>(m, j - 4, v[2 * j], v[2 * j + 1]);
+    uint32_t x[14], o[12];
+#pragma unroll
+    for (int k = 0; k < 14; k++) x[k] = v[k + 1] & kSample;
+    wide<6, 4, 1>(x, o);
+#pragma unroll
+    for (int j = 0; j < 6; j++)
+        st_pair<VERT>(m, j - 3, pick(on, o[2 * j] | kBias, v[2 * j + 2]), pick(on, o[2 * j + 1] | kBias, v[2 * j + 3]));
+}
+
+// The same for the 7-tap (luma) and 5-tap (chroma) ones.
+template <bool VERT>
+__device__ __noinline__ void filter_flat(uint32_t* m, uint32_t on, int plane) {
+    uint32_t v[8];
+#pragma unroll
+    for (int j = 0; j < 4; j++) ld_pair<VERT>(m, j - 2, v[2 * j], v[2 * j + 1]);
+    uint32_t x[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) x[k] = v[k] & kSample;
+    if (plane) {
+        const uint32_t y[6] = {x[1], x[2], x[3], x[4], x[5], x[6]};
+        uint32_t o[4];
+        wide<2, 3, 1>(y, o);
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[k + 2] = pick(on, o[k] | kBias, v[k + 2]);
+    } else {
+        uint32_t o[6];
+        wide<3, 3, 0>(x, o);
+#pragma unroll
+        for (int k = 0; k < 6; k++) v[k + 1] = pick(on, o[k] | kBias, v[k + 1]);
+        st_pair<VERT>(m, -2, v[0], v[1]);
+        st_pair<VERT>(m, 1, v[6], v[7]);
+    }
+    st_pair<VERT>(m, -1, v[2], v[3]);
+    st_pair<VERT>(m, 0, v[4], v[5]);
+}
+
+// sample_filtering + filter_mask + narrow/wide filters (loop_filter.rs:582-822).
+// The edges of one pass share no samples, but two 4-sample edges share the
+// 8 bytes between them: only words with changed samples are written.
+template <bool VERT>
+__device__ __forceinline__ void filter_pair(uint32_t* m, int cls, uint2 st, int plane, const HalfConsts& K) {
+    uint32_t p3 = 0, p2 = 0, p1, p0, q0, q1, q2 = 0, q3 = 0;
+    ld_pair<VERT>(m, -1, p1, p0);
+    ld_pair<VERT>(m, 0, q0, q1);
+    const __half2 dp = __hsub2(h2(p1), h2(q1)), dq = __hsub2(h2(q0), h2(p0));
+    const __half2 d1 = far(__habs2(__hsub2(h2(p1), h2(p0))), q1, q0);
+    __half2 dl = d1;
+    if (cls >= 2) {
+        ld_pair<VERT>(m, -2, p3, p2);
+        ld_pair<VERT>(m, 1, q2, q3);
+        dl = far(far(dl, p2, p1), q2, q1);
+        if (!plane) dl = far(far(dl, p3, p2), q3, q2);
+    }
+    // 2 |p0 - q0| + |p1 - q1| / 2 <= blimit with the half kept: st holds blimit + 1/2
+    const __half2 step = __hfma2(__habs2(dq), dup(2.f), __hmul2(__habs2(dp), dup(0.5f)));
+    const uint32_t on = __hle2_mask(dl, h2(__byte_perm(st.x, 0u, 0x1010))) &
+                        __hle2_mask(step, h2(__byte_perm(st.x, 0u, 0x3232)));
+    if (!on) return;
+    uint32_t flat = 0, flat2 = 0;
+    if (cls >= 2) {
+        __half2 df = far(far(d1, p2, p0), q2, q0);
+        if (!plane) df = far(far(df, p3, p0), q3, q0);
+        flat = on & __hle2_mask(df, K.one);
+    }
+    if (const uint32_t narrow = on & ~flat) {
+        const uint32_t hev = __hgt2_mask(d1, h2(__byte_perm(st.y, 0u, 0x1010)));
+        __half2 f = h2(u32(__hmin2(__hmax2(dp, K.lo), K.hi)) & hev);
+        f = __hmin2(__hmax2(__hfma2(dq, dup(3.f), f), K.lo), K.hi);
+        // min(f + 4, hi) >> 3 and min(f + 3, hi) >> 3: less 3.5, an eighth, to the nearest whole number
+        const __half2 cap = __hsub2(K.hi, dup(3.5f)), big = dup(1536.f);
+        const __half2 f1 = __hsub2(__hfma2(__hmin2(__hadd2(f, dup(0.5f)), cap), dup(0.125f), big), big);
+        const __half2 f2 = __hsub2(__hfma2(__hmin2(__hsub2(f, dup(0.5f)), cap), dup(0.125f), big), big);
+        const __half2 zero = dup(1024.f);
+        const uint32_t r0 = pick(narrow, u32(__hmin2(__hmax2(__hsub2(h2(q0), f1), zero), K.top)), q0);
+        const uint32_t n0 = pick(narrow, u32(__hmin2(__hmax2(__hadd2(h2(p0), f2), zero), K.top)), p0);
+        // (f1 + 1) >> 1
+        const __half2 ff = __hsub2(__hadd2(__hfma2(f1, dup(0.5f), dup(0.25f)), big), big);
+        const uint32_t outer = narrow & ~hev;
+        const uint32_t r1 = pick(outer, u32(__hmin2(__hmax2(__hsub2(h2(q1), ff), zero), K.top)), q1);
+        const uint32_t n1 = pick(outer, u32(__hmin2(__hmax2(__hadd2(h2(p1), ff), zero), K.top)), p1);
+        st_pair<VERT>(m, -1, n1, n0);
+        st_pair<VERT>(m, 0, r0, r1);
+    }
+    if (!flat) return;
+    if (cls == 3) {
+        uint32_t p4, p5, p6, p7, q4, q5, q6, q7;
+        ld_pair<VERT>(m, -3, p5, p4);
+        ld_pair<VERT>(m, 2, q4, q5);
+        ld_pair<VERT>(m, -4, p7, p6);
+        ld_pair<VERT>(m, 3, q6, q7);
+        __half2 d2 = far(far(__habs2(__hsub2(h2(p6), h2(p0))), q6, q0), p5, p0);
+        d2 = far(far(far(d2, q5, q0), p4, p0), q4, q0);
+        const uint32_t flat2 = flat & __hle2_mask(d2, K.one);
+        if (flat2) filter_wide<VERT>(m, flat2);
+        flat &= ~flat2;
+    }
+    if (flat) filter_flat<VERT>(m, flat, plane);
+}
+
+// ---- one line at a time, 12 bits (a difference of two 12-bit samples is no half) ----
+// Line `e` (0 or 1) of a pair; position k counts from q0.
+template <bool VERT>
+__device__ void filter_line(uint16_t* b, int e, int cls, uint32_t st, int plane) {
+    constexpr int bd = 12;
+    auto at = [&](int k) -> uint16_t& {
+        return VERT ? b[2 * kRow * e + k] : b[2 * (kPair * (k >> 1) + kRow * (k & 1)) + e];
+    };
+    const int limit = st & 0xff, blimit = (st >> 8) & 0xff, thresh = st >> 16;
     int bds = bd - 8;
-    int q0 = b[0], q1 = b[st], q2 = b[2 * st], q3 = b[3 * st];
-    int p0 = b[-st], p1 = b[-2 * st], p2 = b[-3 * st], p3 = b[-4 * st];
+    int q0 = at(0), q1 = at(1), q2 = at(2), q3 = at(3);
+    int p0 = at(-1), p1 = at(-2), p2 = at(-3), p3 = at(-4);
     // every test below is "some |difference| > bound": the largest
     // difference against the bound, the shared ones computed once
     const int d1 = max(abs(p1 - p0), abs(q1 - q0));
     int thr = thresh << bds;
     bool hev = d1 > thr;
-    int flen = fs == 4 ? 4 : (plane ? 6 : (fs == 8 ? 8 : 16));
+    int flen = cls == 1 ? 4 : (plane ? 6 : (cls == 2 ? 8 : 16));
     int lim = limit << bds, blim = blimit << bds;
     int dl = d1;
     if (flen >= 6) dl = __vimax3_s32(dl, abs(p2 - p1), abs(q2 - q1));
@@ -305,178 +467,239 @@ __device__ void filter_line(uint16_t* b, int st, uint32_t prm, int plane, int bd
     if (dl > lim || abs(p0 - q0) * 2 + abs(p1 - q1) / 2 > blim) return;
     int one = 1 << bds;
     bool flat = false, flat2 = false;
-    if (fs >= 8) {
+    if (cls >= 2) {
         int df = __vimax3_s32(d1, abs(p2 - p0), abs(q2 - q0));
         if (flen >= 8) df = __vimax3_s32(df, abs(p3 - p0), abs(q3 - q0));
         flat = df <= one;
     }
-    if (fs >= 16 && flat) {
-        int q4 = b[4 * st], q5 = b[5 * st], q6 = b[6 * st];
-        int p4 = b[-5 * st], p5 = b[-6 * st], p6 = b[-7 * st];
+    int p4 = 0, p5 = 0, p6 = 0, q4 = 0, q5 = 0, q6 = 0;
+    if (cls >= 3 && flat) {
+        q4 = at(4), q5 = at(5), q6 = at(6);
+        p4 = at(-5), p5 = at(-6), p6 = at(-7);
         const int d2 = __vimax3_s32(__vimax3_s32(abs(p6 - p0), abs(q6 - q0), abs(p5 - p0)),
                                     __vimax3_s32(abs(q5 - q0), abs(p4 - p0), abs(q4 - q0)), 0);
         flat2 = d2 <= one;
     }
-    if (fs == 4 || !flat) {
+    if (!flat) {
         int half = 0x80 << bds;
         int ps1 = p1 - half, ps0 = p0 - half, qs0 = q0 - half, qs1 = q1 - half;
         int f = hev ? f4clamp(ps1 - qs1, bd) : 0;
         f = f4clamp(f + 3 * (qs0 - ps0), bd);
         int f1 = f4clamp(f + 4, bd) >> 3;
         int f2 = f4clamp(f + 3, bd) >> 3;
-        b[0] = (uint16_t)(f4clamp(qs0 - f1, bd) + half);
-        b[-st] = (uint16_t)(f4clamp(ps0 + f2, bd) + half);
+        at(0) = (uint16_t)(f4clamp(qs0 - f1, bd) + half);
+        at(-1) = (uint16_t)(f4clamp(ps0 + f2, bd) + half);
         if (!hev) {
             int ff = (f1 + 1) >> 1;
-            b[st] = (uint16_t)(f4clamp(qs1 - ff, bd) + half);
-            b[-2 * st] = (uint16_t)(f4clamp(ps1 + ff, bd) + half);
+            at(1) = (uint16_t)(f4clamp(qs1 - ff, bd) + half);
+            at(-2) = (uint16_t)(f4clamp(ps1 + ff, bd) + half);
         }
         return;
     }
-    if (fs == 8 || !flat2) {
-        if (plane == 0) wide<3, 3, 0>(b, st);
-        else wide<2, 3, 1>(b, st);
+    if (!flat2) {
+        if (plane == 0) {
+            const uint32_t v[8] = {(uint32_t)p3, (uint32_t)p2, (uint32_t)p1, (uint32_t)p0,
+                                   (uint32_t)q0, (uint32_t)q1, (uint32_t)q2, (uint32_t)q3};
+            uint32_t o[6];
+            wide<3, 3, 0>(v, o);
+#pragma unroll
+            for (int i = -3; i < 3; i++) at(i) = (uint16_t)o[i + 3];
+        } else {
+            const uint32_t v[6] = {(uint32_t)p2, (uint32_t)p1, (uint32_t)p0, (uint32_t)q0, (uint32_t)q1, (uint32_t)q2};
+            uint32_t o[4];
+            wide<2, 3, 1>(v, o);
+#pragma unroll
+            for (int i = -2; i < 2; i++) at(i) = (uint16_t)o[i + 2];
+        }
     } else {
-        wide<6, 4, 1>(b, st);
+        const uint32_t v[14] = {(uint32_t)p6, (uint32_t)p5, (uint32_t)p4, (uint32_t)p3, (uint32_t)p2,
+                                (uint32_t)p1, (uint32_t)p0, (uint32_t)q0, (uint32_t)q1, (uint32_t)q2,
+                                (uint32_t)q3, (uint32_t)q4, (uint32_t)q5, (uint32_t)q6};
+        uint32_t o[12];
+        wide<6, 4, 1>(v, o);
+#pragma unroll
+        for (int i = -6; i < 6; i++) at(i) = (uint16_t)o[i + 6];
     }
 }
 
-__global__ void __launch_bounds__(kDbThreads, 6) deblock_kernel(const FrameDev* __restrict__ frames,
+template <bool VERT>
+__device__ __noinline__ void filter_lines12(uint32_t* m, int cls, uint32_t st, int plane) {
+    uint16_t* b = reinterpret_cast<uint16_t*>(m);
+    filter_line<VERT>(b, 0, cls, st, plane);
+    filter_line<VERT>(b, 1, cls, st, plane);
+}
+
+// What the CTA needs of a tile, worked out by one thread while the previous tile
+// is filtered.
+struct DbTile {
+    const uint8_t* src;
+    uint8_t* dst;
+    const uint16_t* codes;
+    int src_stride, dst_stride, w, h, dw, dh, x, y;  // (x, y): the tile's first sample
+    int plane, hbd, bd, sharp;
+};
+
+__device__ __noinline__ void plan_tile(const FrameDev* __restrict__ frames, const int32_t* __restrict__ starts, int n,
+                                       int t, DbTile& T) {
+    const int f = find_frame(starts, n, t);
+    const FrameDev& F = frames[f];
+    int local = t - starts[f], plane = 0, tx = 0, ty = 0;
+    // planes with no deblock work have no tiles
+    for (int p = 0; p < F.h.num_planes; p++) {
+        if (p > 0 && F.h.lf_level[1 + p] == 0) continue;
+        const int ntx = (F.recon[p].w + TILE - 1) / TILE, nty = (F.recon[p].h + TILE - 1) / TILE;
+        if (local < ntx * nty) { plane = p; ty = local / ntx; tx = local - ty * ntx; break; }
+        local -= ntx * nty;
+    }
+    const PlaneDev& S = F.recon[plane];
+    const PlaneDev& D = F.deb[plane];
+    T = DbTile{S.p, D.p, F.lf_codes[plane], S.stride, D.stride, S.w, S.h, min(D.w, S.w), min(D.h, S.h),
+               tx * TILE, ty * TILE, plane, F.hbd, F.h.bit_depth, F.h.lf_sharpness};
+}
+
+constexpr int kDbCtas = 6;
+
+__global__ void __launch_bounds__(kDbThreads, kDbCtas) deblock_kernel(const FrameDev* __restrict__ frames,
                                                       const int32_t* __restrict__ starts, int n, int total) {
-    __shared__ __align__(16) uint16_t win[WIN * PITCH];
-    __shared__ uint32_t ev[CELLS * CELLS], eh[CELLS * CELLS];
-    for (int t = blockIdx.x; t < total; t += gridDim.x) {
-        int f = find_frame(starts, n, t);
-        const FrameDev& F = frames[f];
-        int local = t - starts[f];
-        // tile -> (plane, ty, tx); planes with no deblock work have no tiles
-        int plane = 0, tx = 0, ty = 0;
-        for (int p = 0; p < F.h.num_planes; p++) {
-            if (p > 0 && F.h.lf_level[1 + p] == 0) continue;
-            int ntx = (F.recon[p].w + TILE - 1) / TILE, nty = (F.recon[p].h + TILE - 1) / TILE;
-            if (local < ntx * nty) { plane = p; ty = local / ntx; tx = local % ntx; break; }
-            local -= ntx * nty;
-        }
-        const PlaneDev& S = F.recon[plane];
-        const PlaneDev& D = F.deb[plane];
-        const int hbd = F.hbd, bd = F.h.bit_depth;
-        const int gx0 = tx * TILE - HALO, gy0 = ty * TILE - HALO;
-        __syncthreads();  // previous tile done with shared memory
-        // window: 4 consecutive samples per thread, one vector load when the
-        // group lies inside the plane (rows are 4-sample aligned: gx0 % 4 == 0).
-        // A window inside the plane horizontally (almost every tile) issues
-        // all of a thread's loads before it unpacks any, so their latencies
-        // overlap instead of adding up.
-        if (gx0 >= 0 && gx0 + WIN <= S.w) {
-            constexpr int G = WIN / 4, PER = WIN * G / kDbThreads;
-            const uint8_t* base = S.p + (size_t)(hbd ? 2 : 1) * gx0;
-            if (hbd) {
-                uint2 v[PER];
-#pragma unroll
-                for (int q = 0; q < PER; q++) {
-                    const int i = threadIdx.x + q * kDbThreads, r = i / G, c = (i - r * G) * 4;
-                    v[q] = *reinterpret_cast<const uint2*>(base + (size_t)clip3(0, S.h - 1, gy0 + r) * S.stride + 2 * c);
-                }
-#pragma unroll
-                for (int q = 0; q < PER; q++) {
-                    const int i = threadIdx.x + q * kDbThreads, r = i / G, c = (i - r * G) * 4;
-                    uint32_t* w = reinterpret_cast<uint32_t*>(&win[r * PITCH + c]);  // 4-byte aligned
-                    w[0] = v[q].x;
-                    w[1] = v[q].y;
-                }
-            } else {
-                uint32_t v[PER];
-#pragma unroll
-                for (int q = 0; q < PER; q++) {
-                    const int i = threadIdx.x + q * kDbThreads, r = i / G, c = (i - r * G) * 4;
-                    v[q] = *reinterpret_cast<const uint32_t*>(base + (size_t)clip3(0, S.h - 1, gy0 + r) * S.stride + c);
-                }
-#pragma unroll
-                for (int q = 0; q < PER; q++) {
-                    const int i = threadIdx.x + q * kDbThreads, r = i / G, c = (i - r * G) * 4;
-                    uint32_t* w = reinterpret_cast<uint32_t*>(&win[r * PITCH + c]);  // 4-byte aligned
-                    w[0] = __byte_perm(v[q], 0u, 0x4140);
-                    w[1] = __byte_perm(v[q], 0u, 0x4342);
-                }
-            }
-        } else
-        for (int i = threadIdx.x; i < WIN * (WIN / 4); i += blockDim.x) {
-            int r = i / (WIN / 4), c = (i % (WIN / 4)) * 4;
-            int gy = clip3(0, S.h - 1, gy0 + r), gx = gx0 + c;
-            uint16_t* w = &win[r * PITCH + c];
-            const uint8_t* row = S.p + (size_t)gy * S.stride;
-            if (gx >= 0 && gx + 3 < S.w) {
-                uint32_t* w32 = reinterpret_cast<uint32_t*>(w);  // 4-byte aligned
-                if (hbd) {
-                    const uint2 v = *reinterpret_cast<const uint2*>(row + 2 * gx);
-                    w32[0] = v.x;
-                    w32[1] = v.y;
-                } else {
-                    const uint32_t v = *reinterpret_cast<const uint32_t*>(row + gx);
-                    w32[0] = __byte_perm(v, 0u, 0x4140);
-                    w32[1] = __byte_perm(v, 0u, 0x4342);
-                }
-            } else {
-#pragma unroll
-                for (int k = 0; k < 4; k++) w[k] = (uint16_t)ld_px(S, hbd, gy, clip3(0, S.w - 1, gx + k));
-            }
-        }
-        const int cy0 = gy0 / 4, cx0 = gx0 / 4;  // gx0,gy0 are multiples of 4 (may be negative)
-        const int cw = S.w >> 2, ch = S.h >> 2, sharp = F.h.lf_sharpness;
-        const uint16_t* codes = F.lf_codes[plane];
+    __shared__ __align__(16) uint32_t win[WIN / 2 * kPair];
+    __shared__ uint16_t code[CELLS * CELLS];
+    __shared__ uint2 strengths[64];  // by level: halves limit, blimit + 1/2, thresh; 12 bits: bytes
+    __shared__ DbTile plan[2];
+    if (threadIdx.x == 0 && (int)blockIdx.x < total) plan_tile(frames, starts, n, blockIdx.x, plan[0]);
+    int k = 0;
+    for (int t = blockIdx.x; t < total; t += gridDim.x, k ^= 1) {
+        __syncthreads();  // the plan is there, and the previous tile done with shared memory
+        const DbTile& T = plan[k];
+        const int hbd = T.hbd, bd = T.bd, plane = T.plane;
+        const int gx0 = T.x - HALO, gy0 = T.y - HALO;
+        const uint32_t bias = bd == 12 ? 0u : kBias;
         {
-            // the edge codes: a thread's (at most 3) loads first, then the decodes
-            constexpr int PER = (CELLS * CELLS + kDbThreads - 1) / kDbThreads;
-            uint32_t code[PER];
+            // window: 8 consecutive samples per thread.  A window inside the
+            // plane horizontally (almost every tile) issues three loads before it
+            // stores any, so that their latencies overlap (all five at once cost the
+            // filters' loop its registers: 531 against 497 us).
+            constexpr int G = WIN / 8, ITEMS = (kRow1 - kRow0) * G, PER = 3;
+            const uint8_t* src = T.src;
+            const int stride = T.src_stride, h1 = T.h - 1, w = T.w;
+            if (gx0 >= 0 && gx0 + WIN <= w) {
+#pragma unroll 1
+                for (int i0 = threadIdx.x; i0 < ITEMS; i0 += PER * kDbThreads) {
+                    uint4 v[PER];
 #pragma unroll
-            for (int q = 0; q < PER; q++) {
-                const int i = threadIdx.x + q * kDbThreads, cr = i / CELLS, cc = i - cr * CELLS;
-                const int cy = cy0 + cr, cx = cx0 + cc;
-                code[q] = (i < CELLS * CELLS && cy >= 0 && cx >= 0 && cy < ch && cx < cw) ? codes[cy * cw + cx] : 0;
-            }
+                    for (int q = 0; q < PER; q++) {
+                        const int i = i0 + q * kDbThreads, r = kRow0 + i / G, c = i - (i / G) * G;
+                        if (i >= ITEMS) continue;
+                        const uint8_t* row = src + (size_t)clip3(0, h1, gy0 + r) * stride;
+                        if (hbd) v[q] = *reinterpret_cast<const uint4*>(row + 2 * gx0 + 16 * c);
+                        else *reinterpret_cast<uint2*>(&v[q]) = *reinterpret_cast<const uint2*>(row + gx0 + 8 * c);
+                    }
 #pragma unroll
-            for (int q = 0; q < PER; q++) {
-                const int i = threadIdx.x + q * kDbThreads;
-                if (i >= CELLS * CELLS) break;
-                ev[i] = decode_code(code[q] & 0xff, sharp);
-                eh[i] = decode_code(code[q] >> 8, sharp);
-            }
-        }
-        __syncthreads();
-        // vertical pass: window rows x edge columns 12..84 (cells 3..21: a
-        // filter moves at most 6 samples from its edge, so only those edges
-        // move tile columns; all window rows keep each warp's rows aligned to
-        // the 4-row cells)
-        constexpr int VR = WIN, VE = CELLS - 5;
-        for (int i = threadIdx.x; i < VR * VE; i += blockDim.x) {
-            int r = i % VR, cc = 3 + i / VR;
-            uint32_t prm = ev[(r >> 2) * CELLS + cc];
-            if (prm & 0xff) filter_line(&win[r * PITCH + cc * 4], 1, prm, plane, bd);
-        }
-        __syncthreads();
-        // horizontal pass: tile columns x edge rows 12..84
-        constexpr int HE = CELLS - 5;  // cells 3..21
-        for (int i = threadIdx.x; i < TILE * HE; i += blockDim.x) {
-            int c = HALO + i % TILE, cr = 3 + i / TILE;
-            uint32_t prm = eh[cr * CELLS + (c >> 2)];
-            if (prm & 0xff) filter_line(&win[cr * 4 * PITCH + c], PITCH, prm, plane, bd);
-        }
-        __syncthreads();
-        // write the tile, four samples per thread (one vector store inside the plane)
-        const int dh = min(D.h, S.h), dw = min(D.w, S.w);
-        for (int i = threadIdx.x; i < TILE * (TILE / 4); i += blockDim.x) {
-            int r = i / (TILE / 4), c = (i % (TILE / 4)) * 4;
-            int gy = ty * TILE + r, gx = tx * TILE + c;
-            if (gy >= dh) continue;
-            const uint16_t* w = &win[(r + HALO) * PITCH + c + HALO];
-            uint8_t* row = D.p + (size_t)gy * D.stride;
-            if (gx + 3 < dw) {
-                const uint32_t* w32 = reinterpret_cast<const uint32_t*>(w);  // 4-byte aligned
-                const uint2 v = make_uint2(w32[0], w32[1]);
-                if (hbd) *reinterpret_cast<uint2*>(row + 2 * gx) = v;
-                else *reinterpret_cast<uint32_t*>(row + gx) = __byte_perm(v.x, v.y, 0x6420);
+                    for (int q = 0; q < PER; q++) {
+                        const int i = i0 + q * kDbThreads, r = kRow0 + i / G, c = i - (i / G) * G;
+                        if (i >= ITEMS) continue;
+                        uint4 o;
+                        if (hbd) {
+                            o = make_uint4(v[q].x | bias, v[q].y | bias, v[q].z | bias, v[q].w | bias);
+                        } else {
+                            o = make_uint4(__byte_perm(v[q].x, kBias, 0x7170), __byte_perm(v[q].x, kBias, 0x7372),
+                                           __byte_perm(v[q].y, kBias, 0x7170), __byte_perm(v[q].y, kBias, 0x7372));
+                        }
+                        uint2* d = reinterpret_cast<uint2*>(win + (r >> 1) * kPair + (r & 1) * kRow + 4 * c);
+                        d[0] = make_uint2(o.x, o.y);
+                        d[1] = make_uint2(o.z, o.w);
+                    }
+                }
             } else {
-                for (int k = 0; k < 4 && gx + k < dw; k++) st_px(D, hbd, gy, gx + k, w[k]);
+                for (int i = threadIdx.x; i < (kRow1 - kRow0) * kRow; i += kDbThreads) {
+                    const int r = kRow0 + i / kRow, c = i % kRow;
+                    const uint8_t* row = src + (size_t)clip3(0, h1, gy0 + r) * stride;
+                    const int xa = clip3(0, w - 1, gx0 + 2 * c), xb = clip3(0, w - 1, gx0 + 2 * c + 1);
+                    const uint32_t a = hbd ? reinterpret_cast<const uint16_t*>(row)[xa] : row[xa];
+                    const uint32_t b = hbd ? reinterpret_cast<const uint16_t*>(row)[xb] : row[xb];
+                    win[(r >> 1) * kPair + (r & 1) * kRow + c] = a | b << 16 | bias;
+                }
+            }
+        }
+        {
+            const int cy0 = gy0 / 4, cx0 = gx0 / 4;  // gx0,gy0 are multiples of 4 (may be negative)
+            const int cw = T.w >> 2, ch = T.h >> 2;
+            for (int i = threadIdx.x; i < CELLS * CELLS; i += kDbThreads) {
+                const int cr = i / CELLS, cy = cy0 + cr, cx = cx0 + i - cr * CELLS;
+                code[i] = cy >= 0 && cx >= 0 && cy < ch && cx < cw ? T.codes[cy * cw + cx] : (uint16_t)0;
+            }
+        }
+        if (threadIdx.x < 64) {
+            const Strength s = strength(threadIdx.x, T.sharp);
+            uint2 e;
+            if (bd == 12) {
+                e = make_uint2((uint32_t)s.limit | (uint32_t)s.blimit << 8 | (uint32_t)s.thresh << 16, 0u);
+            } else {
+                const float scale = bd == 8 ? 1.f : 4.f;
+                const __half2 a = __floats2half2_rn(scale * s.limit, scale * s.blimit + 0.5f);
+                e = make_uint2(u32(a), u32(__float2half2_rn(scale * s.thresh)));
+            }
+            strengths[threadIdx.x] = e;
+        }
+        __syncthreads();
+        if (threadIdx.x == kDbThreads - 1 && t + (int)gridDim.x < total)
+            plan_tile(frames, starts, n, t + gridDim.x, plan[k ^ 1]);
+        HalfConsts K;
+        K.one = dup(bd == 8 ? 1.f : 4.f);
+        K.lo = dup(bd == 8 ? -128.f : -512.f);
+        K.hi = dup(bd == 8 ? 127.f : 511.f);
+        K.top = dup(bd == 8 ? 1279.f : 2047.f);
+        // vertical pass: pairs of window rows x edge columns 12..84 (cells 3..21: a
+        // filter moves at most 6 samples from its edge, so only those edges
+        // move tile columns)
+        constexpr int VP = (kRow1 - kRow0) / 2, VE = CELLS - 5;
+        for (int i = threadIdx.x; i < VP * VE; i += kDbThreads) {
+            const int e = i / VP, r = kRow0 / 2 + i - e * VP, cc = 3 + e;
+            const int c = code[(r >> 1) * CELLS + cc] & 0xff;
+            if (!c) continue;
+            uint32_t* m = win + r * kPair + cc * 2;
+            if (bd == 12) filter_lines12<true>(m, c >> 6, strengths[c & 63].x, plane);
+            else filter_pair<true>(m, c >> 6, strengths[c & 63], plane, K);
+        }
+        __syncthreads();
+        // horizontal pass: pairs of tile columns x edge rows 12..84
+        constexpr int HP = TILE / 2, HE = CELLS - 5;  // cells 3..21
+        for (int i = threadIdx.x; i < HP * HE; i += kDbThreads) {
+            const int x = HALO / 2 + i % HP, cr = 3 + i / HP;
+            const int c = code[cr * CELLS + (x >> 1)] >> 8;
+            if (!c) continue;
+            uint32_t* m = win + cr * 2 * kPair + x;
+            if (bd == 12) filter_lines12<false>(m, c >> 6, strengths[c & 63].x, plane);
+            else filter_pair<false>(m, c >> 6, strengths[c & 63], plane, K);
+        }
+        __syncthreads();
+        // write the tile, eight samples per thread (one vector store inside the plane)
+        const int dh = T.dh, dw = T.dw, dst_stride = T.dst_stride;
+        uint8_t* dst = T.dst;
+#pragma unroll
+        for (int q = 0; q < TILE * TILE / 8 / kDbThreads; q++) {
+            const int i = threadIdx.x + q * kDbThreads, r = i / (TILE / 8), c = i % (TILE / 8);
+            const int gy = T.y + r, gx = T.x + 8 * c;
+            if (gy >= dh) continue;
+            const int wr = r + HALO;
+            const uint32_t* w = win + (wr >> 1) * kPair + (wr & 1) * kRow + HALO / 2 + 4 * c;
+            const uint2 a = *reinterpret_cast<const uint2*>(w), b = *reinterpret_cast<const uint2*>(w + 2);
+            uint8_t* row = dst + (size_t)gy * dst_stride;
+            const uint32_t keep = bd == 12 ? 0xffffffffu : kSample;
+            if (gx + 7 < dw) {
+                if (hbd)
+                    *reinterpret_cast<uint4*>(row + 2 * gx) = make_uint4(a.x & keep, a.y & keep, b.x & keep, b.y & keep);
+                else
+                    *reinterpret_cast<uint2*>(row + gx) =
+                        make_uint2(__byte_perm(a.x, a.y, 0x6420), __byte_perm(b.x, b.y, 0x6420));
+            } else {
+                const uint32_t v[4] = {a.x & keep, a.y & keep, b.x & keep, b.y & keep};
+#pragma unroll
+                for (int e = 0; e < 8; e++) {
+                    const uint32_t px = (v[e / 2] >> (16 * (e & 1))) & 0xffff;
+                    if (gx + e >= dw) continue;
+                    if (hbd) reinterpret_cast<uint16_t*>(row)[gx + e] = (uint16_t)px;
+                    else row[gx + e] = (uint8_t)px;
+                }
             }
         }
     }
