@@ -134,6 +134,15 @@ void launch_superres(const FrameDev* frames, const int32_t* starts, int n, int t
                      cudaStream_t s);
 void launch_lr(const FrameDev* frames, const int32_t* starts, int n, int total, const StageShape& sh,
                cudaStream_t s);
+// A plane's copy: rows of `row` bytes.  Source rows start on 16-byte boundaries; the
+// destination's do too, or dst_stride == row.  It may be pinned host memory.
+struct PlaneCopy {
+    const uint8_t* src;
+    uint8_t* dst;
+    int32_t src_stride, dst_stride, row, height;
+};
+cudaError_t launch_plane_copies(const PlaneCopy* copies, int n, cudaStream_t s);
+
 void launch_grain(const FrameDev* frames, const int32_t* starts_tmpl, const int32_t* starts_blend,
                   int n, int total_tmpl, int total_blend, const StageShape& sh, cudaStream_t s);
 
