@@ -374,6 +374,8 @@ template <int RB>
 __global__ void __launch_bounds__(kCdefThreads, 4) cdef_kernel(const FrameDev* __restrict__ frames,
                                                       const int32_t* __restrict__ starts, int n, int total,
                                                       int full_chroma) {
+    chain_wait();
+    chain_next();
     extern __shared__ __align__(16) unsigned char cdef_raw[];
     using SM = CdefShared<RB>;
     SM& S = *reinterpret_cast<SM*>(cdef_raw);
@@ -637,7 +639,7 @@ void launch(const FrameDev* frames, const int32_t* starts, int n, int total, boo
     // the largest size either way, so that no concurrent launch finds it lowered
     cudaFuncSetAttribute(cdef_kernel<RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cdef_smem<RB>(true));
     total *= FB / RB;
-    cdef_kernel<RB><<<shape_grid(sh, total), kCdefThreads, bytes, s>>>(frames, starts, n, total, full_chroma);
+    launch_chained(cdef_kernel<RB>, shape_grid(sh, total), kCdefThreads, bytes, s, frames, starts, n, total, full_chroma);
 }
 
 }  // namespace

@@ -134,6 +134,31 @@ void launch_superres(const FrameDev* frames, const int32_t* starts, int n, int t
                      cudaStream_t s);
 void launch_lr(const FrameDev* frames, const int32_t* starts, int n, int total, const StageShape& sh,
                cudaStream_t s);
+// The chain's launches.  A small stage's CTAs take their places as the last ones of the
+// stage before leave them, and wait there (chain_wait) until it has finished and its
+// writes are visible.  Every kernel launched so calls chain_wait before anything else
+// and chain_next after it, so a stage never runs ahead of more than one other.  One
+// CIF frame's chain takes 45.4 us so against 53.4 us.  Stages of more than two CTAs per SM
+// are launched plainly: their CTAs hold places that the stage before could use (twelve
+// 718p 4:4:4 frames 733 against 708 us, sixteen 720p ones in an engine 20.3 against 19.5 ms).
+constexpr int kChainBlocks = 2 * kSMs;
+template <class... P, class... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = (long long)grid.x * grid.y <= kChainBlocks ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // A plane's copy: rows of `row` bytes.  Source rows start on 16-byte boundaries; the
 // destination's do too, or dst_stride == row.  It may be pinned host memory.
 struct PlaneCopy {

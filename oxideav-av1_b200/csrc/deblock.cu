@@ -132,6 +132,8 @@ __device__ __forceinline__ uint32_t edge_code(uint32_t cur, uint32_t prev, int s
 }
 
 __global__ void __launch_bounds__(256) lf_prep_kernel(const FrameDev* __restrict__ frames) {
+    chain_wait();
+    chain_next();
     __shared__ PrepShared S;
     const FrameDev& F = frames[blockIdx.y];
     const av1g_frame_header& h = F.h;
@@ -561,6 +563,8 @@ constexpr int kDbCtas = 6;
 
 __global__ void __launch_bounds__(kDbThreads, kDbCtas) deblock_kernel(const FrameDev* __restrict__ frames,
                                                       const int32_t* __restrict__ starts, int n, int total) {
+    chain_wait();
+    chain_next();
     __shared__ __align__(16) uint32_t win[WIN / 2 * kPair];
     __shared__ uint16_t code[CELLS * CELLS];
     __shared__ uint2 strengths[64];  // by level: halves limit, blimit + 1/2, thresh; 12 bits: bytes
@@ -729,8 +733,8 @@ int tiles_lf_prep(const FrameDev& f) {
 void launch_deblock(const FrameDev* frames, const int32_t* starts, int n, int total, int max_prep,
                     const StageShape& sh, cudaStream_t s) {
     if (total <= 0) return;
-    lf_prep_kernel<<<dim3(max_prep, n), 256, 0, s>>>(frames);
-    deblock_kernel<<<shape_grid(sh, total), kDbThreads, 0, s>>>(frames, starts, n, total);
+    launch_chained(lf_prep_kernel, dim3(max_prep, n), 256, 0, s, frames);
+    launch_chained(deblock_kernel, shape_grid(sh, total), kDbThreads, 0, s, frames, starts, n, total);
 }
 
 }  // namespace av1g

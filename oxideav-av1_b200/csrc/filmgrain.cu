@@ -256,6 +256,8 @@ constexpr int kTmplThreads = 256;
 
 __global__ void __launch_bounds__(kTmplThreads) grain_template_kernel(const FrameDev* __restrict__ frames,
                                                              const int32_t* __restrict__ starts, int n, int total) {
+    chain_wait();
+    chain_next();
     __shared__ int16_t T[3][LH * LW];
     __shared__ int prog;
     __shared__ int16_t gauss[2048];  // the lanes draw different entries: shared, not constant, memory
@@ -578,6 +580,8 @@ __device__ __noinline__ void plan_blend(const FrameDev& F, BlendPlan& P) {
 
 __global__ void __launch_bounds__(kBlendThreads, 4) grain_blend_kernel(const FrameDev* __restrict__ frames,
                                                                    const int32_t* __restrict__ starts, int n, int total) {
+    chain_wait();
+    chain_next();
     __shared__ BlendShared S;
     const BlendPlan& P = S.P;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -637,9 +641,10 @@ int tiles_grain_blend(const FrameDev& f) {
 
 void launch_grain(const FrameDev* frames, const int32_t* starts_tmpl, const int32_t* starts_blend, int n,
                   int total_tmpl, int total_blend, const StageShape& sh, cudaStream_t s) {
-    if (total_tmpl > 0) grain_template_kernel<<<total_tmpl, kTmplThreads, 0, s>>>(frames, starts_tmpl, n, total_tmpl);
+    if (total_tmpl > 0)
+        launch_chained(grain_template_kernel, total_tmpl, kTmplThreads, 0, s, frames, starts_tmpl, n, total_tmpl);
     if (total_blend <= 0) return;
-    grain_blend_kernel<<<shape_grid(sh, total_blend), kBlendThreads, 0, s>>>(frames, starts_blend, n, total_blend);
+    launch_chained(grain_blend_kernel, shape_grid(sh, total_blend), kBlendThreads, 0, s, frames, starts_blend, n, total_blend);
 }
 
 }  // namespace av1g

@@ -311,6 +311,8 @@ __device__ void plan_tile(Tile& T, const FrameDev* __restrict__ frames, const in
 
 __global__ void __launch_bounds__(kLrThreads, 4) lr_kernel(const FrameDev* __restrict__ frames,
                                                  const int32_t* __restrict__ starts, int n, int total) {
+    chain_wait();
+    chain_next();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Smem& s = *reinterpret_cast<Smem*>(smem_raw);
     for (int z = threadIdx.x; z < 256; z += blockDim.x)
@@ -582,7 +584,7 @@ void launch_lr(const FrameDev* frames, const int32_t* starts, int n, int total, 
     if (total <= 0) return;
     size_t bytes = lr_smem_bytes();
     cudaFuncSetAttribute(lr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    lr_kernel<<<shape_grid(sh, total), kLrThreads, bytes, s>>>(frames, starts, n, total);
+    launch_chained(lr_kernel, shape_grid(sh, total), kLrThreads, bytes, s, frames, starts, n, total);
 }
 
 }  // namespace av1g

@@ -157,6 +157,8 @@ __device__ __forceinline__ int dot(const int (&x)[6], const Taps& c, const Taps&
 template <int TILE>
 __global__ void __launch_bounds__(kSrThreads, 4) superres_kernel(const FrameDev* __restrict__ frames,
                                                               const int32_t* __restrict__ starts, int n, int total) {
+    chain_wait();
+    chain_next();
     constexpr int kPitch = sr_pitch(TILE);
     constexpr int kGroups = (TILE + kSrPad - 8) / 4;  // groups of four source samples at most
     constexpr int kLoads = (kGroups + 31) / 32;       // a lane's
@@ -265,7 +267,7 @@ void launch_superres(const FrameDev* frames, const int32_t* starts, int n, int t
                      cudaStream_t s) {
     if (total <= 0) return;
     const auto kernel = sh.tile == 256 ? superres_kernel<256> : sh.tile == 512 ? superres_kernel<512> : superres_kernel<1024>;
-    kernel<<<shape_grid(sh, total), kSrThreads, 0, s>>>(frames, starts, n, total);
+    launch_chained(kernel, shape_grid(sh, total), kSrThreads, 0, s, frames, starts, n, total);
 }
 
 }  // namespace av1g
