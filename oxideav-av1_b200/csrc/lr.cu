@@ -26,11 +26,12 @@
 //    are not computed.
 // Units of type RESTORE_NONE copy the CDEF samples through.
 //
-// Bound by instruction issue (198 thread instructions per sample when every
-// thread worked its tile out for itself, with 64-bit divisions for the box
-// filter's scale): 64 x 1080p 8-bit 1.67 -> 1.38 ms with one thread working out
-// the next tile and the scales in a table.  Four CTAs per SM: five, at 48
-// registers, take 1.50 ms.
+// Bound by instruction issue: 64 x 1080p 8-bit took 1.67 ms at 198 thread instructions
+// per sample, when every thread worked its tile out for itself, with 64-bit divisions
+// for the box filter's scale; 1.38 ms with one thread working out the next tile and
+// the scales in a table; 1.29 ms with a and b in one word and the 3x3 weighting of a
+// pair of rows from one reading of them (three loads per output, not nine).  Four
+// CTAs per SM: five, at 48 registers, took 1.50 against 1.38 ms.
 #include <cstddef>
 
 #include "common.cuh"
@@ -88,8 +89,8 @@ struct Smem {
     uint16_t src[SH * SP];
     int v1[AR * VW];      // column sums; the Wiener intermediate reuses v1/v2
     int v2[AR * VW];
-    int B[AR * AP];
-    uint16_t A[AR * AP];
+    uint32_t AB[AR * AP];  // b << kABits | a; 12 bits: b alone
+    uint16_t A[AR * AP];   // 12 bits: a
     uint16_t a2lut[256];
     Tile tile[2];  // the current one, and the next one while it is worked out
 };
@@ -115,6 +116,12 @@ __device__ __forceinline__ int count_units(int us, int sz) {
     return n > 1 ? n : 1;
 }
 
+// At 8 and 10 bits the coefficients a (at most 256) and b (at most 261,120) share a
+// word, and the sums of up to five of them that the 3x3 weighting needs do too
+// (1,280 below 2^11, 1,305,600 below 2^21).
+constexpr int kABits = 11;
+constexpr uint32_t kAMask = (1u << kABits) - 1;
+
 // Box sums, a/b coefficients (box_filter, loop_restoration.rs:594-700) for
 // radius R over the A/B grid rows i in [-1, th] (stored at i + 1), columns
 // j in [-1, tw].  The self-guided sets use R = 2 only for the first pass,
@@ -123,13 +130,13 @@ __device__ __forceinline__ int count_units(int us, int sz) {
 // the rows and row sums slide along the columns, so each sum costs two loads
 // instead of 2R + 1; the runs have fixed lengths so the loops unroll and the
 // coefficient arithmetic of neighbouring positions overlaps.
-template <int R, bool HBD>
-__device__ void box_coeffs(Smem& s, int th, int tw, int bd, const SgrPass& ps, int y0) {
+template <int R, int BD>
+__device__ void box_coeffs(Smem& s, int th, int tw, const SgrPass& ps, int y0) {
     constexpr bool ODD = R == 2;
     constexpr int n = (2 * R + 1) * (2 * R + 1);
     const unsigned sm = ps.scale, pcap = ps.pcap;
     constexpr int one_over_n = ((1 << 12) + n / 2) / n;
-    const int sa = 2 * (bd - 8), sb = bd - 8;
+    constexpr int sa = 2 * (BD - 8), sb = BD - 8;
     const int vw = tw + 2 * H3;
     const int rows = th + 2;
     // column sums: one thread per (column, run of 12 grid rows): 3 x 71
@@ -189,13 +196,13 @@ __device__ void box_coeffs(Smem& s, int th, int tw, int bd, const SgrPass& ps, i
             a += c2[d];
         }
         uint16_t* ao = s.A + row * AP + ja + 1;
-        int* bo = s.B + row * AP + ja + 1;
+        uint32_t* bo = s.AB + row * AP + ja + 1;
 #pragma unroll
         for (int t = 0; t < CRUN; t++) {
             if (ja + t >= jb) break;
-            // 8-bit: both shifts are 0 (the branch is decided at compile time)
-            const int ar = HBD ? (a + (1 << (sa - 1))) >> sa : a;
-            const int dr = HBD ? (b + (1 << (sb - 1))) >> sb : b;
+            // 8-bit: both shifts are 0
+            const int ar = BD > 8 ? (a + ((1 << sa) >> 1)) >> sa : a;
+            const int dr = BD > 8 ? (b + ((1 << sb) >> 1)) >> sb : b;
             int p = ar * n - dr * dr;
             if (p < 0) p = 0;
             const unsigned z = (min((unsigned)p, pcap) * sm + (1u << 19)) >> 20;
@@ -204,8 +211,9 @@ __device__ void box_coeffs(Smem& s, int th, int tw, int bd, const SgrPass& ps, i
             // (loop_restoration.rs:660-661); (256 - a2) * b * one_over_n
             // stays below 2^32 at every bit depth (b <= 25 * 4095)
             const unsigned b2 = (unsigned)(256 - a2) * (unsigned)b * (unsigned)one_over_n;
-            ao[t] = (uint16_t)a2;
-            bo[t] = (int)((b2 + (1u << 11)) >> 12);
+            const uint32_t bq = (b2 + (1u << 11)) >> 12;
+            if (BD == 12) ao[t] = (uint16_t)a2;
+            bo[t] = BD == 12 ? bq : (bq << kABits | (uint32_t)a2);
             b += c1[t + 2 * R + 1] - c1[t];
             a += c2[t + 2 * R + 1] - c2[t];
         }
@@ -213,62 +221,92 @@ __device__ void box_coeffs(Smem& s, int th, int tw, int bd, const SgrPass& ps, i
     __syncthreads();
 }
 
-// 3x3 weighting of A/B (loop_restoration.rs:700-736) for the four outputs
-// (i, j0 .. j0 + 3), reading each A/B column once.
-__device__ __forceinline__ void box_weight4(const Smem& s, int i, int j0, const int u[4], int pass, int y0,
-                                            int out[4]) {
-    const uint16_t* a = s.A + i * AP + j0;  // top-left of the first 3x3 window
-    const int* b = s.B + i * AP + j0;
-    int ac[3][6], bc[3][6];
-    int shift;
-    if (pass == 0) {
-        const bool odd = (y0 + i) & 1;
-        shift = odd ? 4 : 5;
-        if (odd) {  // centre row only, weights 5 6 5
-#pragma unroll
-            for (int c = 0; c < 6; c++) {
-                ac[1][c] = a[AP + c];
-                bc[1][c] = b[AP + c];
-            }
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                int as = 5 * (ac[1][e] + ac[1][e + 2]) + 6 * ac[1][e + 1];
-                int bs = 5 * (bc[1][e] + bc[1][e + 2]) + 6 * bc[1][e + 1];
-                int v = as * u[e] + bs, sh = 8 + shift - 4;
-                out[e] = (v + (1 << (sh - 1))) >> sh;
-            }
-        } else {    // rows above and below
-#pragma unroll
-            for (int c = 0; c < 6; c++) {
-                ac[0][c] = a[c] + a[2 * AP + c];
-                bc[0][c] = b[c] + b[2 * AP + c];
-            }
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                int as = 5 * (ac[0][e] + ac[0][e + 2]) + 6 * ac[0][e + 1];
-                int bs = 5 * (bc[0][e] + bc[0][e + 2]) + 6 * bc[0][e + 1];
-                int v = as * u[e] + bs, sh = 8 + shift - 4;
-                out[e] = (v + (1 << (sh - 1))) >> sh;
-            }
-        }
-        return;
-    }
-#pragma unroll
-    for (int rr = 0; rr < 3; rr++)
+// 3x3 weighting of A/B (loop_restoration.rs:700-736) for the outputs (i, j0 .. j0 + 3)
+// and (i + 1, j0 .. j0 + 3), i even, reading each A/B entry once.  y0 is even (stripes
+// and their halves start on even rows), so i + 1 is an odd plane row.  Weights: first pass,
+// even rows 5 6 5 above and below, odd rows 5 6 5 in their own row; second pass 4 in the
+// cross, 3 in the corners.
+__device__ __forceinline__ int weigh(int wk, uint32_t k, int wc, uint32_t c, int u, int sh) {
+    const int as = wk * (int)(k & kAMask) + wc * (int)(c & kAMask);
+    const int bs = wk * (int)(k >> kABits) + wc * (int)(c >> kABits);
+    return (as * u + bs + (1 << (sh - 1))) >> sh;
+}
+template <int PASS>
+__device__ __forceinline__ void weight_pair(const Smem& s, int i, int j0, const int (&u)[2][4], int (&out)[2][4]) {
+    const uint32_t* g = s.AB + i * AP + j0;  // top-left of the first 3x3 window
+    uint32_t top[6], mid[6], low[6];
+    if (PASS == 0) {
 #pragma unroll
         for (int c = 0; c < 6; c++) {
-            ac[rr][c] = a[rr * AP + c];
-            bc[rr][c] = b[rr * AP + c];
+            low[c] = g[2 * AP + c];
+            top[c] = g[c] + low[c];
         }
 #pragma unroll
-    for (int e = 0; e < 4; e++) {
-        int ca = ac[0][e + 1] + ac[1][e] + ac[1][e + 1] + ac[1][e + 2] + ac[2][e + 1];
-        int cb = bc[0][e + 1] + bc[1][e] + bc[1][e + 1] + bc[1][e + 2] + bc[2][e + 1];
-        int as = 3 * (ac[0][e] + ac[0][e + 2] + ac[2][e] + ac[2][e + 2]) + 4 * ca;
-        int bs = 3 * (bc[0][e] + bc[0][e + 2] + bc[2][e] + bc[2][e + 2]) + 4 * cb;
-        int v = as * u[e] + bs, sh = 8 + 5 - 4;
-        out[e] = (v + (1 << (sh - 1))) >> sh;
+        for (int e = 0; e < 4; e++) {
+            out[0][e] = weigh(5, top[e] + top[e + 2], 6, top[e + 1], u[0][e], 9);
+            out[1][e] = weigh(5, low[e] + low[e + 2], 6, low[e + 1], u[1][e], 8);
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+            const uint32_t r1 = g[AP + c], r2 = g[2 * AP + c];
+            top[c] = g[c] + r2;         // rows above and below the first output
+            mid[c] = r1;
+            low[c] = r2;
+        }
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            out[0][e] = weigh(3, top[e] + top[e + 2], 4, top[e + 1] + mid[e] + mid[e + 1] + mid[e + 2], u[0][e], 9);
+#pragma unroll
+        for (int c = 0; c < 6; c++) top[c] = mid[c] + g[3 * AP + c];
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+            out[1][e] = weigh(3, top[e] + top[e + 2], 4, top[e + 1] + low[e] + low[e + 1] + low[e + 2], u[1][e], 9);
     }
+}
+
+// The same at 12 bits, one row at a time from the two arrays.
+template <int PASS>
+__device__ __noinline__ int4 weight_row12(const Smem& s, int i, int j0, int4 uq) {
+    const uint16_t* a = s.A + i * AP + j0;
+    const uint32_t* b = s.AB + i * AP + j0;
+    const bool odd = i & 1;
+    // weights of the three rows' side and middle columns
+    const int ws[3] = {PASS ? 3 : (odd ? 0 : 5), PASS ? 4 : (odd ? 5 : 0), PASS ? 3 : (odd ? 0 : 5)};
+    const int wm[3] = {PASS ? 4 : (odd ? 0 : 6), PASS ? 4 : (odd ? 6 : 0), PASS ? 4 : (odd ? 0 : 6)};
+    const int sh = PASS || !odd ? 9 : 8;
+    const int u[4] = {uq.x, uq.y, uq.z, uq.w};
+    int out[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        int as = 0, bs = 0;
+        for (int r = 0; r < 3; r++) {
+            if (!wm[r]) continue;  // the first pass has no other rows' entries
+            const int o = r * AP + e;
+            as += ws[r] * (a[o] + a[o + 2]) + wm[r] * a[o + 1];
+            bs += ws[r] * (int)(b[o] + b[o + 2]) + wm[r] * (int)b[o + 1];
+        }
+        out[e] = (as * u[e] + bs + (1 << (sh - 1))) >> sh;
+    }
+    return make_int4(out[0], out[1], out[2], out[3]);
+}
+template <int PASS>
+__device__ __forceinline__ void weight_pair(const Smem& s, int bd, int i, int j0, const int (&u)[2][4], int (&out)[2][4]) {
+    if (bd == 12) {
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const int4 v = weight_row12<PASS>(s, i + e, j0, make_int4(u[e][0], u[e][1], u[e][2], u[e][3]));
+            out[e][0] = v.x, out[e][1] = v.y, out[e][2] = v.z, out[e][3] = v.w;
+        }
+    } else {
+        weight_pair<PASS>(s, i, j0, u, out);
+    }
+}
+template <int R>
+__device__ __forceinline__ void box_coeffs(Smem& s, int th, int tw, int bd, const SgrPass& ps, int y0) {
+    if (bd == 8) box_coeffs<R, 8>(s, th, tw, ps, y0);
+    else if (bd == 10) box_coeffs<R, 10>(s, th, tw, ps, y0);
+    else box_coeffs<R, 12>(s, th, tw, ps, y0);
 }
 
 // Tile t of the batch: its frame, plane, stripe half, column tile and
@@ -500,48 +538,42 @@ __global__ void __launch_bounds__(kLrThreads, 4) lr_kernel(const FrameDev* __res
         const SgrPass &p0 = c_sgr.pass[set][0], &p1 = c_sgr.pass[set][1];
         const int r0 = p0.r, r1 = p1.r;
         const int w0 = u.sgr_xqd[0], w1 = u.sgr_xqd[1], w2 = 128 - w0 - w1;
-        // outputs in runs of four along a row, two runs per thread, the same
-        // in both passes, so that the first pass's outputs stay in registers.
-        // Rows of one parity run together (the first pass weights odd and even
-        // rows differently), so a warp's two rows share a code path.
-        constexpr int Q = TW / 4, RUNS = TH * Q / kLrThreads;
-        const int n_odd = (th + ((y0 & 1) ? 1 : 0)) >> 1;      // rows i with (y0 + i) odd
-        const int odd0 = (y0 & 1) ? 0 : 1;
-        auto run_row = [&](int rk) { return rk < n_odd ? odd0 + 2 * rk : (1 - odd0) + 2 * (rk - n_odd); };
-        int f0[RUNS][4] = {};
-        if (r0) {
-            if (bd > 8) box_coeffs<2, true>(s, th, tw, bd, p0, y0);  // r0 is 2 in every set that has it
-            else box_coeffs<2, false>(s, th, tw, bd, p0, y0);
+        // a thread's outputs: four along a row in a pair of rows, the same in both
+        // passes, so that the first pass's outputs stay in registers and the rows of
+        // the A/B grid that the two share are read once
+        constexpr int Q = TW / 4;
+        static_assert(TH / 2 * Q == kLrThreads, "one run of four in a pair of rows per thread");
+        const int i0 = 2 * (threadIdx.x / Q), j0 = (threadIdx.x % Q) * 4;
+        const bool mine = i0 < th && j0 < tw;
+        int f0[2][4] = {}, uq[2][4];
+        auto load_u = [&] {
 #pragma unroll
-            for (int e = 0; e < RUNS; e++) {
-                const int k = threadIdx.x + e * kLrThreads, rk = k / Q, j0 = (k - rk * Q) * 4;
-                if (rk >= th || j0 >= tw) continue;
-                const int i = run_row(rk);
-                int uq[4];
+            for (int e = 0; e < 2; e++)
 #pragma unroll
-                for (int q = 0; q < 4; q++) uq[q] = s.src[(i + H3) * SP + j0 + q + H3];
-                box_weight4(s, i, j0, uq, 0, y0, f0[e]);
+                for (int q = 0; q < 4; q++) uq[e][q] = s.src[(i0 + e + H3) * SP + j0 + q + H3];
+        };
+        if (r0) {  // r0 is 2 in every set that has it
+            box_coeffs<2>(s, th, tw, bd, p0, y0);
+            if (mine) {
+                load_u();
+                weight_pair<0>(s, bd, i0, j0, uq, f0);
             }
             __syncthreads();
         }
-        if (r1) {  // r1 is 1 in every set that has it
-            if (bd > 8) box_coeffs<1, true>(s, th, tw, bd, p1, y0);
-            else box_coeffs<1, false>(s, th, tw, bd, p1, y0);
-        }
+        if (r1) box_coeffs<1>(s, th, tw, bd, p1, y0);  // r1 is 1 in every set that has it
+        if (!mine) continue;
+        int f1[2][4];
+        load_u();
+        if (r1) weight_pair<1>(s, bd, i0, j0, uq, f1);
 #pragma unroll
-        for (int e = 0; e < RUNS; e++) {
-            const int k = threadIdx.x + e * kLrThreads, rk = k / Q, j0 = (k - rk * Q) * 4;
-            if (rk >= th || j0 >= tw) continue;
-            const int i = run_row(rk);
-            int uq[4], f1[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) uq[q] = s.src[(i + H3) * SP + j0 + q + H3];
-            if (r1) box_weight4(s, i, j0, uq, 1, y0, f1);
+        for (int e = 0; e < 2; e++) {
+            const int i = i0 + e;
+            if (i >= th) break;
             int o[4];
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                const int uu = uq[q] << 4;
-                const int v = w1 * uu + w0 * (r0 ? f0[e][q] : uu) + w2 * (r1 ? f1[q] : uu);
+                const int uu = uq[e][q] << 4;
+                const int v = w1 * uu + w0 * (r0 ? f0[e][q] : uu) + w2 * (r1 ? f1[e][q] : uu);
                 o[q] = clip3(0, maxv, (v + (1 << 10)) >> 11);
             }
             if (j0 + 4 <= tw && !((x0 + j0) & 3)) {  // one aligned vector store
@@ -553,7 +585,7 @@ __global__ void __launch_bounds__(kLrThreads, 4) lr_kernel(const FrameDev* __res
                     *reinterpret_cast<uint32_t*>(row + x0 + j0) =
                         (uint32_t)o[0] | (uint32_t)o[1] << 8 | (uint32_t)o[2] << 16 | (uint32_t)o[3] << 24;
             } else {
-                for (int e = 0; e < 4 && j0 + e < tw; e++) st_px(O, hbd, y0 + i, x0 + j0 + e, o[e]);
+                for (int q = 0; q < 4 && j0 + q < tw; q++) st_px(O, hbd, y0 + i, x0 + j0 + q, o[q]);
             }
         }
     }
