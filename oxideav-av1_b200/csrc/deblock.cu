@@ -403,7 +403,7 @@ __device__ __forceinline__ void filter_pair(uint32_t* m, int cls, uint2 st, int 
     const uint32_t on = __hle2_mask(dl, h2(__byte_perm(st.x, 0u, 0x1010))) &
                         __hle2_mask(step, h2(__byte_perm(st.x, 0u, 0x3232)));
     if (!on) return;
-    uint32_t flat = 0, flat2 = 0;
+    uint32_t flat = 0;
     if (cls >= 2) {
         __half2 df = far(far(d1, p2, p0), q2, q0);
         if (!plane) df = far(far(df, p3, p0), q3, q0);

@@ -8,6 +8,7 @@
 // prepares on its calling threads.
 #include "host_pool.h"
 
+#include <emmintrin.h>
 #include <unistd.h>
 
 #include <algorithm>
@@ -40,7 +41,7 @@ struct Pool {
     std::condition_variable work, left;
     std::vector<Task*> open;  // tasks with parts not handed out yet, oldest first
     pid_t pid = getpid();
-    int threads = 0;
+    int threads = 0, idle = 0;
     bool started = false;
 
     void run(Task& t) {
@@ -59,7 +60,9 @@ struct Pool {
     void helper() {
         std::unique_lock<std::mutex> lk(mu);
         for (;;) {
+            idle++;
             while (open.empty()) work.wait(lk);
+            idle--;
             Task* t = open.front();
             t->helpers++;
             lk.unlock();
@@ -105,17 +108,31 @@ void parallel_for(int n, long long items, const std::function<void(int)>& fn) {
         return;
     }
     Task t{&fn, n};
+    int wake;
     {
         std::lock_guard<std::mutex> lk(P.mu);
         if (!P.started) P.start();
         P.open.push_back(&t);
+        wake = std::min(n - 1, P.threads);
+        if (P.idle) wake = std::min(wake, P.idle);
     }
-    P.work.notify_all();
+    // no more than there is work for: calls on other threads share the helpers
+    for (int k = 0; k < wake; k++) P.work.notify_one();
     P.run(t);
     std::unique_lock<std::mutex> lk(P.mu);
     P.open.erase(std::remove(P.open.begin(), P.open.end(), &t), P.open.end());
     while (t.helpers > 0) P.left.wait(lk);
     if (t.error) std::rethrow_exception(t.error);
+}
+
+void write_back(void* p, size_t n) {
+    constexpr uintptr_t kLine = 64;
+    const uintptr_t a = ((uintptr_t)p + kLine - 1) & ~(kLine - 1), b = ((uintptr_t)p + n) & ~(kLine - 1);
+    for (uintptr_t q = a; q < b; q += 16) {
+        __m128i* w = reinterpret_cast<__m128i*>(q);
+        _mm_stream_si128(w, _mm_load_si128(w));
+    }
+    _mm_sfence();
 }
 
 }  // namespace av1g

@@ -17,4 +17,10 @@ void parallel_for(int n, long long items, const std::function<void(int)>& fn);
 // each: 1 (no helpers involved) for small calls.
 int parallel_parts(long long items, long long grain);
 
+// Sends the whole cache lines of [p, p + n), which the caller has just written and
+// nobody else touches, to memory.  A part of an upload that stays in its thread's
+// cache is fetched from there by the copy engine: 6 MB written by eight threads took 696 us
+// to copy to the device, against 128 us when one thread had written them.
+void write_back(void* p, size_t n);
+
 }  // namespace av1g

@@ -846,6 +846,9 @@ av1g_status inter_run(const av1g_inter_job* jobs, int n, cudaStream_t st, std::s
                     dst[k] = c;
                     starts[at + k] = first + tiles[k];
                 }
+                if (runs.size() == 1) return;
+                write_back(dst, sizeof(Call) * from.size());
+                write_back(starts + at, sizeof(uint32_t) * from.size());
             };
             put(r.a, o_a, r.at_a, r.sa, sa, r.tile_a);
             put(r.b, o_b, r.at_b, r.sb, sb, r.tile_b);

@@ -1767,6 +1767,11 @@ av1g_status intra_run_status(const av1g_intra_job* jobs, int n, cudaStream_t st,
                     r.res.coeff_offset = (uint32_t)c.ints;
                     c.ints += px;
                 }
+                if (parts > 1) write_back(tus + it.tu_first, sizeof(av1g_intra_tu) * (size_t)(it.tu_end - it.tu_first));
+            }
+            if (parts > 1) {
+                write_back(small + at[u].small, sizeof(ResTask) * (c.small - at[u].small));
+                write_back(large + at[u].large, sizeof(ResTask) * (c.large - at[u].large));
             }
         });
         memcpy(host + off_items, plan.items.data(), sizeof(SbItem) * plan.items.size());

@@ -192,10 +192,13 @@ av1g_status recon_run(const av1g_recon_job* jobs, int n, cudaStream_t s, std::st
         TuDev* dst = reinterpret_cast<TuDev*>(host + off_tus);
         parallel_for((int)runs.size(), (long long)total, [&](int u) {
             Run& r = runs[u];
+            const Run from = r;
             for (int k = r.k0; k < r.k1; k++) {
                 const av1g_tu& t = jobs[r.job].tus[k];
                 dst[r.at[t.tx_size * 16 + t.tx_type]++] = TuDev{t, r.job};
             }
+            if (runs.size() > 1)
+                for (int b = 0; b < kKeys; b++) write_back(dst + from.at[b], sizeof(TuDev) * (r.at[b] - from.at[b]));
         });
         memcpy(host + off_tasks, tasks.data(), sizeof(Task) * tasks.size());
     });

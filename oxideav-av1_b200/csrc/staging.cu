@@ -69,7 +69,7 @@ cudaError_t reap() {
 // cudaMallocAsync with a pool that keeps its memory.  The default pool's
 // release threshold is 0, so whenever the caller synchronises it unmaps all that
 // is free, and the next call maps it again: 0.3 to 3 ms of host time per
-// allocation on a B200 box, paid by every entry point that synchronises (and by
+// allocation, paid by every entry point that synchronises (and by
 // every caller that waits for a result).  The threshold is raised once per device, to a
 // bound that holds a 4K key frame's workspace, and only where it is still 0: one
 // that the application or a serving engine has set stands.  The pool is the
