@@ -542,7 +542,7 @@ def run_recon_stages(args, dev, stream):
         walls.append((time.perf_counter() - h0) * 1e3)
     hms = max(0.0, min(walls) - ms)
     area = int((tw[fi.tus["tx_size"]] * th[fi.tus["tx_size"]]).sum())
-    out["intra"] = {"kernels": ["intra_res_kernel", "intra_kernel"], "ms_per_frame": ms, "host_ms_per_call": hms,
+    out["intra"] = {"kernels": ["intra_pre_kernel", "intra_kernel"], "ms_per_frame": ms, "host_ms_per_call": hms,
                     "tus": len(fi.tus), "tus_per_us": len(fi.tus) / (ms * 1e3),
                     "bound": "latency: the TU dependency chain of the superblock wavefront",
                     "algorithmic_bytes": fi.coeffs.nbytes + 2 * area * S}
@@ -562,7 +562,7 @@ def run_recon_stages(args, dev, stream):
     fu = synth.make_intra_frame(9004, 3840, 2160, bit_depth=10, sb_size=128, tiles=(1, 1))
     du = postfilter.DeviceIntra(fu, device=dev)
     msu, _ = _device_ms(stream, lambda: postfilter.run_intra([du], stream=stream), reps=3)
-    out["intra_uhd"] = {"kernels": ["intra_res_kernel", "intra_kernel"], "frame": "3840x2160 10-bit 4:2:0, "
+    out["intra_uhd"] = {"kernels": ["intra_pre_kernel", "intra_kernel"], "frame": "3840x2160 10-bit 4:2:0, "
                         "128x128 superblocks, 2 x 2 tiles", "ms_per_frame": msu, "tus": len(fu.tus),
                         "tus_per_us": len(fu.tus) / (msu * 1e3)}
     return out
