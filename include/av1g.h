@@ -745,6 +745,10 @@ av1g_status av1g_engine_create(const av1g_config* cfg, av1g_engine** out);
 void av1g_engine_destroy(av1g_engine* e);
 av1g_status av1g_engine_get_stats(av1g_engine* e, av1g_engine_stats* out);
 
+/* Test hook: the engine's next `outputs` output blocks are refused as if no
+ * pinned memory were to be had.  No counterpart in the reference. */
+av1g_status av1g_test_engine_faults(av1g_engine* e, int32_t outputs);
+
 /* AV1G_ENOMEM_BUDGET when the stream's reference slots do not fit the
  * remaining budget (retry after another stream closes). */
 av1g_status av1g_stream_open(av1g_engine* e, const av1g_seq_info* seq, av1g_stream** out);

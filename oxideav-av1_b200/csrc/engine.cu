@@ -181,6 +181,7 @@ struct av1g_engine {
     std::mutex pin_mu;
     std::multimap<size_t, uint8_t*> pinned_free;
     std::vector<uint8_t*> pinned_slabs;
+    std::atomic<int> output_faults{0};  // test hook (av1g_test_engine_faults): output blocks still to be refused
 
     uint8_t* pinned_get(size_t n) {
         // power-of-two capacities (from 256 KiB), so buffers recycle across
@@ -633,7 +634,8 @@ void enqueue_step(av1g_engine* E, cudaStream_t cs, std::vector<std::shared_ptr<T
                 }
                 size_t need = 0;
                 for (int p = 0; p < np; p++) need += (size_t)src[p].width * bps * src[p].height;
-                t.host_out = E->pinned_get(need);
+                const bool refuse = E->output_faults.load() > 0 && E->output_faults.fetch_sub(1) > 0;
+                t.host_out = refuse ? nullptr : E->pinned_get(need);
                 t.host_bytes = need;
                 if (!t.host_out) {
                     fail_work(w, AV1G_EDEVICE, "pinned output allocation failed");
@@ -659,7 +661,9 @@ void enqueue_step(av1g_engine* E, cudaStream_t cs, std::vector<std::shared_ptr<T
     const cudaError_t ce = launch_plane_copies(copies.data(), (int)copies.size(), cs);
     for (Work& w : works) {
         if (!w.failed && ce != cudaSuccess) fail_work(w, AV1G_EDEVICE, std::string("plane copy: ") + cudaGetErrorString(ce));
-        if (!w.failed && w.payload)
+        // whatever became of its output, a frame that is whole in its payload refreshes
+        // its slots: the stream's next frames are predicted from it
+        if (w.payload && ce == cudaSuccess)
             for (int k = 0; k < 8; k++)
                 if ((w.t->refresh >> k) & 1) w.t->st->slots[k] = w.payload;
         if (w.B.dev) cudaFreeAsync(w.B.dev, cs);
@@ -940,6 +944,12 @@ av1g_status av1g_engine_get_stats(av1g_engine* E, av1g_engine_stats* o) {
     o->host_ms = E->host_ms;
     o->device_ms = E->device_ms;
     for (int k = 0; k < 6; k++) o->host_stage_ms[k] = E->host_stage_ms[k];
+    return AV1G_OK;
+}
+
+av1g_status av1g_test_engine_faults(av1g_engine* E, int32_t outputs) {
+    if (!E) return AV1G_EINVAL;
+    E->output_faults.store(outputs);
     return AV1G_OK;
 }
 
