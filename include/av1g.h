@@ -746,8 +746,10 @@ void av1g_engine_destroy(av1g_engine* e);
 av1g_status av1g_engine_get_stats(av1g_engine* e, av1g_engine_stats* out);
 
 /* Test hook: the engine's next `outputs` output blocks are refused as if no
- * pinned memory were to be had.  No counterpart in the reference. */
-av1g_status av1g_test_engine_faults(av1g_engine* e, int32_t outputs);
+ * pinned memory were to be had, and the plane copies of its next `copies`
+ * steps as if their launch failed.  Host side only: nothing of them is
+ * enqueued.  No counterpart in the reference. */
+av1g_status av1g_test_engine_faults(av1g_engine* e, int32_t outputs, int32_t copies);
 
 /* AV1G_ENOMEM_BUDGET when the stream's reference slots do not fit the
  * remaining budget (retry after another stream closes). */

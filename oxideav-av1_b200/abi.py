@@ -460,7 +460,7 @@ _SIGS = {
     "av1g_engine_create": (C.c_int, [C.POINTER(Config), C.POINTER(C.c_void_p)]),
     "av1g_engine_destroy": (None, [C.c_void_p]),
     "av1g_engine_get_stats": (C.c_int, [C.c_void_p, C.POINTER(EngineStats)]),
-    "av1g_test_engine_faults": (C.c_int, [C.c_void_p, C.c_int32]),
+    "av1g_test_engine_faults": (C.c_int, [C.c_void_p, C.c_int32, C.c_int32]),
     "av1g_stream_open": (C.c_int, [C.c_void_p, C.POINTER(SeqInfo), C.POINTER(C.c_void_p)]),
     "av1g_stream_close": (C.c_int, [C.c_void_p]),
     "av1g_stream_reset_refs": (C.c_int, [C.c_void_p]),

@@ -166,7 +166,8 @@ struct PlaneCopy {
     uint8_t* dst;
     int32_t src_stride, dst_stride, row, height;
 };
-cudaError_t launch_plane_copies(const PlaneCopy* copies, int n, cudaStream_t s);
+// done: how many of them are enqueued (all of them unless a launch fails).
+cudaError_t launch_plane_copies(const PlaneCopy* copies, int n, cudaStream_t s, int* done);
 
 void launch_grain(const FrameDev* frames, const int32_t* starts_tmpl, const int32_t* starts_blend,
                   int n, int total_tmpl, int total_blend, const StageShape& sh, cudaStream_t s);

@@ -181,7 +181,8 @@ struct av1g_engine {
     std::mutex pin_mu;
     std::multimap<size_t, uint8_t*> pinned_free;
     std::vector<uint8_t*> pinned_slabs;
-    std::atomic<int> output_faults{0};  // test hook (av1g_test_engine_faults): output blocks still to be refused
+    // test hook (av1g_test_engine_faults): output blocks and copy launches still to be refused
+    std::atomic<int> output_faults{0}, copy_faults{0};
 
     uint8_t* pinned_get(size_t n) {
         // power-of-two capacities (from 256 KiB), so buffers recycle across
@@ -325,6 +326,7 @@ struct Work {
     av1g_ref_frame refs[7] = {};
     av1g_frame_header pf_hdr = {};        // header the post-filter chain sees
     std::shared_ptr<SlotBuf> payload;     // what the frame leaves in its slots
+    int copies = 0, slot_copies = 0, all_copies = 0;  // its plane copies: first, end of the slot's, end of the output's
     bool decode = false, run_chain = false, failed = false;
 };
 
@@ -575,6 +577,7 @@ void enqueue_step(av1g_engine* E, cudaStream_t cs, std::vector<std::shared_ptr<T
         Work& w = works[i];
         Ticket& t = *w.t;
         cudaError_t e = cudaSuccess;
+        w.copies = w.slot_copies = w.all_copies = (int)copies.size();
         if (!w.failed) {
             std::shared_ptr<SlotBuf> payload;
             PlaneDev pre[3] = {}, out[3] = {};
@@ -618,6 +621,7 @@ void enqueue_step(av1g_engine* E, cudaStream_t cs, std::vector<std::shared_ptr<T
                 payload = w.shown_slot;
             }
             if (!w.failed) w.payload = payload;
+            w.slot_copies = (int)copies.size();
             bool shown = !w.failed && (t.show || t.show_existing);
             if (shown) {
                 av1g_plane src[3] = {};
@@ -657,13 +661,19 @@ void enqueue_step(av1g_engine* E, cudaStream_t cs, std::vector<std::shared_ptr<T
                 }
             }
         }
+        w.all_copies = (int)copies.size();
     }
-    const cudaError_t ce = launch_plane_copies(copies.data(), (int)copies.size(), cs);
+    int done = 0;
+    const cudaError_t ce = E->copy_faults.load() > 0 && E->copy_faults.fetch_sub(1) > 0
+                               ? cudaErrorUnknown
+                               : launch_plane_copies(copies.data(), (int)copies.size(), cs, &done);
     for (Work& w : works) {
-        if (!w.failed && ce != cudaSuccess) fail_work(w, AV1G_EDEVICE, std::string("plane copy: ") + cudaGetErrorString(ce));
+        // a frame that owns a copy which was not enqueued fails
+        if (!w.failed && w.all_copies > w.copies && w.all_copies > done)
+            fail_work(w, AV1G_EDEVICE, std::string("plane copy: ") + cudaGetErrorString(ce));
         // whatever became of its output, a frame that is whole in its payload refreshes
         // its slots: the stream's next frames are predicted from it
-        if (w.payload && ce == cudaSuccess)
+        if (w.payload && (w.slot_copies == w.copies || w.slot_copies <= done))
             for (int k = 0; k < 8; k++)
                 if ((w.t->refresh >> k) & 1) w.t->st->slots[k] = w.payload;
         if (w.B.dev) cudaFreeAsync(w.B.dev, cs);
@@ -947,9 +957,10 @@ av1g_status av1g_engine_get_stats(av1g_engine* E, av1g_engine_stats* o) {
     return AV1G_OK;
 }
 
-av1g_status av1g_test_engine_faults(av1g_engine* E, int32_t outputs) {
+av1g_status av1g_test_engine_faults(av1g_engine* E, int32_t outputs, int32_t copies) {
     if (!E) return AV1G_EINVAL;
     E->output_faults.store(outputs);
+    E->copy_faults.store(copies);
     return AV1G_OK;
 }
 

@@ -88,7 +88,8 @@ __global__ void __launch_bounds__(kCopyThreads) plane_copy_kernel(const __grid_c
 
 }  // namespace
 
-cudaError_t launch_plane_copies(const PlaneCopy* copies, int n, cudaStream_t s) {
+cudaError_t launch_plane_copies(const PlaneCopy* copies, int n, cudaStream_t s, int* done) {
+    *done = 0;
     for (int i = 0; i < n;) {
         Chunk C;
         int blocks = 0;
@@ -99,10 +100,12 @@ cudaError_t launch_plane_copies(const PlaneCopy* copies, int n, cudaStream_t s) 
             C.first[C.n++] = blocks;
             blocks += (units(copies[i]) + kCopyThreads * kUnits - 1) / (kCopyThreads * kUnits);
         }
-        if (!blocks) continue;
-        plane_copy_kernel<<<blocks, kCopyThreads, 0, s>>>(C);
-        const cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
+        if (blocks) {
+            plane_copy_kernel<<<blocks, kCopyThreads, 0, s>>>(C);
+            const cudaError_t e = cudaGetLastError();
+            if (e != cudaSuccess) return e;
+        }
+        *done = i;
     }
     return cudaSuccess;
 }
