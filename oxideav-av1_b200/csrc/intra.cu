@@ -128,7 +128,8 @@ enum : uint8_t {  // TuHead::where
     W_COPY = 1,      // every edge sample lies in the superblock's copy
     W_DIRECT = 2,    // and the prediction reads both edges there, in place
     W_CFL = 4,       // CfL's luma lies in the copy, in aligned pairs
-    W_ALIGNED = 8,   // x is a multiple of four
+    W_ALIGNED = 8,   // x and the plane's width are multiples of four: a group of four samples
+                     // lies wholly inside or outside the plane
     W_FAST = 16      // a small TU that fast_decode / fast_run take
 };
 
@@ -314,7 +315,7 @@ __device__ void prep_tu(const IntraFrame& F, int log2sb, const av1g_intra_tu& t,
     r.dims = (uint8_t)((31 - __clz(W)) | (31 - __clz(H)) << 4);
     r.plane = t.plane;
     r.res = t.res.coeff_offset;
-    if (!(sx & 3)) r.where |= W_ALIGNED;
+    if (!(sx & 3) && !(F.planes[pl].w & 3)) r.where |= W_ALIGNED;
     if (t.flags & AV1G_INTRA_RESIDUAL) r.bits |= R_RES;
     if ((t.flags & AV1G_INTRA_CFL) && pl > 0) {
         r.bits |= R_CFL;
@@ -1253,8 +1254,7 @@ __device__ __forceinline__ void run_tu(const G& g, S& s, const TuRec* rec, const
                 if (pl == 0 || (row_in && j + e < wlim)) v[e] = min(max(v[e] + r[e], 0), maxv);
         }
         // the final samples to the copy and to HBM: other superblocks read
-        // them once this level is published.  Plane widths are multiples of
-        // four, so an aligned group lies wholly inside or outside the plane.
+        // them once this level is published.
         uint8_t* out = dst + (size_t)i * P.stride + (j << hbd);
         if (t.where & W_ALIGNED) {
             const uint2 pk = make_uint2((uint32_t)v[0] | (uint32_t)v[1] << 16, (uint32_t)v[2] | (uint32_t)v[3] << 16);
@@ -1295,14 +1295,16 @@ __device__ __forceinline__ uint2 ld_quad(const uint8_t* row, int hbd, int x) {
     return make_uint2(__byte_perm(u, 0u, 0x4140), __byte_perm(u, 0u, 0x4342));
 }
 
-// HBM -> the superblock's area of the copy, four samples per thread (plane
-// widths, superblock origins and row pitches are multiples of four samples).
+// HBM -> the superblock's area of the copy, four samples per thread (superblock
+// origins and row pitches are multiples of four samples).  Subsampled planes of an odd
+// number of mode info columns end half a group short: the group's rest is row
+// padding, which nothing reads from the copy.
 __device__ void load_area(const IntraFrame& F, const SbCtx& c, uint16_t* cache) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int p = 0; p < F.np; p++) {
         const PlaneDev& P = F.planes[p];
         const int4 r = c.rect[p];
-        const int rows = min(r.w, P.h - r.y), quads = min(r.z, P.w - r.x) >> 2;
+        const int rows = min(r.w, P.h - r.y), quads = (min(r.z, P.w - r.x) + 3) >> 2;
         uint16_t* cp = cache + c.off[p];
         for (int k = warp; k < rows; k += kIT / 32) {
             const uint8_t* row = P.p + (size_t)(r.y + k) * P.stride;
