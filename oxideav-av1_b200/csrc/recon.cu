@@ -107,16 +107,19 @@ av1g_status recon_run(const av1g_recon_job* jobs, int n, cudaStream_t s, std::st
         uint32_t at[kKeys];
     };
     std::vector<Run> runs;
+    av1g_status bad_frame = AV1G_OK;
     for (int i = 0; i < n; i++) {
         const av1g_recon_job& j = jobs[i];
         if (!j.hdr || !j.quant || (j.num_tus > 0 && (!j.tus || !j.coeffs)) || j.num_tus < 0) {
             err = "recon job " + std::to_string(i) + ": missing header, quantizer state, TU list or coefficients";
-            return AV1G_EINVAL;
+            bad_frame = AV1G_EINVAL;
+            break;
         }
         const av1g_frame_header& h = *j.hdr;
         if (h.bit_depth != 8 && h.bit_depth != 10 && h.bit_depth != 12) {
             err = "recon job " + std::to_string(i) + ": bit depth";
-            return AV1G_EINVAL;
+            bad_frame = AV1G_EINVAL;
+            break;
         }
         ReconFrame& F = frames[i];
         memset(&F, 0, sizeof F);
@@ -130,10 +133,12 @@ av1g_status recon_run(const av1g_recon_job* jobs, int n, cudaStream_t s, std::st
             const av1g_plane& pl = j.planes[p];
             if (!pl.data || pl.width < pw || pl.height < ph || pl.stride < pw * (F.hbd ? 2 : 1) || (pl.stride & 15)) {
                 err = "recon job " + std::to_string(i) + ": plane " + std::to_string(p);
-                return AV1G_EINVAL;
+                bad_frame = AV1G_EINVAL;
+                break;
             }
             F.planes[p] = PlaneDev{(uint8_t*)pl.data, pl.stride, pw, ph};
         }
+        if (bad_frame != AV1G_OK) break;
         const int parts = parallel_parts(j.num_tus, 4096);
         for (int u = 0; u < parts; u++)
             runs.push_back(Run{i, (int)((long long)j.num_tus * u / parts), (int)((long long)j.num_tus * (u + 1) / parts),
@@ -151,12 +156,14 @@ av1g_status recon_run(const av1g_recon_job* jobs, int n, cudaStream_t s, std::st
             r.at[t.tx_size * 16 + t.tx_type]++;
         }
     });
+    // the first bad TU in call order, then a bad frame's error (its job comes after the runs)
     for (const Run& r : runs)
         if (r.bad >= 0) {
             err = "recon job " + std::to_string(r.job) + ": TU " + std::to_string(r.bad) +
                   " has an invalid size/type/plane";
             return AV1G_EINVAL;
         }
+    if (bad_frame != AV1G_OK) return bad_frame;
     if (total == 0) return AV1G_OK;
     // count[key]: TUs with a smaller key; a run's at[key]: where its own go
     for (int k = 0; k < kKeys; k++) {
