@@ -8,12 +8,15 @@
 // prepares on its calling threads.
 #include "host_pool.h"
 
+#ifdef __SSE2__
 #include <emmintrin.h>
+#endif
 #include <unistd.h>
 
 #include <algorithm>
 #include <atomic>
 #include <condition_variable>
+#include <cstdint>
 #include <exception>
 #include <mutex>
 #include <thread>
@@ -126,6 +129,7 @@ void parallel_for(int n, long long items, const std::function<void(int)>& fn) {
 }
 
 void write_back(void* p, size_t n) {
+#ifdef __SSE2__
     constexpr uintptr_t kLine = 64;
     const uintptr_t a = ((uintptr_t)p + kLine - 1) & ~(kLine - 1), b = ((uintptr_t)p + n) & ~(kLine - 1);
     for (uintptr_t q = a; q < b; q += 16) {
@@ -133,6 +137,9 @@ void write_back(void* p, size_t n) {
         _mm_stream_si128(w, _mm_load_si128(w));
     }
     _mm_sfence();
+#else
+    (void)p, (void)n;
+#endif
 }
 
 }  // namespace av1g

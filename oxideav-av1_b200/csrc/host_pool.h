@@ -2,6 +2,7 @@
 // (validation, dependency analysis, record building) with the calling thread.
 #pragma once
 
+#include <cstddef>
 #include <functional>
 
 namespace av1g {
@@ -20,7 +21,8 @@ int parallel_parts(long long items, long long grain);
 // Sends the whole cache lines of [p, p + n), which the caller has just written and
 // nobody else touches, to memory.  A part of an upload that stays in its thread's
 // cache is fetched from there by the copy engine: 6 MB written by eight threads took 696 us
-// to copy to the device, against 128 us when one thread had written them.
+// to copy to the device, against 128 us when one thread had written them.  Does
+// nothing on hosts without SSE2: only the copy's time depends on it.
 void write_back(void* p, size_t n);
 
 }  // namespace av1g
