@@ -85,6 +85,8 @@ __device__ __forceinline__ int floor_log2u(unsigned x) { return x ? 31 - __clz(x
 // The device's default pool keeps up to kWorkspaceKeep bytes of what is freed.
 constexpr unsigned long long kWorkspaceKeep = 256ull << 20;
 cudaError_t workspace_alloc(uint8_t** p, size_t n, cudaStream_t s);
+// Sets the release threshold of a device's default pool; without `replace` only one that is 0.
+void keep_pool_memory(int device, uint64_t keep, bool replace);
 
 // Enqueues a host-to-device copy of n bytes through a pinned staging block
 // (returns once enqueued; the host bytes may be reused immediately).

@@ -891,11 +891,7 @@ av1g_status av1g_engine_create(const av1g_config* cfg, av1g_engine** out) {
         E->lanes.push_back(std::move(L));
     }
     // keep freed stream-ordered memory in the pool between steps
-    cudaMemPool_t pool;
-    if (cudaDeviceGetDefaultMemPool(&pool, E->device) == cudaSuccess) {
-        uint64_t thr = E->budget;
-        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
-    }
+    keep_pool_memory(E->device, E->budget, true);
     for (auto& L : E->lanes) L->thread = std::thread(worker_loop, E, L.get());
     E->completer = std::thread(completer_loop, E);
     *out = E;

@@ -66,27 +66,36 @@ cudaError_t reap() {
 
 }  // namespace
 
+// The one place that sets the release threshold of a device's default pool, which the
+// whole process shares: to `keep` if it is 0, or in any case (`replace`).  The mutex
+// keeps a call that has read 0 from undoing what an engine sets meanwhile.
+void keep_pool_memory(int device, uint64_t keep, bool replace) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    cudaMemPool_t pool;
+    uint64_t now = 0;
+    if (cudaDeviceGetDefaultMemPool(&pool, device) != cudaSuccess) return;
+    if (!replace && (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &now) != cudaSuccess || now != 0)) return;
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+}
+
 // cudaMallocAsync with a pool that keeps its memory.  The default pool's
 // release threshold is 0, so whenever the caller synchronises it unmaps all that
 // is free, and the next call maps it again: 0.3 to 3 ms of host time per
 // allocation, paid by every entry point that synchronises (and by
-// every caller that waits for a result).  The threshold is raised once per device, to a
+// every caller that waits for a result).  The first call on a device raises it, to a
 // bound that holds a 4K key frame's workspace, and only where it is still 0: one
-// that the application or a serving engine has set stands.  The pool is the
-// device's own, so the application can trim it (cudaMemPoolTrimTo).
+// that the application or a serving engine has set stands.  An application that wants
+// the memory unmapped says so with a threshold of 1 byte before its first call (an
+// explicit 0 cannot be told from the default), or with any value after it; it can
+// trim the pool at any time (cudaMemPoolTrimTo).
 cudaError_t workspace_alloc(uint8_t** p, size_t n, cudaStream_t s) {
     static std::atomic<bool> seen[64];
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
     if (device < 64 && !seen[device].load(std::memory_order_acquire)) {
-        cudaMemPool_t pool;
-        uint64_t keep = 0;
-        if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess &&
-            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess && keep == 0) {
-            keep = kWorkspaceKeep;
-            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        }
+        keep_pool_memory(device, kWorkspaceKeep, false);
         seen[device].store(true, std::memory_order_release);
     }
     return cudaMallocAsync(reinterpret_cast<void**>(p), n, s);
