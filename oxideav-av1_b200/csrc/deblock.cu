@@ -19,7 +19,8 @@
 //
 // A thread filters two lines at a time, the halves of a word, in
 // half-precision differences and 16-bit sums that are exact for 8 and 10 bits
-// (12-bit lines go one by one); both passes read two lines' samples as pairs of
+// (12-bit lines go one by one, and so do the lines of a 10-bit tile with a sample above
+// 1023, which a valid stream does not have); both passes read two lines' samples as pairs of
 // words without bank conflicts.  Bound by issue, and by warps whose edges take
 // different filters: 713 us for 64 1080p 8-bit frames and 119 us for four 3840x2160
 // 10-bit ones with a line per thread, every thread deriving its tile and a pass that
@@ -277,19 +278,19 @@ __device__ __forceinline__ int f4clamp(int v, int bd) { return clip3(-(1 << (bd 
 
 // wide_filter (loop_filter.rs:789-822) for one (n, log2Size) case: outputs
 // i in [-n, n) from taps j in [-n, n] weighted 2 for |j| <= n2 else 1, source
-// positions clamped to [-(n + 1), n].  Two lines at a time, one per half of a word:
-// no sum passes 16 bits (16 times 4095, plus the rounding).
-template <int N, int LOG2, int N2>
+// positions clamped to [-(n + 1), n].  PAIR: two lines at a time, one per half of a
+// word: at 10 bits no sum passes 16 bits (16 times 1023, plus the rounding).
+template <bool PAIR, int N, int LOG2, int N2>
 __device__ __forceinline__ void wide(const uint32_t (&v)[2 * N + 2], uint32_t (&o)[2 * N]) {
     auto at = [&](int k) { return v[(k < -(N + 1) ? -(N + 1) : (k > N ? N : k)) + N + 1]; };
-    uint32_t box = (1u << (LOG2 - 1)) * 0x10001u;
+    uint32_t box = (1u << (LOG2 - 1)) * (PAIR ? 0x10001u : 1u);
 #pragma unroll
     for (int j = -N; j <= N; j++) box += at(j - N);
 #pragma unroll
     for (int i = -N; i < N; i++) {
         uint32_t t = box + at(i);
         if (N2) t += at(i - 1) + at(i + 1);
-        o[i + N] = (t >> LOG2) & 0x0fff0fffu;
+        o[i + N] = PAIR ? (t >> LOG2) & 0x0fff0fffu : t >> LOG2;
         box += at(i + N + 1) - at(i - N);
     }
 }
@@ -348,7 +349,7 @@ __device__ __noinline__ void filter_wide(uint32_t* m, uint32_t on) {
     uint32_t x[14], o[12];
 #pragma unroll
     for (int k = 0; k < 14; k++) x[k] = v[k + 1] & kSample;
-    wide<6, 4, 1>(x, o);
+    wide<true, 6, 4, 1>(x, o);
 #pragma unroll
     for (int j = 0; j < 6; j++)
         st_pair<VERT>(m, j - 3, pick(on, o[2 * j] | kBias, v[2 * j + 2]), pick(on, o[2 * j + 1] | kBias, v[2 * j + 3]));
@@ -366,12 +367,12 @@ __device__ __noinline__ void filter_flat(uint32_t* m, uint32_t on, int plane) {
     if (plane) {
         const uint32_t y[6] = {x[1], x[2], x[3], x[4], x[5], x[6]};
         uint32_t o[4];
-        wide<2, 3, 1>(y, o);
+        wide<true, 2, 3, 1>(y, o);
 #pragma unroll
         for (int k = 0; k < 4; k++) v[k + 2] = pick(on, o[k] | kBias, v[k + 2]);
     } else {
         uint32_t o[6];
-        wide<3, 3, 0>(x, o);
+        wide<true, 3, 3, 0>(x, o);
 #pragma unroll
         for (int k = 0; k < 6; k++) v[k + 1] = pick(on, o[k] | kBias, v[k + 1]);
         st_pair<VERT>(m, -2, v[0], v[1]);
@@ -444,11 +445,11 @@ __device__ __forceinline__ void filter_pair(uint32_t* m, int cls, uint2 st, int 
     if (flat) filter_flat<VERT>(m, flat, plane);
 }
 
-// ---- one line at a time, 12 bits (a difference of two 12-bit samples is no half) ----
+// ---- one line at a time, any 16-bit samples: 12 bits (a difference of two 12-bit
+// samples is no half), and 10-bit tiles in which a sample has more than 10 bits ----
 // Line `e` (0 or 1) of a pair; position k counts from q0.
-template <bool VERT>
+template <bool VERT, int bd>
 __device__ void filter_line(uint16_t* b, int e, int cls, uint32_t st, int plane) {
-    constexpr int bd = 12;
     auto at = [&](int k) -> uint16_t& {
         return VERT ? b[2 * kRow * e + k] : b[2 * (kPair * (k >> 1) + kRow * (k & 1)) + e];
     };
@@ -503,13 +504,13 @@ __device__ void filter_line(uint16_t* b, int e, int cls, uint32_t st, int plane)
             const uint32_t v[8] = {(uint32_t)p3, (uint32_t)p2, (uint32_t)p1, (uint32_t)p0,
                                    (uint32_t)q0, (uint32_t)q1, (uint32_t)q2, (uint32_t)q3};
             uint32_t o[6];
-            wide<3, 3, 0>(v, o);
+            wide<false, 3, 3, 0>(v, o);
 #pragma unroll
             for (int i = -3; i < 3; i++) at(i) = (uint16_t)o[i + 3];
         } else {
             const uint32_t v[6] = {(uint32_t)p2, (uint32_t)p1, (uint32_t)p0, (uint32_t)q0, (uint32_t)q1, (uint32_t)q2};
             uint32_t o[4];
-            wide<2, 3, 1>(v, o);
+            wide<false, 2, 3, 1>(v, o);
 #pragma unroll
             for (int i = -2; i < 2; i++) at(i) = (uint16_t)o[i + 2];
         }
@@ -518,17 +519,17 @@ __device__ void filter_line(uint16_t* b, int e, int cls, uint32_t st, int plane)
                                 (uint32_t)p1, (uint32_t)p0, (uint32_t)q0, (uint32_t)q1, (uint32_t)q2,
                                 (uint32_t)q3, (uint32_t)q4, (uint32_t)q5, (uint32_t)q6};
         uint32_t o[12];
-        wide<6, 4, 1>(v, o);
+        wide<false, 6, 4, 1>(v, o);
 #pragma unroll
         for (int i = -6; i < 6; i++) at(i) = (uint16_t)o[i + 6];
     }
 }
 
-template <bool VERT>
-__device__ __noinline__ void filter_lines12(uint32_t* m, int cls, uint32_t st, int plane) {
+template <bool VERT, int BD>
+__device__ __forceinline__ void filter_lines(uint32_t* m, int cls, uint32_t st, int plane) {
     uint16_t* b = reinterpret_cast<uint16_t*>(m);
-    filter_line<VERT>(b, 0, cls, st, plane);
-    filter_line<VERT>(b, 1, cls, st, plane);
+    filter_line<VERT, BD>(b, 0, cls, st, plane);
+    filter_line<VERT, BD>(b, 1, cls, st, plane);
 }
 
 // What the CTA needs of a tile, worked out by one thread while the previous tile
@@ -539,6 +540,7 @@ struct DbTile {
     const uint16_t* codes;
     int src_stride, dst_stride, w, h, dw, dh, x, y;  // (x, y): the tile's first sample
     int plane, hbd, bd, sharp;
+    int lines;  // filtered line by line: 12 bits, or samples of more than ten found while staging
 };
 
 __device__ __noinline__ void plan_tile(const FrameDev* __restrict__ frames, const int32_t* __restrict__ starts, int n,
@@ -556,7 +558,80 @@ __device__ __noinline__ void plan_tile(const FrameDev* __restrict__ frames, cons
     const PlaneDev& S = F.recon[plane];
     const PlaneDev& D = F.deb[plane];
     T = DbTile{S.p, D.p, F.lf_codes[plane], S.stride, D.stride, S.w, S.h, min(D.w, S.w), min(D.h, S.h),
-               tx * TILE, ty * TILE, plane, F.hbd, F.h.bit_depth, F.h.lf_sharpness};
+               tx * TILE, ty * TILE, plane, F.hbd, F.h.bit_depth, F.h.lf_sharpness,
+               F.h.bit_depth == 12};
+}
+
+// Writes the tile, the bits `keep` of its samples, eight per thread (one vector store
+// inside the plane).
+__device__ __forceinline__ void write_tile(const DbTile& T, const uint32_t* __restrict__ win, uint32_t keep) {
+    const int dh = T.dh, dw = T.dw, dst_stride = T.dst_stride, hbd = T.hbd;
+    uint8_t* dst = T.dst;
+#pragma unroll
+    for (int q = 0; q < TILE * TILE / 8 / kDbThreads; q++) {
+        const int i = threadIdx.x + q * kDbThreads, r = i / (TILE / 8), c = i % (TILE / 8);
+        const int gy = T.y + r, gx = T.x + 8 * c;
+        if (gy >= dh) continue;
+        const int wr = r + HALO;
+        const uint32_t* w = win + (wr >> 1) * kPair + (wr & 1) * kRow + HALO / 2 + 4 * c;
+        const uint2 a = *reinterpret_cast<const uint2*>(w), b = *reinterpret_cast<const uint2*>(w + 2);
+        uint8_t* row = dst + (size_t)gy * dst_stride;
+        if (gx + 7 < dw) {
+            if (hbd)
+                *reinterpret_cast<uint4*>(row + 2 * gx) = make_uint4(a.x & keep, a.y & keep, b.x & keep, b.y & keep);
+            else
+                *reinterpret_cast<uint2*>(row + gx) =
+                    make_uint2(__byte_perm(a.x, a.y, 0x6420), __byte_perm(b.x, b.y, 0x6420));
+        } else {
+            const uint32_t v[4] = {a.x & keep, a.y & keep, b.x & keep, b.y & keep};
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                const uint32_t px = (v[e / 2] >> (16 * (e & 1))) & 0xffff;
+                if (gx + e >= dw) continue;
+                if (hbd) reinterpret_cast<uint16_t*>(row)[gx + e] = (uint16_t)px;
+                else row[gx + e] = (uint8_t)px;
+            }
+        }
+    }
+}
+
+// The passes over pairs of window rows (vertical edges) and of tile columns (horizontal
+// ones), edge columns and rows 12..84 (cells 3..21: a filter moves at most 6 samples from
+// its edge, so only those edges move tile samples).
+constexpr int VP = (kRow1 - kRow0) / 2, HP = TILE / 2, EDGES = CELLS - 5;
+
+__device__ __forceinline__ uint2 line_strength(int lvl, int sharp) {
+    const Strength s = strength(lvl, sharp);
+    return make_uint2((uint32_t)s.limit | (uint32_t)s.blimit << 8 | (uint32_t)s.thresh << 16, 0u);
+}
+
+// A staged tile of any 16-bit samples, line by line: 12 bits, and 10-bit tiles with a
+// sample of more than 10 bits, whose bias comes off first.  A call of its own, so that
+// it costs the other tiles no registers: 32 1080p frames take 348 us at 8 bits and 365
+// at 10 (376 and 393 with the choice made at each edge; 346 and 362 with none).
+template <int BD>
+__device__ __noinline__ void filter_tile_by_lines(const DbTile& T, uint32_t* win, const uint16_t* code, uint2* strengths) {
+    if (BD != 12) {
+        for (int i = threadIdx.x; i < (kRow1 - kRow0) * kRow; i += kDbThreads) {
+            const int r = kRow0 + i / kRow;
+            win[(r >> 1) * kPair + (r & 1) * kRow + i % kRow] -= kBias;
+        }
+        if (threadIdx.x < 64) strengths[threadIdx.x] = line_strength(threadIdx.x, T.sharp);
+        __syncthreads();
+    }
+    for (int i = threadIdx.x; i < VP * EDGES; i += kDbThreads) {
+        const int e = i / VP, r = kRow0 / 2 + i - e * VP, cc = 3 + e;
+        const int c = code[(r >> 1) * CELLS + cc] & 0xff;
+        if (c) filter_lines<true, BD>(win + r * kPair + cc * 2, c >> 6, strengths[c & 63].x, T.plane);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < HP * EDGES; i += kDbThreads) {
+        const int x = HALO / 2 + i % HP, cr = 3 + i / HP;
+        const int c = code[cr * CELLS + (x >> 1)] >> 8;
+        if (c) filter_lines<false, BD>(win + cr * 2 * kPair + x, c >> 6, strengths[c & 63].x, T.plane);
+    }
+    __syncthreads();
+    write_tile(T, win, 0xffffffffu);
 }
 
 constexpr int kDbCtas = 6;
@@ -567,7 +642,7 @@ __global__ void __launch_bounds__(kDbThreads, kDbCtas) deblock_kernel(const Fram
     chain_next();
     __shared__ __align__(16) uint32_t win[WIN / 2 * kPair];
     __shared__ uint16_t code[CELLS * CELLS];
-    __shared__ uint2 strengths[64];  // by level: halves limit, blimit + 1/2, thresh; 12 bits: bytes
+    __shared__ uint2 strengths[64];  // by level: halves limit, blimit + 1/2, thresh; by lines: bytes
     __shared__ DbTile plan[2];
     if (threadIdx.x == 0 && (int)blockIdx.x < total) plan_tile(frames, starts, n, blockIdx.x, plan[0]);
     int k = 0;
@@ -576,7 +651,9 @@ __global__ void __launch_bounds__(kDbThreads, kDbCtas) deblock_kernel(const Fram
         const DbTile& T = plan[k];
         const int hbd = T.hbd, bd = T.bd, plane = T.plane;
         const int gx0 = T.x - HALO, gy0 = T.y - HALO;
+        // added, so that it comes off again whatever the samples are
         const uint32_t bias = bd == 12 ? 0u : kBias;
+        uint32_t seen = 0;  // high bit depths: the bits of the samples staged
         {
             // window: 8 consecutive samples per thread.  A window inside the
             // plane horizontally (almost every tile) issues three loads before it
@@ -603,7 +680,8 @@ __global__ void __launch_bounds__(kDbThreads, kDbCtas) deblock_kernel(const Fram
                         if (i >= ITEMS) continue;
                         uint4 o;
                         if (hbd) {
-                            o = make_uint4(v[q].x | bias, v[q].y | bias, v[q].z | bias, v[q].w | bias);
+                            seen |= (v[q].x | v[q].y) | (v[q].z | v[q].w);
+                            o = make_uint4(v[q].x + bias, v[q].y + bias, v[q].z + bias, v[q].w + bias);
                         } else {
                             o = make_uint4(__byte_perm(v[q].x, kBias, 0x7170), __byte_perm(v[q].x, kBias, 0x7372),
                                            __byte_perm(v[q].y, kBias, 0x7170), __byte_perm(v[q].y, kBias, 0x7372));
@@ -620,7 +698,8 @@ __global__ void __launch_bounds__(kDbThreads, kDbCtas) deblock_kernel(const Fram
                     const int xa = clip3(0, w - 1, gx0 + 2 * c), xb = clip3(0, w - 1, gx0 + 2 * c + 1);
                     const uint32_t a = hbd ? reinterpret_cast<const uint16_t*>(row)[xa] : row[xa];
                     const uint32_t b = hbd ? reinterpret_cast<const uint16_t*>(row)[xb] : row[xb];
-                    win[(r >> 1) * kPair + (r & 1) * kRow + c] = a | b << 16 | bias;
+                    seen |= a | b << 16;
+                    win[(r >> 1) * kPair + (r & 1) * kRow + c] = (a | b << 16) + bias;
                 }
             }
         }
@@ -633,79 +712,50 @@ __global__ void __launch_bounds__(kDbThreads, kDbCtas) deblock_kernel(const Fram
             }
         }
         if (threadIdx.x < 64) {
-            const Strength s = strength(threadIdx.x, T.sharp);
             uint2 e;
             if (bd == 12) {
-                e = make_uint2((uint32_t)s.limit | (uint32_t)s.blimit << 8 | (uint32_t)s.thresh << 16, 0u);
+                e = line_strength(threadIdx.x, T.sharp);
             } else {
+                const Strength s = strength(threadIdx.x, T.sharp);
                 const float scale = bd == 8 ? 1.f : 4.f;
                 const __half2 a = __floats2half2_rn(scale * s.limit, scale * s.blimit + 0.5f);
                 e = make_uint2(u32(a), u32(__float2half2_rn(scale * s.thresh)));
             }
             strengths[threadIdx.x] = e;
         }
+        if (seen & ~kSample) plan[k].lines = 1;
         __syncthreads();
         if (threadIdx.x == kDbThreads - 1 && t + (int)gridDim.x < total)
             plan_tile(frames, starts, n, t + gridDim.x, plan[k ^ 1]);
+        if (T.lines) {
+            if (bd == 12) filter_tile_by_lines<12>(T, win, code, strengths);
+            else filter_tile_by_lines<10>(T, win, code, strengths);
+            continue;
+        }
         HalfConsts K;
         K.one = dup(bd == 8 ? 1.f : 4.f);
         K.lo = dup(bd == 8 ? -128.f : -512.f);
         K.hi = dup(bd == 8 ? 127.f : 511.f);
         K.top = dup(bd == 8 ? 1279.f : 2047.f);
-        // vertical pass: pairs of window rows x edge columns 12..84 (cells 3..21: a
-        // filter moves at most 6 samples from its edge, so only those edges
-        // move tile columns)
-        constexpr int VP = (kRow1 - kRow0) / 2, VE = CELLS - 5;
-        for (int i = threadIdx.x; i < VP * VE; i += kDbThreads) {
+        // vertical pass
+        for (int i = threadIdx.x; i < VP * EDGES; i += kDbThreads) {
             const int e = i / VP, r = kRow0 / 2 + i - e * VP, cc = 3 + e;
             const int c = code[(r >> 1) * CELLS + cc] & 0xff;
             if (!c) continue;
             uint32_t* m = win + r * kPair + cc * 2;
-            if (bd == 12) filter_lines12<true>(m, c >> 6, strengths[c & 63].x, plane);
-            else filter_pair<true>(m, c >> 6, strengths[c & 63], plane, K);
+            filter_pair<true>(m, c >> 6, strengths[c & 63], plane, K);
         }
         __syncthreads();
-        // horizontal pass: pairs of tile columns x edge rows 12..84
-        constexpr int HP = TILE / 2, HE = CELLS - 5;  // cells 3..21
-        for (int i = threadIdx.x; i < HP * HE; i += kDbThreads) {
+        // horizontal pass
+        for (int i = threadIdx.x; i < HP * EDGES; i += kDbThreads) {
             const int x = HALO / 2 + i % HP, cr = 3 + i / HP;
             const int c = code[cr * CELLS + (x >> 1)] >> 8;
             if (!c) continue;
             uint32_t* m = win + cr * 2 * kPair + x;
-            if (bd == 12) filter_lines12<false>(m, c >> 6, strengths[c & 63].x, plane);
-            else filter_pair<false>(m, c >> 6, strengths[c & 63], plane, K);
+            filter_pair<false>(m, c >> 6, strengths[c & 63], plane, K);
         }
         __syncthreads();
-        // write the tile, eight samples per thread (one vector store inside the plane)
-        const int dh = T.dh, dw = T.dw, dst_stride = T.dst_stride;
-        uint8_t* dst = T.dst;
-#pragma unroll
-        for (int q = 0; q < TILE * TILE / 8 / kDbThreads; q++) {
-            const int i = threadIdx.x + q * kDbThreads, r = i / (TILE / 8), c = i % (TILE / 8);
-            const int gy = T.y + r, gx = T.x + 8 * c;
-            if (gy >= dh) continue;
-            const int wr = r + HALO;
-            const uint32_t* w = win + (wr >> 1) * kPair + (wr & 1) * kRow + HALO / 2 + 4 * c;
-            const uint2 a = *reinterpret_cast<const uint2*>(w), b = *reinterpret_cast<const uint2*>(w + 2);
-            uint8_t* row = dst + (size_t)gy * dst_stride;
-            const uint32_t keep = bd == 12 ? 0xffffffffu : kSample;
-            if (gx + 7 < dw) {
-                if (hbd)
-                    *reinterpret_cast<uint4*>(row + 2 * gx) = make_uint4(a.x & keep, a.y & keep, b.x & keep, b.y & keep);
-                else
-                    *reinterpret_cast<uint2*>(row + gx) =
-                        make_uint2(__byte_perm(a.x, a.y, 0x6420), __byte_perm(b.x, b.y, 0x6420));
-            } else {
-                const uint32_t v[4] = {a.x & keep, a.y & keep, b.x & keep, b.y & keep};
-#pragma unroll
-                for (int e = 0; e < 8; e++) {
-                    const uint32_t px = (v[e / 2] >> (16 * (e & 1))) & 0xffff;
-                    if (gx + e >= dw) continue;
-                    if (hbd) reinterpret_cast<uint16_t*>(row)[gx + e] = (uint16_t)px;
-                    else row[gx + e] = (uint8_t)px;
-                }
-            }
-        }
+        write_tile(T, win, kSample);
     }
 }
 

@@ -1,0 +1,51 @@
+"""Deblocking of 16-bit planes whose samples have more bits than the frame's
+depth: the filter's arithmetic is defined for them all the same, tile by tile.  Against the oracle, no tolerance."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+import oracle  # noqa: E402
+from oxideav_av1_b200 import postfilter, synth  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+FORMATS = [dict(bit_depth=10), dict(bit_depth=10, ssx=0, ssy=0), dict(bit_depth=12)]
+IDS = ["10", "10-444", "12"]
+
+
+def _raise(f, seed, most):
+    """Lifts a few areas of each plane, their shape kept, and single samples, to values up to `most`."""
+    rng = np.random.default_rng(seed)
+    for p, a in enumerate(f.recon):
+        v = a.astype(np.int64)
+        h, w = v.shape
+        for k in range(3):
+            y, x = int(rng.integers(0, h)), int(rng.integers(0, w))
+            v[y:y + 24, x:x + 40] += int(rng.integers(1, most - int(v.max())))
+        v = np.minimum(v, most)
+        v[int(rng.integers(0, h)), int(rng.integers(0, w))] = most
+        f.recon[p] = v.astype(np.uint16)
+
+
+def _run(f):
+    d = postfilter.DeviceFrame(f)
+    postfilter.run_postfilter([d])
+    torch.cuda.synchronize()
+    return d
+
+
+def _same(got, exp):
+    for p, (g, e) in enumerate(zip(got, exp)):
+        bad = np.argwhere(g.astype(np.int64) != e)
+        assert len(bad) == 0, f"plane {p}: {len(bad)} samples differ, first at {tuple(bad[0])}"
+
+
+@pytest.mark.parametrize("fmt", FORMATS, ids=IDS)
+@pytest.mark.parametrize("most", [1024 + 200, 65535])
+def test_deblock(fmt, most):
+    f = synth.make_frame(seed=901, width=328, height=200, cdef=False, lr=False, **fmt)
+    f.hdr.lf_level[2], f.hdr.lf_level[3] = 40, 50
+    if most > 1 << fmt["bit_depth"]:
+        _raise(f, 7, most)
+    _same(_run(f).download("deblocked"), oracle.loop_filter(f, [r.astype(np.int32) for r in f.recon]))
