@@ -83,14 +83,15 @@ __constant__ SgrSets c_sgr = make_sgr();
 struct Tile {
     int frame, plane, x0, y0, tw, th, sstart, send, pw, ph;
     av1g_lr_unit u;
+    int packed;  // a and b share a word: not at 12 bits, nor with samples of more than ten
 };
 
 struct Smem {
     uint16_t src[SH * SP];
     int v1[AR * VW];      // column sums; the Wiener intermediate reuses v1/v2
     int v2[AR * VW];
-    uint32_t AB[AR * AP];  // b << kABits | a; 12 bits: b alone
-    uint16_t A[AR * AP];   // 12 bits: a
+    uint32_t AB[AR * AP];  // packed: b << kABits | a; else b alone
+    uint16_t A[AR * AP];   // not packed: a
     uint16_t a2lut[256];
     Tile tile[2];  // the current one, and the next one while it is worked out
 };
@@ -118,7 +119,8 @@ __device__ __forceinline__ int count_units(int us, int sz) {
 
 // At 8 and 10 bits the coefficients a (at most 256) and b (at most 261,120) share a
 // word, and the sums of up to five of them that the 3x3 weighting needs do too
-// (1,280 below 2^11, 1,305,600 below 2^21).
+// (1,280 below 2^11, 1,305,600 below 2^21).  Not packed: 12 bits, and 10-bit tiles in
+// whose window a sample has more than 10 bits.
 constexpr int kABits = 11;
 constexpr uint32_t kAMask = (1u << kABits) - 1;
 
@@ -130,7 +132,7 @@ constexpr uint32_t kAMask = (1u << kABits) - 1;
 // the rows and row sums slide along the columns, so each sum costs two loads
 // instead of 2R + 1; the runs have fixed lengths so the loops unroll and the
 // coefficient arithmetic of neighbouring positions overlaps.
-template <int R, int BD>
+template <int R, int BD, bool PACK>
 __device__ void box_coeffs(Smem& s, int th, int tw, const SgrPass& ps, int y0) {
     constexpr bool ODD = R == 2;
     constexpr int n = (2 * R + 1) * (2 * R + 1);
@@ -212,8 +214,8 @@ __device__ void box_coeffs(Smem& s, int th, int tw, const SgrPass& ps, int y0) {
             // stays below 2^32 at every bit depth (b <= 25 * 4095)
             const unsigned b2 = (unsigned)(256 - a2) * (unsigned)b * (unsigned)one_over_n;
             const uint32_t bq = (b2 + (1u << 11)) >> 12;
-            if (BD == 12) ao[t] = (uint16_t)a2;
-            bo[t] = BD == 12 ? bq : (bq << kABits | (uint32_t)a2);
+            if (!PACK) ao[t] = (uint16_t)a2;
+            bo[t] = PACK ? (bq << kABits | (uint32_t)a2) : bq;
             b += c1[t + 2 * R + 1] - c1[t];
             a += c2[t + 2 * R + 1] - c2[t];
         }
@@ -265,9 +267,9 @@ __device__ __forceinline__ void weight_pair(const Smem& s, int i, int j0, const 
     }
 }
 
-// The same at 12 bits, one row at a time from the two arrays.
+// The same from the two arrays, one row at a time.
 template <int PASS>
-__device__ __noinline__ int4 weight_row12(const Smem& s, int i, int j0, int4 uq) {
+__device__ __noinline__ int4 weight_row(const Smem& s, int i, int j0, int4 uq) {
     const uint16_t* a = s.A + i * AP + j0;
     const uint32_t* b = s.AB + i * AP + j0;
     const bool odd = i & 1;
@@ -291,11 +293,11 @@ __device__ __noinline__ int4 weight_row12(const Smem& s, int i, int j0, int4 uq)
     return make_int4(out[0], out[1], out[2], out[3]);
 }
 template <int PASS>
-__device__ __forceinline__ void weight_pair(const Smem& s, int bd, int i, int j0, const int (&u)[2][4], int (&out)[2][4]) {
-    if (bd == 12) {
+__device__ __forceinline__ void weight_pair(const Smem& s, bool packed, int i, int j0, const int (&u)[2][4], int (&out)[2][4]) {
+    if (!packed) {
 #pragma unroll
         for (int e = 0; e < 2; e++) {
-            const int4 v = weight_row12<PASS>(s, i + e, j0, make_int4(u[e][0], u[e][1], u[e][2], u[e][3]));
+            const int4 v = weight_row<PASS>(s, i + e, j0, make_int4(u[e][0], u[e][1], u[e][2], u[e][3]));
             out[e][0] = v.x, out[e][1] = v.y, out[e][2] = v.z, out[e][3] = v.w;
         }
     } else {
@@ -303,10 +305,11 @@ __device__ __forceinline__ void weight_pair(const Smem& s, int bd, int i, int j0
     }
 }
 template <int R>
-__device__ __forceinline__ void box_coeffs(Smem& s, int th, int tw, int bd, const SgrPass& ps, int y0) {
-    if (bd == 8) box_coeffs<R, 8>(s, th, tw, ps, y0);
-    else if (bd == 10) box_coeffs<R, 10>(s, th, tw, ps, y0);
-    else box_coeffs<R, 12>(s, th, tw, ps, y0);
+__device__ __forceinline__ void box_coeffs(Smem& s, int th, int tw, int bd, bool packed, const SgrPass& ps, int y0) {
+    if (bd == 8) box_coeffs<R, 8, true>(s, th, tw, ps, y0);
+    else if (bd == 12) box_coeffs<R, 12, false>(s, th, tw, ps, y0);
+    else if (packed) box_coeffs<R, 10, true>(s, th, tw, ps, y0);
+    else box_coeffs<R, 10, false>(s, th, tw, ps, y0);
 }
 
 // Tile t of the batch: its frame, plane, stripe half, column tile and
@@ -344,7 +347,7 @@ __device__ void plan_tile(Tile& T, const FrameDev* __restrict__ frames, const in
     av1g_lr_unit u{};
     if (F.lr_units[plane] && ur < F.lr_unit_rows[plane] && uc < F.lr_unit_cols[plane])
         u = F.lr_units[plane][ur * F.lr_unit_cols[plane] + uc];
-    T = Tile{f, plane, x0, y0, min(x0 + tw, pw) - x0, y1 - y0, sstart, send, pw, ph, u};
+    T = Tile{f, plane, x0, y0, min(x0 + tw, pw) - x0, y1 - y0, sstart, send, pw, ph, u, h.bit_depth != 12};
 }
 
 __global__ void __launch_bounds__(kLrThreads, 4) lr_kernel(const FrameDev* __restrict__ frames,
@@ -394,6 +397,7 @@ __global__ void __launch_bounds__(kLrThreads, 4) lr_kernel(const FrameDev* __res
         }
         // source window: get_source_sample (loop_restoration.rs:862-883)
         const int sw = tw + 2 * H3;
+        uint32_t seen = 0;  // high bit depths: the bits of the samples staged
         if (x0 >= 4 && x0 + tw + 4 <= pw && !(x0 & 3) && !(tw & 3)) {
             // columns [x0 - 4, x0 + tw + 4) lie inside the plane (and inside
             // both source planes, which are at least pw wide): aligned
@@ -435,6 +439,7 @@ __global__ void __launch_bounds__(kLrThreads, 4) lr_kernel(const FrameDev* __res
                 const int i = (int)(((unsigned)k * mag) >> 16), g = k - i * ng;
                 int v[4];
                 if (hbd) {
+                    seen |= q[e].x | q[e].y;
                     v[0] = q[e].x & 0xffff;
                     v[1] = q[e].x >> 16;
                     v[2] = q[e].y & 0xffff;
@@ -460,10 +465,13 @@ __global__ void __launch_bounds__(kLrThreads, 4) lr_kernel(const FrameDev* __res
                 if (y < sstart) v = ld_px(Dq, hbd, clip3(0, Dq.h - 1, max(y, sstart - 2)), min(x, Dq.w - 1));
                 else if (y > send) v = ld_px(Dq, hbd, clip3(0, Dq.h - 1, min(y, send + 2)), min(x, Dq.w - 1));
                 else v = ld_px(C, hbd, min(y, C.h - 1), min(x, C.w - 1));
+                seen |= (uint32_t)v;
                 s.src[i * SP + j] = (uint16_t)v;
             }
         }
+        if (seen & 0xfc00fc00u) s.tile[cur].packed = 0;
         __syncthreads();
+        const bool packed = T.packed;
         const int maxv = (1 << bd) - 1;
         if (u.type == 1) {
             int hf[7], vf[7];
@@ -553,18 +561,18 @@ __global__ void __launch_bounds__(kLrThreads, 4) lr_kernel(const FrameDev* __res
                 for (int q = 0; q < 4; q++) uq[e][q] = s.src[(i0 + e + H3) * SP + j0 + q + H3];
         };
         if (r0) {  // r0 is 2 in every set that has it
-            box_coeffs<2>(s, th, tw, bd, p0, y0);
+            box_coeffs<2>(s, th, tw, bd, packed, p0, y0);
             if (mine) {
                 load_u();
-                weight_pair<0>(s, bd, i0, j0, uq, f0);
+                weight_pair<0>(s, packed, i0, j0, uq, f0);
             }
             __syncthreads();
         }
-        if (r1) box_coeffs<1>(s, th, tw, bd, p1, y0);  // r1 is 1 in every set that has it
+        if (r1) box_coeffs<1>(s, th, tw, bd, packed, p1, y0);  // r1 is 1 in every set that has it
         if (!mine) continue;
         int f1[2][4];
         load_u();
-        if (r1) weight_pair<1>(s, bd, i0, j0, uq, f1);
+        if (r1) weight_pair<1>(s, packed, i0, j0, uq, f1);
 #pragma unroll
         for (int e = 0; e < 2; e++) {
             const int i = i0 + e;

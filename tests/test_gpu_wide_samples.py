@@ -1,5 +1,6 @@
-"""Deblocking of 16-bit planes whose samples have more bits than the frame's
-depth: the filter's arithmetic is defined for them all the same, tile by tile.  Against the oracle, no tolerance."""
+"""Deblocking and loop restoration of 16-bit planes whose samples have
+more bits than the frame's depth: the filters' arithmetic is defined for them all
+the same, tile by tile.  Against the oracle, no tolerance."""
 import numpy as np
 import pytest
 
@@ -49,3 +50,16 @@ def test_deblock(fmt, most):
     if most > 1 << fmt["bit_depth"]:
         _raise(f, 7, most)
     _same(_run(f).download("deblocked"), oracle.loop_filter(f, [r.astype(np.int32) for r in f.recon]))
+
+
+# at 10 bits up to 12: beyond, the box sums' products pass 32 bits
+@pytest.mark.parametrize("fmt", FORMATS[:2], ids=IDS[:2])
+@pytest.mark.parametrize("unit", [1, 2])
+def test_loop_restoration(fmt, unit):
+    f = synth.make_frame(seed=902, width=328, height=200, deblock=False, cdef=False, lr_types=(unit,) * 3, **fmt)
+    for u in f.lr_units:
+        u["type"] = unit
+    _raise(f, 8, 4095)
+    src = [r.astype(np.int32) for r in f.recon]
+    exp = oracle.loop_restoration(f, src, src)
+    _same(_run(f).download("lr"), [e[: f.out_dims(p)[0], : f.out_dims(p)[1]] for p, e in enumerate(exp)])
