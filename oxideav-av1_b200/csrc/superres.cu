@@ -137,19 +137,33 @@ __device__ __forceinline__ Taps place_taps(uint32_t lo, uint32_t hi, int by) {
                  (int)__funnelshift_lc(hi, 0u, 8 * by)}};
 }
 
+// sum + two products of an unsigned 16-bit sample and a signed byte: the samples of x
+// (low, high half) with the lower (dp_lo) or upper (dp_hi) two bytes of w.  (__dp2a
+// takes both operands' signs alike, and samples may use all 16 bits.)
+__device__ __forceinline__ int dp_lo(int x, int w, int sum) {
+    int d;
+    asm("dp2a.lo.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(x), "r"(w), "r"(sum));
+    return d;
+}
+__device__ __forceinline__ int dp_hi(int x, int w, int sum) {
+    int d;
+    asm("dp2a.hi.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(x), "r"(w), "r"(sum));
+    return d;
+}
+
 // Output J of a quad: its window starts at most J + 1 samples after the quad's first word.
 template <int J>
 __device__ __forceinline__ int dot(const int (&x)[6], const Taps& c, const Taps& m, int maxv) {
-    int sum = __dp2a_hi(x[1], m.w[0], 64);  // round2 by 7 bits
-    sum = __dp2a_lo(x[2], m.w[1], sum);
-    if (J >= 1) sum = __dp2a_hi(x[3], m.w[1], sum);
-    if (J >= 3) sum = __dp2a_lo(x[4], m.w[2], sum);
-    sum = __dp2a_lo(x[0], c.w[0], sum);
-    sum = __dp2a_hi(x[1], c.w[0], sum);
-    sum = __dp2a_lo(x[2], c.w[1], sum);
-    sum = __dp2a_hi(x[3], c.w[1], sum);
-    sum = __dp2a_lo(x[4], c.w[2], sum);
-    if (J >= 2) sum = __dp2a_hi(x[5], c.w[2], sum);
+    int sum = dp_hi(x[1], m.w[0], 64);  // round2 by 7 bits
+    sum = dp_lo(x[2], m.w[1], sum);
+    if (J >= 1) sum = dp_hi(x[3], m.w[1], sum);
+    if (J >= 3) sum = dp_lo(x[4], m.w[2], sum);
+    sum = dp_lo(x[0], c.w[0], sum);
+    sum = dp_hi(x[1], c.w[0], sum);
+    sum = dp_lo(x[2], c.w[1], sum);
+    sum = dp_hi(x[3], c.w[1], sum);
+    sum = dp_lo(x[4], c.w[2], sum);
+    if (J >= 2) sum = dp_hi(x[5], c.w[2], sum);
     return __vimin_s32_relu(sum >> 7, maxv);
 }
 

@@ -1,4 +1,4 @@
-"""Deblocking and loop restoration of 16-bit planes whose samples have
+"""Deblocking, loop restoration and superres of 16-bit planes whose samples have
 more bits than the frame's depth: the filters' arithmetic is defined for them all
 the same, tile by tile.  Against the oracle, no tolerance."""
 import numpy as np
@@ -63,3 +63,11 @@ def test_loop_restoration(fmt, unit):
     src = [r.astype(np.int32) for r in f.recon]
     exp = oracle.loop_restoration(f, src, src)
     _same(_run(f).download("lr"), [e[: f.out_dims(p)[0], : f.out_dims(p)[1]] for p, e in enumerate(exp)])
+
+
+@pytest.mark.parametrize("fmt", FORMATS, ids=IDS)
+def test_superres(fmt):
+    f = synth.make_frame(seed=903, width=600, height=60, superres_denom=13, deblock=False, cdef=False, lr=False, **fmt)
+    _raise(f, 9, 65535)
+    exp = oracle.upscale(f, [r.astype(np.int32) for r in f.recon])
+    _same([p.download() for p in _run(f).stage_planes()["up_cdef"]], exp)
