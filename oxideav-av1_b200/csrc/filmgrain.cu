@@ -45,6 +45,7 @@ __device__ const AV1T_GAUSSIAN_SEQUENCE_TYPE g_gauss AV1T_GAUSSIAN_SEQUENCE_DIMS
 namespace {
 
 constexpr int LW = 82, LH = 73;
+constexpr int kSpins = 1 << 22;  // readings of a progress word by one wait, some 30 cycles each
 
 // ---- LFSR jump tables: M^(w * 2^b) for row widths 82 and 44 ---------------
 struct Jumps {
@@ -180,7 +181,9 @@ __device__ void ar_filter(int16_t* C, const int16_t* L, const uint8_t* coef, con
         if (luma) {
             const int need = min(ssy ? 2 * (T + 1) : ssx ? T + 1 + w : T + 1, LW - 1 + 4 * (LH - 1));
             if (seen <= need) {
-                while ((seen = *prog) <= need) {}
+                // the luma warp waits for nothing, so this ends within its few hundred steps; the
+                // bound, a thousand times that, only guards against a broken invariant
+                for (int k = 0; (seen = *prog) <= need && k < kSpins; k++) {}
                 __threadfence_block();
             }
         }

@@ -67,6 +67,10 @@ constexpr int kSmallPx = kIntraSmallPx;
 constexpr int kLvStage = 512;       // level-table entries staged per superblock (more: read from HBM)
 constexpr int kTuStage = 512;       // TU records staged per superblock (more: read from HBM)
 constexpr long long kWaitNs = 2000000000LL;  // the bound of one dependency wait
+// Readings of a shared word by one wait inside a CTA.  The workers wait for the waiting
+// warp, whose own waits are bounded by time, and the publishing warp for the workers: both
+// end well before this many (20 s and more), which mark the frame as a wait that ran out.
+constexpr int kSpins = 1 << 30;
 
 __constant__ AV1T_TX_WIDTH_TYPE c_txw_d AV1T_TX_WIDTH_DIMS = AV1T_TX_WIDTH_INIT;
 __constant__ AV1T_TX_HEIGHT_TYPE c_txh_d AV1T_TX_HEIGHT_DIMS = AV1T_TX_HEIGHT_INIT;
@@ -242,6 +246,7 @@ struct alignas(16) Shared {
     int idx;
     int done;   // levels finished, as far as they are published (workers -> publishing warp)
     int ready;  // levels below this one may run (waiting warp -> workers)
+    int stuck;  // a wait inside the CTA ran out (-> publishing warp)
 };
 static_assert(sizeof(IntraFrame) % 4 == 0, "frame record copied as words");
 constexpr size_t kSharedBytes = (sizeof(Shared) + 15) & ~(size_t)15;
@@ -1529,6 +1534,7 @@ __global__ void __launch_bounds__(kIT, 1) intra_kernel(const IntraFrame* __restr
         }
         if (tid == 3) {
             S.done = 0;
+            S.stuck = 0;
             S.ready = it.nwait > 0 ? __ldg(waits + it.wait_first).x : kNoWait;
         }
         __syncthreads();
@@ -1546,15 +1552,19 @@ __global__ void __launch_bounds__(kIT, 1) intra_kernel(const IntraFrame* __restr
         __syncthreads();
         if (warp == kWW) {
             if (lane == 0)
-                for (int last = 0; last < it.nlv;) {
-                    const int done = *(volatile int*)&S.done;
+                for (int last = 0, spins = 0; last < it.nlv;) {
+                    int done = *(volatile int*)&S.done;
                     if (done == last) {
                         __nanosleep(20);
-                        continue;
+                        if (spins++ < kSpins) continue;
+                        S.stuck = 1;
+                        done = it.nlv;
                     }
+                    if (*(volatile int*)&S.stuck) atomicExch(ctl + 1 + it.frame, 1);
                     __threadfence();
                     atomicExch(prog + idx, done);
                     last = done;
+                    spins = 0;
                 }
             continue;
         }
@@ -1596,7 +1606,9 @@ __global__ void __launch_bounds__(kIT, 1) intra_kernel(const IntraFrame* __restr
             }
             if (lg == it.nlv) break;
             if (ready <= lg) {
-                while ((ready = *(volatile int*)&S.ready) <= lg) {}
+                int k = kSpins;
+                while ((ready = *(volatile int*)&S.ready) <= lg && --k) {}
+                if (!k) S.stuck = 1;
                 __threadfence_block();
             }
             WScr& ws = S.s[grp].w[wi];
