@@ -140,7 +140,7 @@ void launch_lr(const FrameDev* frames, const int32_t* starts, int n, int total, 
 // stage before leave them, and wait there (chain_wait) until it has finished and its
 // writes are visible.  Every kernel launched so calls chain_wait before anything else
 // and chain_next after it, so a stage never runs ahead of more than one other.  One
-// CIF frame's chain takes 45.4 us so against 53.4 us.  Stages of more than two CTAs per SM
+// CIF frame's chain takes 44.4 us so against 52.1 us.  Stages of more than two CTAs per SM
 // are launched plainly: their CTAs hold places that the stage before could use (twelve
 // 718p 4:4:4 frames 733 against 708 us, sixteen 720p ones in an engine 20.3 against 19.5 ms).
 constexpr int kChainBlocks = 2 * kSMs;

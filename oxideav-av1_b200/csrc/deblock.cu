@@ -20,13 +20,11 @@
 // A thread filters two lines at a time, the halves of a word, in
 // half-precision differences and 16-bit sums that are exact for 8 and 10 bits
 // (12-bit lines go one by one, and so do the lines of a 10-bit tile with a sample above
-// 1023, which a valid stream does not have); both passes read two lines' samples as pairs of
-// words without bank conflicts.  Bound by issue, and by warps whose edges take
-// different filters: 713 us for 64 1080p 8-bit frames and 119 us for four 3840x2160
-// 10-bit ones with a line per thread, every thread deriving its tile and a pass that
-// unpacked each cell's strengths; 608 and 101 us with pairs and a planning thread;
-// 540 and 95 us with the filters that few edges take in calls of their own, and 497 and
-// 88 us (1.4 TB/s of planes read and written) at six CTAs per SM.
+// 1023, which a valid stream does not have); both passes read two lines' samples as
+// pairs of words without bank conflicts, and the filters that few edges take are calls
+// of their own.  Bound by issue, and by warps whose edges take different filters: 500 us for 64
+// 1080p 8-bit frames and 89 us for four 3840x2160 10-bit ones (1.4 TB/s of planes read
+// and written), against 713 and 119 us with a line per thread.
 #include <cuda_fp16.h>
 #include "common.cuh"
 #include "av1_spec_tables.h"

@@ -28,13 +28,11 @@
 //    (film_grain.rs:599-760).  Chroma is blended first from the un-noised
 //    luma, then luma, as the reference orders it (film_grain.rs:758-828).
 //    A CTA lays the frame's templates out in shared memory, with a scaling table
-//    of one entry per sample value.  Bound by issue and the latency of the
-//    samples' loads: 193 us for four 3840x2160 10-bit 4:2:0 frames and 170 us for
-//    twelve 718p 4:4:4 ones when a thread took four columns, interpolated each
-//    scaling value and reread the frame's parameters after every store; 112 and
-//    87 us with tiles, tables and templates in shared memory; 89 and 67 us with
-//    all of a row's samples asked for at once (2.2 TB/s and 2.3 TB/s of planes
-//    read and written).
+//    of one entry per sample value, and asks for all of a row's samples at once.
+//    Bound by issue and the latency of the samples' loads: 89 us for four 3840x2160
+//    10-bit 4:2:0 frames and 67 us for twelve 718p 4:4:4 ones (2.2 TB/s and 2.3 TB/s of
+//    planes read and written), against 193 and 170 us when a thread took four columns,
+//    interpolated each scaling value and reread the frame's parameters after every store.
 #include "common.cuh"
 #include "av1_spec_tables.h"
 

@@ -34,8 +34,8 @@
 // What bounds it is the chain of levels: a 1920x1080 key frame's longest one has
 // about 2,200, nearly all with one to four TUs of at most 256 samples.  Measured
 // on that frame (one launch, B200): 8.5 ms with a body per transform size and
-// every level on one barrier, 2.5 ms in this form; 3840x2160 10-bit in 2 x 2
-// tiles 10.0 against 2.6 ms, eight 640x360 frames 2.7 against 0.78 ms.
+// every level on one barrier, 2.2 ms in this form; 3840x2160 10-bit in 2 x 2
+// tiles 10.0 against 2.3 ms, eight 640x360 frames 2.7 against 0.78 ms.
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -390,7 +390,7 @@ __device__ void prep_tu(const IntraFrame& F, int log2sb, const av1g_intra_tu& t,
         r.ea = (uint16_t)ea;
         r.el = (uint16_t)el;
         if (r.cls == C_DC && ea + el) recip = (uint32_t)(((1ull << 32) + ea + el - 1) / (ea + el));
-        // the copy holds the row above up to kIntraCopyExt samples past the
+        // the copy holds the row above up to intra_copy_ext samples past the
         // superblock, and otherwise the superblock's own columns
         const int wide = ly == 0 ? sbw + intra_copy_ext(sbw) : sbw;
         if (lx + min(ea, (int)r.na) <= wide && ly + min(el, (int)r.nl) <= sbh) {
@@ -1635,10 +1635,6 @@ __global__ void __launch_bounds__(kIT, 1) intra_kernel(const IntraFrame* __restr
     }
 }
 
-}  // namespace
-
-
-namespace {
 // Test hook state: a never-satisfied wait is planned into the first
 // superblock of every job whose frame is this wide (0: none).
 std::atomic<int> g_fault_width{0};

@@ -40,14 +40,9 @@ struct Cells {
     int base, stride, cx0, cx1, cy0, cy1;
 };
 
-}  // namespace
-
-namespace {
-
 // One job's part of the plan.
 struct JobPlan {
     const av1g_intra_job* j;
-    int index;
     int pw[3] = {}, ph[3] = {};
     int sb = 64, log2sb = 6, ssx = 0, ssy = 0, sb_cols = 0, sb_rows = 0;
     struct Sb {
@@ -410,7 +405,6 @@ av1g_status intra_plan(const av1g_intra_job* jobs, int n, IntraPlan& plan, std::
         F.np = h.num_planes;
         JobPlan& P = J[i];
         P.j = &j;
-        P.index = i;
         P.sb = j.sb_size;
         P.log2sb = P.sb == 128 ? 7 : 6;
         P.ssx = h.subsampling_x;

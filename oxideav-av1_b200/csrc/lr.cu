@@ -26,12 +26,11 @@
 //    are not computed.
 // Units of type RESTORE_NONE copy the CDEF samples through.
 //
-// Bound by instruction issue: 64 x 1080p 8-bit took 1.67 ms at 198 thread instructions
-// per sample, when every thread worked its tile out for itself, with 64-bit divisions
-// for the box filter's scale; 1.38 ms with one thread working out the next tile and
-// the scales in a table; 1.29 ms with a and b in one word and the 3x3 weighting of a
-// pair of rows from one reading of them (three loads per output, not nine).  Four
-// CTAs per SM: five, at 48 registers, took 1.50 against 1.38 ms.
+// Bound by instruction issue: 64 x 1080p 8-bit take 1.29 ms at 127 thread instructions
+// per sample, with one thread working out the next tile, the scales in a table, a and b
+// in one word and the 3x3 weighting of a pair of rows from one reading of them (three
+// loads per output, not nine), against 1.67 ms at 198 without any of these.  Four CTAs
+// per SM: five leave 48 registers and are slower.
 #include <cstddef>
 
 #include "common.cuh"

@@ -14,11 +14,9 @@
 // The next tile's samples are in registers while this one is filtered, so a tile
 // costs one barrier.
 //
-// Both source sets of four 3840x2160 10-bit 4:2:0 frames at denominator 12: 402 us
-// with tiles of one row, each tap a load and a multiply-add of its own; 194 us with
-// eight rows and two-way dot products on two copies of the window, one a sample
-// off; 165 us with the taps placed instead; 128 us with the next tile in
-// registers.  That is 40 % of the copy rate on the planes read and written; what
+// Both source sets of four 3840x2160 10-bit 4:2:0 frames at denominator 12: 128 us,
+// against 402 us with tiles of one row and each tap a load and a multiply-add of its
+// own.  That is 40 % of the copy rate on the planes read and written; what
 // remains is the dot products and the window's way through shared memory.
 #include "common.cuh"
 #include "av1_spec_tables.h"
