@@ -721,11 +721,11 @@ __global__ void __launch_bounds__(kDbThreads, kDbCtas) deblock_kernel(const Fram
             }
             strengths[threadIdx.x] = e;
         }
-        if (seen & ~kSample) plan[k].lines = 1;
+        if (__builtin_expect(seen & ~kSample, 0)) plan[k].lines = 1;
         __syncthreads();
         if (threadIdx.x == kDbThreads - 1 && t + (int)gridDim.x < total)
             plan_tile(frames, starts, n, t + gridDim.x, plan[k ^ 1]);
-        if (T.lines) {
+        if (__builtin_expect(T.lines, 0)) {
             if (bd == 12) filter_tile_by_lines<12>(T, win, code, strengths);
             else filter_tile_by_lines<10>(T, win, code, strengths);
             continue;

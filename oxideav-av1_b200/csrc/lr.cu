@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(kLrThreads, 4) lr_kernel(const FrameDev* __res
         }
         if (seen & 0xfc00fc00u) s.tile[cur].packed = 0;
         __syncthreads();
-        const bool packed = T.packed;
+        const bool packed = bd == 8 || __builtin_expect(T.packed, 1);
         const int maxv = (1 << bd) - 1;
         if (u.type == 1) {
             int hf[7], vf[7];
